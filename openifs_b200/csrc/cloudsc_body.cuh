@@ -14,24 +14,24 @@
 #define CSC_LEVEL_SYNC()
 #endif
 
-// Every division of the column code: fast_div when FAST_ (the fast pass),
-// recording in divbad_ the operands outside its exact window; IEEE division
+// Every division of the column code: the branch-free division when FAST_ (the
+// fast pass; with CHK_ recording its operands in divbad_), IEEE division
 // otherwise (cdiv, cloudsc_column.cuh).
-#define DIV(...) cdiv<FAST_>(__VA_ARGS__, divbad_)
+#define DIV(...) cdiv<FAST_, CHK_>(__VA_ARGS__, divbad_)
 // A literal divisor: its reciprocal folded at compile time (cdivk).
-#define DIVK(A, B) cdivk<FAST_>(A, B, 1.0 / (B), divbad_)
+#define DIVK(A, B) cdivk<FAST_, CHK_>(A, B, 1.0 / (B), divbad_)
 // A power-of-two literal divisor: multiplication by its exact reciprocal,
 // the same bits as the division for every operand.
 #define DIV2(A, B) ((A) * decltype(A)(1.0 / (B)))
 // A parameter divisor with its reciprocal computed on the host (KParams rcp_*).
-#define DIVP(A, B, Y) cdivk<FAST_>(A, B, Y, divbad_)
-// The quotient 1/B (crcp): in the fast pass the reciprocal half of fast_div,
-// recording B's window.
-#define RCP(B) crcp<FAST_>(B, divbad_)
+#define DIVP(A, B, Y) cdivk<FAST_, CHK_>(A, B, Y, divbad_)
+// The quotient 1/B (crcp): in the fast pass the reciprocal half of the division.
+#define RCP(B) crcp<FAST_, CHK_>(B, divbad_)
 // A / B for a divisor shared by several quotients, Y = RCP(B) computed once:
-// the same operations as DIV(A, B) (fast_div is fast_rcp followed by
-// fast_div_k's corrections), so the same bits.
-#define DIVY(A, B, Y) cdivk<FAST_>(A, B, Y, divbad_)
+// the same operations as DIV(A, B), so the same bits.
+#define DIVY(A, B, Y) cdivk<FAST_, CHK_>(A, B, Y, divbad_)
+// Report the column to the rerun when C holds.
+#define REPORT_IF(C) divbad_.pos |= (C) ? kPosRange : 0u
 
 namespace cloudsc {
 
@@ -75,7 +75,7 @@ CSC_DEV double sink_sum(int jo, const QA &q) {
   }
 #define SCL1(F, A) \
   if (F) A = A * zr;
-template <bool FAST_>
+template <bool FAST_, bool CHK_>
 CSC_DEV void scale_row(int jo, QA &q, const double qx[5], DivCheck &divbad_) {
   const double zepsec = 1.E-14;
   const double ss = sink_sum(jo, q);
@@ -109,7 +109,7 @@ CSC_DEV void scale_row(int jo, QA &q, const double qx[5], DivCheck &divbad_) {
 #undef SCL2
 
 // ZRATIO for every species from the current ZSOLQA (cloudsc.F90:3455-3474).
-template <bool FAST_>
+template <bool FAST_, bool CHK_>
 CSC_DEV void sink_ratios(const QA &q, const double qx[5], double r[5], DivCheck &divbad_) {
   const double zepsec = 1.E-14;
 #pragma unroll
@@ -122,7 +122,7 @@ CSC_DEV void sink_ratios(const QA &q, const double qx[5], double r[5], DivCheck 
 // ---------------------------------------------------------------------------
 // CLOUD_SUPERSATCHECK (cloud_supersatcheck.F90:111-226, KFTLIQICE=1), double.
 // ---------------------------------------------------------------------------
-template <bool FAST_>
+template <bool FAST_, bool CHK_>
 CSC_DEV void supersatcheck(double pt, double pq, double pa, double pp, double &t_adj, double &q_adj,
                            double &a_adj, double &l_adj, double &i_adj, DivCheck &divbad_) {
   const KParamsD &k = c_kd;
@@ -131,13 +131,13 @@ CSC_DEV void supersatcheck(double pt, double pq, double pa, double pp, double &t
   double zt = mx(pt, 160.0);
   double za = mx(mn(pa, 1.0), 0.0);
   double zp_r = RCP(pp);
-  double el = xexp(DIV(k.r3les * (zt - k.rtt), (zt - k.r4les)));
+  double el = mexp<false, FAST_>(DIV(k.r3les * (zt - k.rtt), (zt - k.r4les)));
   double x = (mx(k.rtice, mn(k.rtwat, zt)) - k.rtice) * k.rtwat_rtice_r;
   double alfa = mn(1.0, x * x);
   bool delta = copysign(1.0, zt - k.rtt) > 0.0;  // FOEDELTA = 1
   // computed whether or not a term needs it: without the branch the two
   // exponentials overlap (the same bits where it is used)
-  double ei = xexp(DIV(k.r3ies * (zt - k.rtt), (zt - k.r4ies)));
+  double ei = mexp<false, FAST_>(DIV(k.r3ies * (zt - k.rtt), (zt - k.r4ies)));
   double zfoeeliq = mn((k.r2es * el) * zp_r, 0.5);
   double foeew = delta ? k.r2es * el : k.r2es * ei;
   double zfoeeice = mn(foeew * zp_r, 0.5);
@@ -369,15 +369,16 @@ CSC_DEV void write_budgets(const Fields &F, const KParams<Real> &P, const double
 // for the uploaded parameters (gen_exponents_ok); same results, fewer
 // branches.
 // PASS (kPassPlain, kPassFast, kPassRedo; cloudsc_column.cuh): the fast pass
-// divides with fast_div, sets *bad when an operand of one of its divisions
-// fell outside that division's exact window, and saves the PLUDE input of every level in
-// plude_in[0..KLEV-1]; the redo pass, the column run again with IEEE division,
-// reads PLUDE from plude_in.  A column whose fast pass sets *bad must be rerun
+// runs the branch-free divisions, exps, logs and pows, sets *bad when one of
+// its input checks left the window in which those are exact, and saves the
+// PLUDE input of every level in plude_in[0..KLEV-1]; the redo pass, the column
+// run again with IEEE division and plibm's full functions, reads PLUDE from
+// plude_in.  A column whose fast pass sets *bad must be rerun
 // (its outputs, stored in the same places by both passes, are then final) and
 // leaves its warning count to the rerun.
 // With BUD, PEXTRA is accumulated in place, so the two passes share its
-// levels: the fast pass adds a level's budget terms only while no division
-// has reported (everything it computed up to there is IEEE's), and records
+// levels: the fast pass adds a level's budget terms only while no check has
+// reported (everything it computed up to there is IEEE's), and records
 // in *kbud the first level it left out; the redo pass adds the terms of the
 // levels from *kbud on.  Every slot then receives IEEE's terms once each, in
 // level order, as in one IEEE run.
@@ -390,9 +391,18 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
   typedef double D;
 #define C(x) Real(x)
   constexpr bool FAST_ = PASS == kPassFast;
+  // the optional forms' factors and inputs are not among the level's input
+  // checks: their divisions check their own operands
+  constexpr bool CHK_ = OPT;
   DivCheck divbad_;
   if constexpr (FAST_) {
-    if (P.rcp_force) divbad_.acc = ~0u;  // a parameter divisor fast_div_k cannot take: rerun
+    if (P.rcp_force) divbad_.acc = ~0u;  // a parameter outside the fast pass's ranges: rerun
+#if defined(CLOUDSC_HOST_WINDOW_CHECK) && !defined(__CUDA_ARCH__)
+    g_column = &divbad_;
+#endif
+#if defined(CLOUDSC_HOST_FORCE_REDO) && !defined(__CUDA_ARCH__)
+    divbad_.acc = ~0u;
+#endif
   }
   const int np = sh.nproma, klev = sh.klev;
   const size_t s2 = (size_t)np * klev, s2h = (size_t)np * (klev + 1);
@@ -415,6 +425,10 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
   // reciprocals of the column's constant divisors (time step, surface
   // pressure), taken once
   const Real rrdt = RCP(rdt), rpsurf = RCP(Real(paph_surf));
+  if constexpr (FAST_) {
+    see_pos(dt, -10, divbad_);
+    see_pos(paph_surf, -8, divbad_);
+  }
   Real zadvw = C(1.0), zadvwd = C(1.0);
   if (ktype == 1 && P.rmfadvw > C(0.0)) {
     zadvw = C(1.0) - P.rmfadvw;
@@ -520,14 +534,41 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
     // 1/(1 - RETV FOEEW) for the mixed, ice and liquid saturation pressures:
     // the divisors of ZQSMIX/ZQSICE/ZQSLIQ and the ZCOR factors below
     Real rmix = C(0.0), rice = C(0.0), rliq = C(0.0);
+    // The fast pass's input checks.  With T in [128, 1024) K, the pressures,
+    // the layer thickness, the amounts, the cloud fraction and the convective
+    // inputs inside the bounds below, and the parameters inside those of
+    // fast_pass_params_ok, every operand of the level's divisions, exps, logs
+    // and pows lies in the window where the fast forms are exact:
+    //  * T bounds the saturation exponentials (1e-13 .. 1e8 relative to
+    //    their value at RTT) and T - R4xES away from zero; with the pressure
+    //    it bounds the saturation humidities (below 0.5) and their 1 - RETV q;
+    //  * after the tidy-up an amount is zero or >= RLMIN and the cloud
+    //    fraction zero or >= RAMIN; the divisors formed from amounts sit
+    //    behind the scheme's own > ZEPSEC, RLMIN or RCOVPMIN tests, the others
+    //    are 1 plus a non-negative term or bounded by T and the pressures;
+    //  * a dividend is a product of bounded factors or a sum of doubles that
+    //    are each zero or above 2^-600, so it is zero or above 2^-700: its
+    //    residuals do not underflow;
+    //  * what is carried down the column is bounded again by the checks of
+    //    the solved amounts and of the updated T and q below.
+    // (Checking each operand instead cost about ten instructions a division
+    // and a branch a pow.)
+    if constexpr (FAST_) {
+      if (k >= ncldtop0) {
+        REPORT_IF(!(tD >= 128.0 && tD < 1024.0));
+        see_pos(pap_kd, -8, divbad_);
+        see_pos(paph_k1, -8, divbad_);
+        see_pos(paph_k1 - paph_k, -10, divbad_);
+      }
+    }
     if (k >= ncldtop0) {
       Real x = (mx(P.rtice, mn(P.rtwat, t)) - P.rtice) * P.rtwat_rtice_r;
       alfa = mn(C(1.0), x * x);
-      el_e = mexp<F32M>(DIV(P.r3les * (t - P.rtt), (t - P.r4les)));
+      el_e = mexp<F32M, FAST_>(DIV(P.r3les * (t - P.rtt), (t - P.r4les)));
       bool delta = xsign(C(1.0), t - P.rtt) > C(0.0);
       // the ice exponential whether or not a term needs it (no branch: the
       // two exponentials overlap)
-      ei_e = mexp<F32M>(DIV(P.r3ies * (t - P.rtt), (t - P.r4ies)));
+      ei_e = mexp<F32M, FAST_>(DIV(P.r3ies * (t - P.rtt), (t - P.r4ies)));
       Real wsum = (alfa < C(1.0)) ? alfa * el_e + (C(1.0) - alfa) * ei_e : el_e;
       const Real rpap = RCP(pap_k);
       zfoeewm = mn(DIVY((P.r2es * wsum), pap_k, rpap), C(0.5));
@@ -582,6 +623,19 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
     TIDY(qsD, lneg_s, ralsdcp)
 #undef TIDY
     aD = mx(0.0, mn(1.0, aD));
+    if constexpr (FAST_) {
+      if (k >= ncldtop0) {
+        see(qvD, divbad_);
+        const D sum = qlD + qiD + qrD + qsD + aD + (qvD < 0.0 ? -qvD : qvD);
+        REPORT_IF(!(sum < 8.0));
+        see(pmfu_k1, divbad_);
+        see(pmfd_k1, divbad_);
+        see(plu_k1, divbad_);
+        see(plude_k, divbad_);
+        see(pludeli1, divbad_);
+        see(pludeli2, divbad_);
+      }
+    }
     const Real qv = Real(qvD), a = Real(aD);
     const Real ql = Real(qlD), qi = Real(qiD), qr = Real(qrD), qs = Real(qsD);
     const Real zli = ql + qi;
@@ -642,13 +696,13 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
       const Real zrho = DIV(pap_k, (P.rd * t));
       const Real rrho = RCP(zrho);
       // (RDENSREF/ZRHO)**0.4 appears in three processes: one shared logarithm
-      const PowBase b_dens = mbase<F32M>(DIVY(P.rdensref, zrho, rrho));
+      const PowBase b_dens = mbase<F32M, FAST_>(DIVY(P.rdensref, zrho, rrho));
       // its two powers (0.4 in the rain fall speed, the binary32 0.4 in rain
       // evaporation and riming), computed here for every point so that they
       // overlap with the code around them instead of waiting inside their
       // processes' branches
-      const Real fallcorr_r = mpowb<F32M>(b_dens, C(0.4));
-      const Real fallcorr_f = mpowbp<F32M, GEN>(b_dens, P.flt_0p4);
+      const Real fallcorr_r = mpowb<F32M, FAST_>(b_dens, C(0.4));
+      const Real fallcorr_f = mpowbp<F32M, GEN, FAST_>(b_dens, P.flt_0p4);
       const Real zdtgdp = rdt * zgdp;
       const Real zrdtgdp = zdp * zrdtgdp_f;
       Real zcorqsliq, zcorqsice, zcorqsmix, zdqsmixdt, zevaplimmix, rcqsmix;
@@ -704,8 +758,13 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
           plude_k = 0.0;
         }
         if (P.lmfdsnow) {
-          convsrce_r = Real(ld(F.psnde + ok2s)) * zdtgdp;
-          convsrce_s = Real(ld(F.psnde + ok2s + s2)) * zdtgdp;
+          const D psnde_r = ld(F.psnde + ok2s), psnde_s = ld(F.psnde + ok2s + s2);
+          if constexpr (FAST_) {
+            see(psnde_r, divbad_);
+            see(psnde_s, divbad_);
+          }
+          convsrce_r = Real(psnde_r) * zdtgdp;
+          convsrce_s = Real(psnde_s) * zdtgdp;
           QADD(RR, convsrce_r);
           QADD(SS, convsrce_s);
         }
@@ -809,8 +868,8 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
         Real ztemp = C(0.5) * (qr + qxnm1_r);
         if (ztemp != C(0.0)) {
           Real zfallcorr = fallcorr_r;
-          Real zrlambda = mpowp<F32M, GEN>(DIVP(zrho * ztemp, P.rcl_lam1r, P.rcp_rcl_lam1r), P.rcl_lam2r);
-          fs_r = P.rxfallspeedrain * zfallcorr * P.rcl_const7r * mpowp<F32M, GEN>(zrlambda, P.rcl_dr);
+          Real zrlambda = mpowp<F32M, GEN, FAST_>(DIVP(zrho * ztemp, P.rcl_lam1r, P.rcp_rcl_lam1r), P.rcl_lam2r);
+          fs_r = P.rxfallspeedrain * zfallcorr * P.rcl_const7r * mpowp<F32M, GEN, FAST_>(zrlambda, P.rcl_dr);
         }
       }
       if (k > ncldtop0) {
@@ -854,7 +913,7 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
 
       // 4.3 warm rain, IWARMRAIN=3, IRAINACC=1 (:1930-2259)
       if (zliqcld > zepsec) {
-        const PowBase b_liq = mbase<F32M>(zliqcld);
+        const PowBase b_liq = mbase<F32M, FAST_>(zliqcld);
         Real zeaut = P.rcl_inhomogaut, zeacc = P.rcl_inhomogacc;
         if constexpr (OPT) {
           double zcldraincorr = 0.0;
@@ -890,12 +949,12 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
             zeacc = zeacc * Real(sppf[8]);
           }
         }
-        Real zrainaut = zeaut * rdt * P.rcl_kkaau * mpowbp<F32M, GEN>(b_liq, P.kkbauq_m1) * zconstpow;
+        Real zrainaut = zeaut * rdt * P.rcl_kkaau * mpowbp<F32M, GEN, FAST_>(b_liq, P.kkbauq_m1) * zconstpow;
         qb_rl = qb_rl + zrainaut;
         Real zrainacc = C(0.0);
         if (zraincld > zepsec) {
-          zrainacc = zeacc * rdt * P.rcl_kkaac * mpowbp<F32M, GEN>(b_liq, P.kkbac_m1) *
-                     mpowp<F32M, GEN>(zraincld, P.rcl_kkbac);
+          zrainacc = zeacc * rdt * P.rcl_kkaac * mpowbp<F32M, GEN, FAST_>(b_liq, P.kkbac_m1) *
+                     mpowp<F32M, GEN, FAST_>(zraincld, P.rcl_kkbac);
         }
         qb_rl = qb_rl + zrainacc;
         if constexpr (BUD) {
@@ -926,15 +985,15 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
           Real zpreclr = zraincldm1;
           Real zfallcorr = fallcorr_f;
           Real zesatliq = P.rv_rd * (P.r2es * el_e);
-          Real zlambda = mpowp<F32M, GEN>(DIV(P.rcl_lam1r, (zrho * zpreclr)), P.rcl_lam2r);
-          const PowBase b_lam = mbase<F32M>(zlambda);
+          Real zlambda = mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1r, (zrho * zpreclr)), P.rcl_lam2r);
+          const PowBase b_lam = mbase<F32M, FAST_>(zlambda);
           Real zevap_denom = P.rcl_cdenom1 * zesatliq - P.rcl_cdenom2 * t * zesatliq +
-                             P.rcl_cdenom3 * mpow<F32M>(t, C(3.0)) * pap_k;
-          Real zcorr2 = DIV(mpow<F32M>(DIVK(t, 273.), C(1.5)) * C(393.), (t + C(120.)));
+                             P.rcl_cdenom3 * mpow<F32M, FAST_>(t, C(3.0)) * pap_k;
+          Real zcorr2 = DIV(mpow<F32M, FAST_>(DIVK(t, 273.), C(1.5)) * C(393.), (t + C(120.)));
           Real zsubsat = mx(zzrh * zqsliq - zqe, C(0.0));
           Real zbeta = (DIV(C(0.15), zqsliq)) * (t * t) * zesatliq * P.rcl_const1r * (DIV(zcorr2, zevap_denom)) *
-                       (DIV(C(0.78), (mpowbp<F32M, GEN>(b_lam, P.rcl_const4r))) +
-                        DIV(P.rcl_const2r * mpow<F32M>(zrho * zfallcorr, C(0.5)), (mpow<F32M>(zcorr2, C(0.5)) * mpowbp<F32M, GEN>(b_lam, P.rcl_const3r))));
+                       (DIV(C(0.78), (mpowbp<F32M, GEN, FAST_>(b_lam, P.rcl_const4r))) +
+                        DIV(P.rcl_const2r * mpow<F32M, FAST_>(zrho * zfallcorr, C(0.5)), (mpow<F32M, FAST_>(zcorr2, C(0.5)) * mpowbp<F32M, GEN, FAST_>(b_lam, P.rcl_const3r))));
           Real zdenom = C(1.0) + zbeta * rdt * zcorqsliq;
           Real zdpevap = DIV(zcovpclr * zbeta * rdt * zsubsat, zdenom);
           if (spp && P.spp_on[CLOUDSC_SPP_RAINEVAP]) zdpevap = zdpevap * Real(sppf[CLOUDSC_SPP_RAINEVAP]);
@@ -955,12 +1014,12 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
         if (t < (P.rtt - C(5.)) && qxfg_l > P.rlmin) {
           Real zsupersatice = DIV((zqsliq - zqsice), zqsice);
           Real zvpice = DIVP((P.r2es * ei_e) * P.rv, P.rd, P.rcp_rd);
-          Real zicenuclei = C(1000.0) * mexp<F32M>(C(12.96) * zsupersatice - C(0.639));
+          Real zicenuclei = C(1000.0) * mexp<F32M, FAST_>(C(12.96) * zsupersatice - C(0.639));
           Real zadd = DIV(P.rlstt * (DIV(P.rlstt, (P.rv * t)) - C(1.0)), (C(2.4E-2) * t));
           Real zbdd = DIV(P.rv * t * pap_k, (C(2.21) * zvpice));
-          Real zcvds = DIV(C(7.8) * mpow<F32M>(DIVY(zicenuclei, zrho, rrho), C(0.666)) * zsupersatice, (C(8.87) * (zadd + zbdd)));
+          Real zcvds = DIV(C(7.8) * mpow<F32M, FAST_>(DIVY(zicenuclei, zrho, rrho), C(0.666)) * zsupersatice, (C(8.87) * (zadd + zbdd)));
           Real zice0 = mx(zicecld, DIVY(zicenuclei * P.riceinit, zrho, rrho));
-          Real zinew = mpow<F32M>(C(0.666) * zcvds * rdt + mpow<F32M>(zice0, C(0.666)), C(1.5));
+          Real zinew = mpow<F32M, FAST_>(C(0.666) * zcvds * rdt + mpow<F32M, FAST_>(zice0, C(0.666)), C(1.5));
           D zdepos = D(mx(P.rcl_overlapliqice * a * (zinew - zice0), C(0.0)));
           zdepos = mn(zdepos, qxfg_l);
           Real zinfactor = mn(DIVK(zicenuclei, 15000.), C(1.0));
@@ -983,14 +1042,14 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
         if (t < P.rtt && zsnowcld > zepsec && zsupersatice > C(0.0)) {
           Real zvpice = DIVP((P.r2es * ei_e) * P.rv, P.rd, P.rcp_rd);
           Real zaplusb = P.rcl_apb1 * zvpice - P.rcl_apb2 * zvpice * t + pap_k * P.rcl_apb3 * (t * t * t);
-          Real zcorrfac = mpow<F32M>(rrho, C(0.5));
-          Real zcorrfac2 = (mpow<F32M>(DIVK(t, 273.0), C(1.5))) * (DIV(C(393.0), (t + C(120.0))));
+          Real zcorrfac = mpow<F32M, FAST_>(rrho, C(0.5));
+          Real zcorrfac2 = (mpow<F32M, FAST_>(DIVK(t, 273.0), C(1.5))) * (DIV(C(393.0), (t + C(120.0))));
           Real zpr02 = zrho * zsnowcld * P.rcl_const1s;
-          const PowBase b_pr02 = mbase<F32M>(zpr02);
+          const PowBase b_pr02 = mbase<F32M, FAST_>(zpr02);
           Real zterm1 = DIV(zsupersatice * (t * t) * zvpice * zcorrfac2 * P.rcl_const2s, (zrho * zaplusb));
-          Real zterm2 = C(0.65) * P.rcl_const6s * mpowbp<F32M, GEN>(b_pr02, P.rcl_const4s) +
-                        DIV(P.rcl_const3s * mpow<F32M>(zcorrfac, C(0.5)) * mpow<F32M>(zrho, C(0.5)) *
-                            mpowbp<F32M, GEN>(b_pr02, P.rcl_const5s), mpow<F32M>(zcorrfac2, C(0.5)));
+          Real zterm2 = C(0.65) * P.rcl_const6s * mpowbp<F32M, GEN, FAST_>(b_pr02, P.rcl_const4s) +
+                        DIV(P.rcl_const3s * mpow<F32M, FAST_>(zcorrfac, C(0.5)) * mpow<F32M, FAST_>(zrho, C(0.5)) *
+                            mpowbp<F32M, GEN, FAST_>(b_pr02, P.rcl_const5s), mpow<F32M, FAST_>(zcorrfac2, C(0.5)));
           Real zpsdep = mx(zcovptot * zterm1 * zterm2 * rdt, C(0.0));
           zpsdep = DIVY(mn(zpsdep, qv - zqsmix), zcorqsmix, rcqsmix);
           QADD(SV, zpsdep);  // (S,V) += zpsdep, (V,S) -= zpsdep
@@ -1004,7 +1063,7 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
 
       // 4.8 ice -> snow autoconversion (:2769-2800)
       if (t <= P.rtt && zicecld > zepsec) {
-        Real zzco = rdt * P.rsnowlin1 * mexp<F32M>(P.rsnowlin2 * (t - P.rtt));
+        Real zzco = rdt * P.rsnowlin1 * mexp<F32M, FAST_>(P.rsnowlin2 * (t - P.rtt));
         Real zlcrit = P.rlcritsnow;
         bool aer = false;
         if constexpr (OPT) {
@@ -1012,7 +1071,7 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
           // (RNICE/PNICE)**0.333 (:2776-2779)
           if (P.laericeauto) {
             zlcrit = Real(ld(F.picrit_aer + ok));
-            zzco = zzco * mpow<F32M>(DIV(P.rnice, Real(ld(F.pnice + ok))), C(0.333));
+            zzco = zzco * mpow<F32M, FAST_>(DIV(P.rnice, Real(ld(F.pnice + ok))), C(0.333));
             aer = true;
           }
         }
@@ -1020,7 +1079,10 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
           zlcrit = P.rlcritsnow * Real(sppf[CLOUDSC_SPP_RLCRITSNOW]);
         Real r = DIV(zicecld, zlcrit);
         Real ztemp = C(-1.) * (r * r);
-        Real zsnowaut = (ztemp < C(50.0)) ? zzco * (C(1.0) - mexp<F32M>(ztemp)) : zzco;
+        // 1 - exp(x) is 1 for every x <= -100: the bound changes nothing and
+        // keeps the argument in the fast exp's window
+        if (FAST_ && !F32M) ztemp = mx(ztemp, C(-100.0));
+        Real zsnowaut = (ztemp < C(50.0)) ? zzco * (C(1.0) - mexp<F32M, FAST_>(ztemp)) : zzco;
         qb_si = qb_si + zsnowaut;
         if constexpr (BUD) b_snowaut = zsnowaut;
       }
@@ -1066,9 +1128,9 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
         if (t < P.rtt) {
           Real zfrzmax;
           if (llrainliq) {
-            Real zlambda = mpowp<F32M, GEN>(DIV(P.rcl_lam1r, (zrho * qr)), P.rcl_lam2r);
+            Real zlambda = mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1r, (zrho * qr)), P.rcl_lam2r);
             Real ztemp = mn(P.rcl_fzrab * (t - P.rtt), C(50.));
-            Real zfrz = rdt * (DIVY(P.rcl_const5r, zrho, rrho)) * (mexp<F32M>(ztemp) - C(1.)) * mpowp<F32M, GEN>(zlambda, P.rcl_const6r);
+            Real zfrz = rdt * (DIVY(P.rcl_const5r, zrho, rrho)) * (mexp<F32M, FAST_>(ztemp) - C(1.)) * mpowp<F32M, GEN, FAST_>(zlambda, P.rcl_const6r);
             zfrzmax = mx(zfrz, C(0.0));
           } else {
             Real zcons1 = xabs(DIVP(rdt * (C(1.0) + C(0.5) * (P.rtt - t)), P.rtaumel, P.rcp_rtaumel));
@@ -1096,7 +1158,7 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
       if (t <= P.rtt && zliqcld > zepsec && zsnowcld > zepsec && zcovptot > C(0.01)) {
         Real zfallcorr = fallcorr_f;
         Real zsnowrime = P.rcl_effrime * zcovptot * rdt * P.rcl_const7s * zfallcorr *
-                         mpowp<F32M, GEN>(zrho * zsnowcld * P.rcl_const1s, P.rcl_const8s);
+                         mpowp<F32M, GEN, FAST_>(zrho * zsnowcld * P.rcl_const1s, P.rcl_const8s);
         zsnowrime = mn(zsnowrime, C(1.0));
         qb_sl = qb_sl + zsnowrime;
         if constexpr (BUD) b_snowrime = zsnowrime;
@@ -1104,11 +1166,11 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
 
       // PSD slopes (:3026-3069), PSACR (:3084-3115), PIACR (:3171-3198)
       if (t <= P.rtt && prainfrac < zepsec && zraincld > zepsec) {
-        Real zlamr = mpowp<F32M, GEN>(DIV(P.rcl_lam1r, (zrho * zraincld)), P.rcl_lam2r);
-        Real zn0r = P.rcl_x1r * mpowp<F32M, GEN>(zlamr, P.rcl_x2r);
+        Real zlamr = mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1r, (zrho * zraincld)), P.rcl_lam2r);
+        Real zn0r = P.rcl_x1r * mpowp<F32M, GEN, FAST_>(zlamr, P.rcl_x2r);
         Real zlamr3 = zlamr * zlamr * zlamr;
         if (zsnowcld > zepsec) {
-          Real zlams = mpowp<F32M, GEN>(DIV(P.rcl_lam1s, (zrho * zsnowcld)), P.rcl_lam2s);
+          Real zlams = mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1s, (zrho * zsnowcld)), P.rcl_lam2s);
           Real zn0s = P.rcl_x1s;
           Real zfalldiff = mx(xabs(fs_r - fs_s), DIV2((fs_r + fs_s), C(8.)));
           Real zfac = DIV(P.rpi * P.rpi * P.rdenswat * zrho * zn0r * zn0s, (zlams * zlamr3));
@@ -1119,7 +1181,7 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
           if constexpr (BUD) b_psacr = zpsacr;
         }
         if (zicecld > zepsec) {
-          Real zlami = mpowp<F32M, GEN>(DIV(P.rcl_lam1s, (zrho * zicecld)), P.rcl_lam2s);
+          Real zlami = mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1s, (zrho * zicecld)), P.rcl_lam2s);
           Real zn0i = P.rcl_x1s;
           Real zfalldiff = mx(xabs(fs_r - fs_i), DIV2((fs_r + fs_i), C(8.)));
           Real zfac = DIV(P.rpi * P.rpi * P.rdenswat * C(0.1) * zrho * zn0r * zn0i, (zlami * zlamr3));
@@ -1141,7 +1203,7 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
           Real aa = zcovptot * zdtgdp;
           Real zpreclr = DIV(Real(qxfg_s) * zcovpclr, xsign(mx(xabs(aa), zepsilon), aa));
           Real zbeta1 = DIV(DIVP(xsqrt(DIVY(pap_k, Real(paph_surf), rpsurf)), P.rvrfactor, P.rcp_rvrfactor) * zpreclr, mx(zcovpclr, zepsec));
-          Real zbeta = P.rg * P.rpecons * mpow<F32M>(zbeta1, C(0.5777));
+          Real zbeta = P.rg * P.rpecons * mpow<F32M, FAST_>(zbeta1, C(0.5777));
           Real zdenom = C(1.0) + zbeta * rdt * zcorqsice;
           Real zdpr = DIV(zcovpclr * zbeta * (zqsice - zqe), zdenom) * zdp * P.zrg_r;
           Real zdpevap = zdpr * zdtgdp;
@@ -1176,7 +1238,7 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
       const double qx[5] = {qlD, qiD, qrD, qsD, qvD};
       {
         double ratio[5];
-        sink_ratios<FAST_>(q, qx, ratio, divbad_);
+        sink_ratios<FAST_, CHK_>(q, qx, ratio, divbad_);
         double sr[5];
         int ord[5];
         sr[0] = ratio[0];
@@ -1208,7 +1270,7 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
 #pragma unroll
         for (int jm = 0; jm < 5; ++jm) code |= (unsigned)ord[jm] << (3 * jm);
 #pragma unroll 1
-        for (int jm = 0; jm < 5; ++jm) scale_row<FAST_>((int)((code >> (3 * jm)) & 7u), q, qx, divbad_);
+        for (int jm = 0; jm < 5; ++jm) scale_row<FAST_, CHK_>((int)((code >> (3 * jm)) & 7u), q, qx, divbad_);
       }
 
       // 5.2.2 solve (:3546-3628), double, lower-triangular form
@@ -1240,6 +1302,7 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
         if (x_r < zepsecd) { x_v = x_v + x_r; x_r = 0.0; }
         if (x_s < zepsecd) { x_v = x_v + x_s; x_s = 0.0; }
       }
+      if constexpr (FAST_) REPORT_IF(!(x_l + x_i + x_r + x_s < 16.0));
       qxnm1_l = Real(x_l);
       qxnm1_i = Real(x_i);
       qxnm1_r = Real(x_r);
@@ -1286,8 +1349,9 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
         D q_upd = pq_k + dt * (loc_q + cml_q);
         D t_upd = pt_k + dt * (loc_t + cml_t);
         D a_upd = pa_k + dt * (loc_a + cml_a);
+        if constexpr (FAST_) REPORT_IF(!(t_upd < 1024.0 && xabs(q_upd) < 16.0));
         D t_adj, q_adj, a_adj, l_adj, i_adj;
-        supersatcheck<FAST_>(t_upd, q_upd, a_upd, pap_kd, t_adj, q_adj, a_adj, l_adj, i_adj, divbad_);
+        supersatcheck<FAST_, CHK_>(t_upd, q_upd, a_upd, pap_kd, t_adj, q_adj, a_adj, l_adj, i_adj, divbad_);
         loc_q = loc_q + q_adj * zqtmst;
         loc_t = loc_t + t_adj * zqtmst;
         loc_a = loc_a + a_adj * zqtmst;
@@ -1462,5 +1526,6 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
 #undef DIVP
 #undef RCP
 #undef DIVY
+#undef REPORT_IF
 
 }  // namespace cloudsc

@@ -42,6 +42,7 @@
 // result: with an FP32 state the scheme's thresholds and MIN() limiters flip
 // (a measured 5-7 % RMS error on the T tendency).
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <type_traits>
@@ -60,54 +61,54 @@ CSC_DEV T mn(T a, T b) { return a < b ? a : b; }
 template <typename T>
 CSC_DEV T mx(T a, T b) { return a > b ? a : b; }
 
-// What the fast division reports, accumulated over every division of a
-// column.  acc ORs, for each dividend a and divisor b, the offsets
-// (2 * hi(x)) - kDivBase, whose top bits are clear exactly when x's biased
-// exponent lies in [767, 1278], i.e. 2^-256 <= |x| < 2^256 (a zero dividend
-// adds 0).  bad(): some operand left that window.
+// What the fast pass reports about a column.  A column whose operands all stay
+// inside the windows below has every fast division, exp, log and pow equal to
+// the IEEE / plibm ones bit for bit; any other column is run again with those.
+//   acc   ORs, for each checked value that may be zero, the offset
+//         2 * hi(x) - kDivBase, whose top two bits are clear exactly when
+//         2^-256 <= |x| < 2^256 (a zero adds 0);
+//   pos   ORs, for each checked positive value, hi(x) - hi(lowest allowed),
+//         below kPosRange exactly for x in [lowest, 2^32 * lowest);
+//   ones  the largest (hi(b) | 0xfff00000) & lo(b) of any divisor b: all bits
+//         set for a divisor whose significand is all ones (fast_rcp_y).
 constexpr unsigned kDivBase = 767u << 21, kDivRange = 1u << 30;
+constexpr unsigned kPosRange = 32u << 20;
 struct DivCheck {
-  unsigned acc = 0u;
-  CSC_DEV bool bad() const { return acc >= kDivRange; }
+  unsigned acc = 0u, pos = 0u, ones = 0u;
+  CSC_DEV bool bad() const { return acc >= kDivRange || pos >= kPosRange || ones == ~0u; }
 };
 
-#if !defined(__CUDA_ARCH__)
-// The window offset of x on the host (the GPU code takes hi(x) with
-// __double2hiint): host builds report the operands the GPU kernels report.
-inline unsigned div_offset_host(double x) {
+#if defined(__CUDA_ARCH__)
+CSC_DEV unsigned hi_word(double x) { return (unsigned)__double2hiint(x); }
+CSC_DEV unsigned lo_word(double x) { return (unsigned)__double2loint(x); }
+#else
+inline unsigned hi_word(double x) {
   uint64_t u;
   std::memcpy(&u, &x, sizeof u);
-  return (unsigned)(u >> 32) * 2u - kDivBase;
+  return (unsigned)(u >> 32);
+}
+inline unsigned lo_word(double x) {
+  uint64_t u;
+  std::memcpy(&u, &x, sizeof u);
+  return (unsigned)u;
 }
 #endif
+// Record a value that must be zero or inside 2^-256 <= |x| < 2^256.
+CSC_DEV void see(double x, DivCheck &dc) { dc.acc |= x == 0.0 ? 0u : hi_word(x) * 2u - kDivBase; }
+// Record a value that must lie in [2^e, 2^(e+32)).
+CSC_DEV void see_pos(double x, int e, DivCheck &dc) { dc.pos |= hi_word(x) - ((unsigned)(1023 + e) << 20); }
 
-// Branch-free double division for the column code.  A reciprocal estimate
-// (rcp.approx.ftz.f64) is refined by three Newton-Raphson steps
-// y <- y + y(1 - by), each error term and update one fused multiply-add; the
-// last step returns y = RN(1/b), the correctly rounded reciprocal, for every
-// divisor whose significand is not all ones (Markstein, IBM J. Res. Dev.
-// 34(1), 1990; Muller et al., Handbook of Floating-Point Arithmetic, ch. 5).
-// For b = (2 - 2^-52) 2^E the step ends on the tie 2^(-E-1) while
-// 1/b = 2^(-E-1) (1 + 2^-53 + 2^-106 + ...): the low significand bit of y is
-// then set, which gives RN(1/b) = 2^(-E-1) (1 + 2^-52).  The quotient of |a|,
-// q0 = RN(|a| y), within 1.5 ulp of |a|/b, is corrected twice with its
-// residual, q <- RN(q + RN(|a| - b q) y): the first correction brings it
-// within one ulp, where the residual is exact, and by Markstein's theorem the
-// second then returns RN(|a|/b).  The sign of a is put back by flipping the
-// sign bit, so that the result equals IEEE a/b bit for bit, zeros included,
-// when no step under- or overflows: that holds for 2^-256 <= |b| < 2^256 and
-// a = 0 or 2^-256 <= |a| < 2^256 (the quotient and every residual then stay
-// normal).  Operands outside that window (zeros, subnormals, infinities and
-// NaNs among them, a zero dividend excepted) are recorded in dc, and a column
-// with any is rerun with IEEE division.  The GPU tests compare it with IEEE
-// division on random operands and on hard ones (significands of all ones or
-// all zeros, quotients next to a rounding tie).  The host build divides with
-// IEEE division and reports the operands the GPU would report
-// (CLOUDSC_HOST_FORCE_REDO makes every call report, to drive the caller's
-// rerun in host tests).
-CSC_DEV double fast_div(double a, double b, DivCheck &dc) {
+// Branch-free double division, in two halves.
+//
+// The reciprocal: an estimate (rcp.approx.ftz.f64) is refined by three
+// Newton-Raphson steps y <- y + y(1 - by), each error term and update one
+// fused multiply-add; the last step returns y = RN(1/b), the correctly
+// rounded reciprocal, for every divisor whose significand is not all ones
+// (Markstein, IBM J. Res. Dev. 34(1), 1990; Muller et al., Handbook of
+// Floating-Point Arithmetic, ch. 5).  For b = (2 - 2^-52) 2^E the step ends on
+// the tie 2^(-E-1) while 1/b = 2^(-E-1) (1 + 2^-53 + 2^-106 + ...).
+CSC_DEV double fast_rcp_y(double b) {
 #if defined(__CUDA_ARCH__)
-  const int ha = __double2hiint(a), hb = __double2hiint(b);
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
   double e = __fma_rn(-b, y, 1.0);
@@ -115,104 +116,126 @@ CSC_DEV double fast_div(double a, double b, DivCheck &dc) {
   e = __fma_rn(-b, y, 1.0);
   y = __fma_rn(y, e, y);
   e = __fma_rn(-b, y, 1.0);
-  y = __fma_rn(y, e, y);
-  // all-ones significand of b: w == 0, and the clamped shift gives 1 (else 0)
-  const unsigned w = ~(((unsigned)hb | 0xfff00000u) & (unsigned)__double2loint(b));
-  y = __hiloint2double(__double2hiint(y), __double2loint(y) | (int)__funnelshift_rc(1u, 0u, w));
-  const double aa = fabs(a);
-  const double q0 = __dmul_rn(aa, y);
-  double r = __fma_rn(-b, q0, aa);
-  const double q1 = __fma_rn(r, y, q0);
-  r = __fma_rn(-b, q1, aa);
-  const double q = __fma_rn(r, y, q1);
-  const unsigned da = a == 0.0 ? 0u : (unsigned)ha * 2u - kDivBase;
-  dc.acc |= da | ((unsigned)hb * 2u - kDivBase);
-  return __hiloint2double(__double2hiint(q) ^ (ha & (int)0x80000000), __double2loint(q));
+  return __fma_rn(y, e, y);
 #else
-#if defined(CLOUDSC_HOST_FORCE_REDO)
-  dc.acc = ~0u;
-#else
-  dc.acc |= (a == 0.0 ? 0u : div_offset_host(a)) | div_offset_host(b);
-#endif
-  return a / b;
-#endif
-}
-
-// The reciprocal half of fast_div on its own: y = RN(1/b), the correctly
-// rounded reciprocal (IEEE 1/b), for 2^-256 <= |b| < 2^256; b outside that
-// window is recorded in dc.  Used for the quotients 1/b and, through
-// fast_div_k, for several dividends over one divisor.
-CSC_DEV double fast_rcp(double b, DivCheck &dc) {
-#if defined(__CUDA_ARCH__)
-  const int hb = __double2hiint(b);
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  double e = __fma_rn(-b, y, 1.0);
-  y = __fma_rn(y, e, y);
-  e = __fma_rn(-b, y, 1.0);
-  y = __fma_rn(y, e, y);
-  e = __fma_rn(-b, y, 1.0);
-  y = __fma_rn(y, e, y);
-  const unsigned w = ~(((unsigned)hb | 0xfff00000u) & (unsigned)__double2loint(b));
-  y = __hiloint2double(__double2hiint(y), __double2loint(y) | (int)__funnelshift_rc(1u, 0u, w));
-  dc.acc |= (unsigned)hb * 2u - kDivBase;
-  return y;
-#else
-#if defined(CLOUDSC_HOST_FORCE_REDO)
-  dc.acc = ~0u;
-#else
-  dc.acc |= div_offset_host(b);
-#endif
   return 1.0 / b;
 #endif
 }
-
-// fast_div for a literal divisor b, given y = RN(1/b) folded at compile
-// time (IEEE division of two constants): only the two residual corrections
-// and the dividend's window test remain.  Exact as fast_div is: every such
-// divisor lies in the window and has no all-ones significand, so y is the
-// correctly rounded reciprocal Markstein's theorem needs.
-CSC_DEV double fast_div_k(double a, double b, double y, DivCheck &dc) {
+// The quotient from y = RN(1/b): q0 = RN(a y), within 1.5 ulp of a/b, is
+// corrected twice with its residual, q <- RN(q + RN(a - b q) y): the first
+// correction brings it within one ulp, where the residual is exact, and by
+// Markstein's theorem the second then returns RN(a/b).  Equal to IEEE a/b
+// (up to the sign of a zero) when no step under- or overflows, for instance
+// for 2^-256 <= |b| < 2^256 and a = 0 or 2^-256 <= |a| < 2^256.
+CSC_DEV double fast_quot(double a, double b, double y) {
 #if defined(__CUDA_ARCH__)
-  const int ha = __double2hiint(a);
-  const double aa = fabs(a);
-  const double q0 = __dmul_rn(aa, y);
-  double r = __fma_rn(-b, q0, aa);
+  const double q0 = __dmul_rn(a, y);
+  double r = __fma_rn(-b, q0, a);
   const double q1 = __fma_rn(r, y, q0);
-  r = __fma_rn(-b, q1, aa);
-  const double q = __fma_rn(r, y, q1);
-  dc.acc |= a == 0.0 ? 0u : (unsigned)ha * 2u - kDivBase;
-  return __hiloint2double(__double2hiint(q) ^ (ha & (int)0x80000000), __double2loint(q));
+  r = __fma_rn(-b, q1, a);
+  return __fma_rn(r, y, q1);
 #else
   (void)y;
-#if defined(CLOUDSC_HOST_FORCE_REDO)
-  dc.acc = ~0u;
-#else
-  dc.acc |= a == 0.0 ? 0u : div_offset_host(a);
+  return a / b;
 #endif
+}
+// All ones exactly for a divisor with an all-ones significand.
+CSC_DEV unsigned ones_word(double b) { return (hi_word(b) | 0xfff00000u) & lo_word(b); }
+
+// The two halves as one self-contained division with its own checks (the
+// division and reciprocal check entries): an all-ones divisor's reciprocal
+// gets its low significand bit set (which gives RN(1/b) = 2^(-E-1)(1 + 2^-52);
+// a clamped shift of the all-ones test, no branch), a's sign is put back at
+// the end so that zero quotients have IEEE's sign, and operands outside the
+// windows 2^-256 <= |b| < 2^256, a = 0 or 2^-256 <= |a| < 2^256 are recorded.
+CSC_DEV double fast_rcp(double b, DivCheck &dc) {
+#if defined(__CUDA_ARCH__)
+  double y = fast_rcp_y(b);
+  y = __hiloint2double(__double2hiint(y), __double2loint(y) | (int)__funnelshift_rc(1u, 0u, ~ones_word(b)));
+  dc.acc |= hi_word(b) * 2u - kDivBase;
+  return y;
+#else
+  dc.acc |= hi_word(b) * 2u - kDivBase;
+  return 1.0 / b;
+#endif
+}
+CSC_DEV double fast_div(double a, double b, DivCheck &dc) {
+#if defined(__CUDA_ARCH__)
+  const double y = fast_rcp(b, dc);
+  const double q = fast_quot(fabs(a), b, y);
+  see(a, dc);
+  return __hiloint2double(__double2hiint(q) ^ (__double2hiint(a) & (int)0x80000000), __double2loint(q));
+#else
+  see(a, dc);
+  dc.acc |= hi_word(b) * 2u - kDivBase;
   return a / b;
 #endif
 }
 
-// a / b for a literal b (y = 1/b folded): fast_div_k when FAST and the
-// quotient is a double; IEEE otherwise.
-template <bool FAST, typename A>
+#if defined(CLOUDSC_HOST_WINDOW_CHECK) && !defined(__CUDA_ARCH__)
+// Test builds: count the operands of the fast pass outside the range its
+// operations are exact in, in columns that have not been reported.
+inline unsigned long long g_window_violations = 0;
+inline const DivCheck *g_column = nullptr;  // the checks of the column being run
+inline bool host_in(double x, int e) { return std::fabs(x) >= std::ldexp(1.0, -e) && std::fabs(x) < std::ldexp(1.0, e); }
+inline void host_count(bool ok) { g_window_violations += !ok && !(g_column && g_column->bad()); }
+inline void host_check_div(double a, double b) { host_count((a == 0.0 || host_in(a, 800)) && host_in(b, 400)); }
+inline void host_check_exp(double x) { host_count(std::fabs(x) < 700.0); }
+inline void host_check_log(double x) { host_count(x > 0.0 && host_in(x, 256)); }
+#else
+#define host_check_div(A, B)
+#define host_check_exp(X)
+#define host_check_log(X)
+#endif
+
+// Divisions of the column code.  In the fast pass (FAST) a double division is
+// fast_quot over fast_rcp_y; its operands need no check of their own, because
+// the level's input checks (cloudsc_body.cuh) bound them, except with CHK
+// (forms whose extra inputs are not among those), which records them.  A
+// divisor's all-ones significand is always recorded.  Otherwise IEEE.
+template <bool FAST, bool CHK, typename A, typename B>
+CSC_DEV auto cdiv(A a, B b, DivCheck &dc) -> decltype(a / b) {
+  typedef decltype(a / b) T;
+  if constexpr (FAST && std::is_same<T, double>::value) {
+    const double ad = double(a), bd = double(b);
+    if constexpr (CHK) {
+      see(ad, dc);
+      dc.acc |= hi_word(bd) * 2u - kDivBase;
+    }
+    const unsigned o = ones_word(bd);
+    dc.ones = dc.ones > o ? dc.ones : o;
+    host_check_div(ad, bd);
+    return fast_quot(ad, bd, fast_rcp_y(bd));
+  } else {
+    (void)dc;
+    return a / b;
+  }
+}
+// a / b given y = RN(1/b): a literal or parameter divisor (inside the window
+// and without an all-ones significand, so its folded or host-computed
+// reciprocal is exact), or one whose reciprocal several quotients share.
+template <bool FAST, bool CHK, typename A>
 CSC_DEV auto cdivk(A a, double b, double y, DivCheck &dc) -> decltype(a / A(b)) {
   typedef decltype(a / A(b)) T;
   if constexpr (FAST && std::is_same<T, double>::value) {
-    return fast_div_k(double(a), b, y, dc);
+    if constexpr (CHK) see(double(a), dc);
+    host_check_div(double(a), b);
+    return fast_quot(double(a), b, y);
   } else {
     (void)dc;
     (void)y;
     return a / A(b);
   }
 }
-
-// 1 / b: fast_rcp when FAST and b is a double; IEEE otherwise.
-template <bool FAST, typename B>
+// 1 / b.
+template <bool FAST, bool CHK, typename B>
 CSC_DEV B crcp(B b, DivCheck &dc) {
   if constexpr (FAST && std::is_same<B, double>::value) {
-    return fast_rcp(b, dc);
+    if constexpr (CHK) dc.acc |= hi_word(b) * 2u - kDivBase;
+    const unsigned o = ones_word(b);
+    dc.ones = dc.ones > o ? dc.ones : o;
+    host_check_div(1.0, b);
+    return fast_rcp_y(b);
   } else {
     (void)dc;
     return B(1) / b;
@@ -224,18 +247,6 @@ CSC_DEV B crcp(B b, DivCheck &dc) {
 // exact window; redo, the rerun with IEEE division of a column whose fast
 // pass recorded one.
 enum { kPassPlain = 0, kPassFast = 1, kPassRedo = 2 };
-
-// a / b, by fast_div when FAST and the quotient is a double; IEEE otherwise.
-template <bool FAST, typename A, typename B>
-CSC_DEV auto cdiv(A a, B b, DivCheck &dc) -> decltype(a / b) {
-  typedef decltype(a / b) T;
-  if constexpr (FAST && std::is_same<T, double>::value) {
-    return fast_div(double(a), double(b), dc);
-  } else {
-    (void)dc;
-    return a / b;
-  }
-}
 
 // Double precision uses the portable exp/pow of plibm.h (bit-identical on the
 // host and the GPU).
@@ -275,16 +286,27 @@ CSC_DEV float xpow(float x, float y) {
 
 // Transcendentals of the microphysics: FP64 (plibm) in the FP64 kernel,
 // FP32 (xexp/xpow above, on the argument rounded to float) in the FP32-mixed
-// kernel.  Everything else in both kernels is FP64.
-template <bool F32>
+// kernel.  Everything else in both kernels is FP64.  With WIN (the fast pass,
+// whose input checks bound the arguments) plibm's windowed forms: the same
+// bits without the range selects and special-value branches, each of which
+// ends a basic block.  Together with the unchecked divisions, FP64 at 262,144
+// columns 12.17 -> 10.12 ms, FP32-mixed 9.08 -> 8.27 ms, a CTA of 32 columns
+// alone on its SM 1.59 -> 1.41 ms.
+#if defined(CLOUDSC_HOST_LIBM_GLIBC) && !defined(__CUDA_ARCH__)
+#define CSC_GLIBC 1
+#else
+#define CSC_GLIBC 0
+#endif
+template <bool F32, bool WIN = false>
 CSC_DEV double mexp(double x) {
   if (F32) return (double)xexp((float)x);
+#if !CSC_GLIBC
+  if (WIN) {
+    host_check_exp(x);
+    return plibm_exp_win(x, 0.0, 0);
+  }
+#endif
   return xexp(x);
-}
-template <bool F32>
-CSC_DEV double mpow(double x, double y) {
-  if (F32) return (double)xpow((float)x, (float)y);
-  return xpow(x, y);
 }
 
 // A pow base whose logarithm several calls share (FP64: plibm's double-double
@@ -293,25 +315,42 @@ CSC_DEV double mpow(double x, double y) {
 struct PowBase {
   double x, lhi, llo;
 };
-template <bool F32>
+template <bool F32, bool WIN = false>
 CSC_DEV PowBase mbase(double x) {
   PowBase b;
   b.x = x;
   b.lhi = 0.0;
   b.llo = 0.0;
-#if !(defined(CLOUDSC_HOST_LIBM_GLIBC) && !defined(__CUDA_ARCH__))
-  if (!F32) plibm_log_base(x, &b.lhi, &b.llo);
+#if !CSC_GLIBC
+  if (!F32) {
+    if (WIN) {
+      host_check_log(x);
+      plibm_log_win(x, &b.lhi, &b.llo);
+    } else {
+      plibm_log_base(x, &b.lhi, &b.llo);
+    }
+  }
 #endif
   return b;
 }
-template <bool F32>
+template <bool F32, bool WIN = false>
 CSC_DEV double mpowb(const PowBase &b, double y) {
   if (F32) return (double)xpow((float)b.x, (float)y);
-#if defined(CLOUDSC_HOST_LIBM_GLIBC) && !defined(__CUDA_ARCH__)
+#if CSC_GLIBC
   return pow(b.x, y);
 #else
+  if (WIN) return plibm_pow_with_log_win(b.x, y, b.lhi, b.llo);
   return plibm_pow_with_log(b.x, y, b.lhi, b.llo);
 #endif
+}
+template <bool F32, bool WIN = false>
+CSC_DEV double mpow(double x, double y) {
+  if (F32) return (double)xpow((float)x, (float)y);
+#if !CSC_GLIBC
+  if (WIN && y == 3.0) return plibm_cube_win(x);
+  if (WIN && !plibm_pow_is_direct(y)) return mpowb<F32, WIN>(mbase<F32, WIN>(x), y);
+#endif
+  return xpow(x, y);
 }
 // pow with a parameter as exponent.  With GEN the host has checked that the
 // exponent is none of 0.5, 1.5, 2 and 3, in double and rounded to float
@@ -324,27 +363,21 @@ CSC_DEV float xpow_gen(float x, float y) {
   return powf(x, y);
 #endif
 }
-template <bool F32, bool GEN>
-CSC_DEV double mpowp(double x, double y) {
-  if (!GEN) return mpow<F32>(x, y);
-  if (F32) return (double)xpow_gen((float)x, (float)y);
-#if defined(CLOUDSC_HOST_LIBM_GLIBC) && !defined(__CUDA_ARCH__)
-  return pow(x, y);
-#else
-  double lhi, llo;
-  plibm_log_base(x, &lhi, &llo);
-  return plibm_pow_with_log_gen(x, y, lhi, llo);
-#endif
-}
-template <bool F32, bool GEN>
+template <bool F32, bool GEN, bool WIN = false>
 CSC_DEV double mpowbp(const PowBase &b, double y) {
-  if (!GEN) return mpowb<F32>(b, y);
+  if (!GEN) return mpowb<F32, WIN>(b, y);
   if (F32) return (double)xpow_gen((float)b.x, (float)y);
-#if defined(CLOUDSC_HOST_LIBM_GLIBC) && !defined(__CUDA_ARCH__)
+#if CSC_GLIBC
   return pow(b.x, y);
 #else
+  if (WIN) return plibm_pow_log_win(b.lhi, b.llo, y);
   return plibm_pow_with_log_gen(b.x, y, b.lhi, b.llo);
 #endif
+}
+template <bool F32, bool GEN, bool WIN = false>
+CSC_DEV double mpowp(double x, double y) {
+  if (!GEN && !WIN) return mpow<F32>(x, y);
+  return mpowbp<F32, GEN, WIN>(mbase<F32, WIN>(x), y);
 }
 CSC_DEV double xsqrt(double x) { return sqrt(x); }
 CSC_DEV float xsqrt(float x) { return sqrtf(x); }

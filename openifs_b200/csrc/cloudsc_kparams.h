@@ -6,6 +6,62 @@
 
 namespace cloudsc {
 
+// Whether the parameters lie inside the ranges the column code's fast pass
+// assumes (its input checks bound the fields, these the parameters): positive
+// divisors and pow bases of moderate size, exponents small enough that
+// |y ln x| < 700 for every base x the checks allow, saturation constants that
+// keep T - R4xES and 1 - RETV q away from zero for T in [128, 1024) K.  The
+// defaults lie well inside; with any other value every column takes the
+// rerun with IEEE division and plibm's full functions.
+inline bool fast_pass_params_ok(const cloudsc_params &p) {
+  bool ok = true;
+  auto in = [&ok](double x, double lo, double hi) { ok = ok && x >= lo && x <= hi; };
+  // positive scale factors, divisors and thresholds
+  const double pos[] = {p.rg, p.rd, p.rv, p.rcpd, p.rtt, p.rlvtt, p.rlstt, p.r2es, p.r5les, p.r5ies, p.r5alvcp,
+                        p.r5alscp, p.ralvdcp, p.ralsdcp, p.ramin, p.rlmin, p.rcovpmin, p.rvrfactor, p.rtaumel,
+                        p.rlcritsnow, p.rxfallspeedrain, p.rdepliqrefdepth, p.riceinit, p.rdensref, p.rdenswat,
+                        p.rcl_kkaac, p.rcl_kkaau, p.rcl_x1r, p.rcl_lam1r, p.rcl_const1r, p.rcl_const2r,
+                        p.rcl_const5r, p.rcl_const7r, p.rcl_cdenom1, p.rcl_cdenom2, p.rcl_cdenom3, p.rcl_x1s,
+                        p.rcl_lam1s, p.rcl_const1s, p.rcl_const2s, p.rcl_const3s, p.rcl_const6s, p.rcl_const7s,
+                        p.rcl_apb1, p.rcl_apb2, p.rcl_apb3};
+  for (double x : pos) in(x, 1e-14, 1e14);
+  // factors that may be zero
+  const double fac[] = {p.rcldiff, p.rcldiff_convi, p.ramid, p.rprecrhmax, p.rpecons, p.rssicefactor, p.rsnowlin1,
+                        p.rvice, p.rvsnow, p.rdepliqrefrate, p.rcl_overlapliqice, p.rcl_effrime, p.rcl_inhomogaut,
+                        p.rcl_inhomogacc, p.rmfadvw, p.rmfadvwdd, p.rcl_kk_cloud_num_land, p.rcl_kk_cloud_num_sea};
+  for (double x : fac)
+    if (x != 0.0) in(x, 1e-14, 1e14);
+  // exponents
+  const double ex[] = {p.rcl_kkbac, p.rcl_kkbauq, p.rcl_kkbac - 1.0, p.rcl_kkbauq - 1.0, p.rcl_dr, p.rcl_x2r,
+                       p.rcl_const6r, p.rcl_const4s, p.rcl_const5s, p.rcl_const8s};
+  for (double x : ex) in(x < 0.0 ? -x : x, 1e-3, 5.0);
+  in(p.rcl_const3r, -2.0, 2.0);
+  in(p.rcl_const4r, -2.0, 2.0);
+  in(p.rcl_x2r, 0.1, 3.0);
+  // the slopes (LAM1/(RHO q))**LAM2: below 1e22
+  in(p.rcl_lam1r, 1.0, 1e8);
+  in(p.rcl_lam1s, 1.0, 1e8);
+  in(p.rcl_lam2r, 0.1, 0.7);
+  in(p.rcl_lam2s, 0.1, 0.7);
+  in(p.rtt, 200.0, 400.0);
+  in(p.retv, 0.0, 1.0);
+  in(p.r3les, 1.0, 40.0);
+  in(p.r3ies, 1.0, 40.0);
+  in(p.r4les, -60.0, 60.0);
+  in(p.r4ies, -60.0, 60.0);
+  in(p.rtice, 100.0, p.rtwat);
+  in(p.rtwat, p.rtice, 400.0);
+  in(p.rkoop1, 0.0, 100.0);
+  in(p.rkoop2, 0.0, 1.0);
+  in(p.rsnowlin2, 0.0, 0.5);
+  in(p.rcl_fzrab, -1.0, 1.0);
+  // the differences of the evaporation and deposition denominators positive
+  // over the temperatures they are used at
+  ok = ok && p.rcl_cdenom1 > 1.001 * 1024.0 * p.rcl_cdenom2 && p.rcl_apb1 > 1.001 * p.rtt * p.rcl_apb2 &&
+       p.rlstt > 2.0 * p.rv * p.rtt;
+  return ok;
+}
+
 template <typename Real>
 inline void fill_kparams(const cloudsc_params &p, const Derived &d, KParams<Real> &k) {
 #define F_(n) k.n = Real(p.n)
@@ -66,9 +122,9 @@ inline void fill_kparams(const cloudsc_params &p, const Derived &d, KParams<Real
   // RV/RD with the division the kernels would perform (IEEE, in Real)
   k.rv_rd = Real(p.rv) / Real(p.rd);
   // 1/b correctly rounded (IEEE on the host) for each parameter divisor;
-  // usable by fast_div_k only inside its window and without an all-ones
-  // significand (the conditions of fast_div)
-  bool ok = true;
+  // usable by cdivk only inside its window and without an all-ones
+  // significand
+  bool ok = fast_pass_params_ok(p);
   auto rcp = [&ok](double b) {
     uint64_t u;
     std::memcpy(&u, &b, 8);

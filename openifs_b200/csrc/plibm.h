@@ -310,6 +310,103 @@ PLIBM_FN_COLD double plibm_pow_special(double x, double y, double res) {
   return y != y ? y : res;
 }
 
+/* ------------------------------------------------------------------------
+ * Windowed forms: the same bits as the functions above for arguments inside a
+ * stated window, without the selects, branches and scalings that only other
+ * arguments need.  The column kernels' fast pass uses them where the level's
+ * input checks place the arguments in the window (cloudsc_column.cuh).
+ * ------------------------------------------------------------------------ */
+
+/* exp(hi + lo) for |hi| < 700: no clamp and no NaN select; the result is
+ * normal, so 2^m goes straight into the exponent field (the same bits as the
+ * two exact factors). */
+PLIBM_FN double plibm_exp_win(double hi, double lo, int use_lo) {
+  double kd = plibm_fma(hi, PLIBM_INV_LN2_128, PLIBM_SHIFT);
+  int k = (int)(uint32_t)plibm_bits(kd); /* |k| < 2^31: the low word, as two's complement */
+  kd = kd - PLIBM_SHIFT;
+  double r = plibm_fma(-kd, PLIBM_LN2_128_HI, hi);
+  r = plibm_fma(-kd, PLIBM_LN2_128_LO, r);
+  if (use_lo) r = r + lo;
+  int j = k & 127;
+  double thi = plibm_exp_t(2 * j), tlo = plibm_exp_t(2 * j + 1);
+  double p = plibm_fma(r, 0x1.1111111111111p-7, 0x1.5555555555555p-5); /* 1/120, 1/24 */
+  p = plibm_fma(p, r, 0x1.5555555555555p-3);                          /* 1/6 */
+  p = plibm_fma(p, r, 0x1.0000000000000p-1);                          /* 1/2 */
+  p = plibm_fma(p, r * r, r);                                         /* expm1(r) */
+  double s = plibm_fma(thi, p, tlo);
+  double e = thi + s;
+#if defined(__CUDA_ARCH__)
+  return __hiloint2double(__double2hiint(e) + ((k & ~127) << 13), __double2loint(e));
+#else
+  return plibm_from_bits(plibm_bits(e) + ((uint64_t)(int64_t)(k >> 7) << 52));
+#endif
+}
+
+/* ln(x) as hi + lo for normal x > 0: plibm_log_dd without its subnormal
+ * test.  The exponent is converted by placing it in the low word of 2^52 and
+ * subtracting (exact), not by the conversion unit. */
+PLIBM_FN void plibm_log_win(double x, double *hi, double *lo) {
+#if defined(__CUDA_ARCH__)
+  const unsigned h32 = (unsigned)__double2hiint(x);
+  int j = (int)((h32 >> 13) & 127u);
+  double m = __hiloint2double((int)((h32 & 0xfffffu) | 0x3ff00000u), __double2loint(x));
+  double ed = __hiloint2double(0x43300000, (int)(h32 >> 20)) - (0x1p52 + 1023.0);
+#else
+  uint64_t u = plibm_bits(x);
+  uint64_t mant = u & 0xfffffffffffffULL;
+  int j = (int)(mant >> 45);
+  double m = plibm_from_bits(mant | 0x3ff0000000000000ULL);
+  double ed = (double)((int)(u >> 52) - 1023);
+#endif
+  double invc = plibm_log_t(3 * j), lchi = plibm_log_t(3 * j + 1), lclo = plibm_log_t(3 * j + 2);
+  double p = m * invc;
+  double perr = plibm_fma(m, invc, -p); /* m*invc = p + perr exactly */
+  double r1 = p - 1.0;                  /* exact */
+  double q = plibm_fma(r1, 0x1.2492492492492p-3, -0x1.5555555555555p-3); /* 1/7, -1/6 */
+  q = plibm_fma(q, r1, 0x1.999999999999ap-3);                           /* 1/5 */
+  q = plibm_fma(q, r1, -0x1.0000000000000p-2);                          /* -1/4 */
+  q = plibm_fma(q, r1, 0x1.5555555555555p-2);                           /* 1/3 */
+  q = plibm_fma(q, r1, -0x1.0000000000000p-1);                          /* -1/2 */
+  double poly = q * (r1 * r1);
+  double corr = plibm_fma(-perr, r1, perr);
+  double a = ed * PLIBM_LN2_HI42; /* exact */
+  double s1 = a + lchi;
+  double err1 = lchi - (s1 - a);
+  double s2 = s1 + r1; /* two-sum */
+  double b2 = s2 - s1;
+  double err2 = (s1 - (s2 - b2)) + (r1 - b2);
+  double low = ((err1 + err2) + (lclo + ed * PLIBM_LN2_LO42)) + (corr + poly);
+  double h = s2 + low;
+  *lo = low - (h - s2);
+  *hi = h;
+}
+
+/* x^y given plibm_log_win(x) = lhi + llo, |y ln x| < 700, y none of 0, 0.5,
+ * 1.5, 2 and 3. */
+PLIBM_FN double plibm_pow_log_win(double lhi, double llo, double y) {
+  double t_hi = y * lhi;
+  double t_lo = plibm_fma(y, lhi, -t_hi) + y * llo;
+  return plibm_exp_win(t_hi, t_lo, 1);
+}
+
+/* The same for any finite nonzero y. */
+PLIBM_FN double plibm_pow_with_log_win(double x, double y, double lhi, double llo) {
+  if (y == 0.5) return plibm_sqrt(x);
+  if (y == 1.5) return plibm_pow1p5(x);
+  if (y == 2.0) return x * x;
+  if (y == 3.0) return plibm_cube(x);
+  return plibm_pow_log_win(lhi, llo, y);
+}
+
+/* x^3 for 1e-90 < |x| < 1e90 (plibm_cube without its range test). */
+PLIBM_FN double plibm_cube_win(double x) {
+  double h = x * x;
+  double l = plibm_fma(x, x, -h);
+  double p = h * x;
+  double pe = plibm_fma(h, x, -p);
+  return p + (pe + l * x);
+}
+
 /* True when pow(x, y) does not need ln x (an exact-operation exponent). */
 PLIBM_FN int plibm_pow_is_direct(double y) { return y == 0.5 || y == 1.5 || y == 2.0 || y == 3.0; }
 

@@ -186,6 +186,12 @@ extern "C" int hostemu_sltend_batched(const cloudsc_params *p, int nproma, int k
   return 0;
 }
 
+#if defined(CLOUDSC_HOST_WINDOW_CHECK)
+// operands of the fast pass so far outside the windows its operations are
+// exact in, in columns its input checks had not reported
+extern "C" unsigned long long hostemu_window_violations() { return g_window_violations; }
+#endif
+
 // The kernels' forms 3-5 on one column: the plain column code, or (FD) the
 // fast pass and, for a column it reported, the rerun, the two passes
 // splitting PEXTRA's levels as the kernels do.

@@ -76,10 +76,10 @@ def run_hostemu(p, arrs, nproma, ngpblks, ngptot, precision=0, libm="plibm", kle
     import ctypes
     import os
     here = os.path.join(os.path.dirname(os.path.abspath(__file__)), "hostemu")
-    # "redo": every fast division of a FASTDIV column reports bad, so each
-    # level also runs its IEEE-division pass
+    # "redo": every column of the fast pass reports and runs again with IEEE
+    # division; "window": counts operands outside the fast pass's windows
     name = {"plibm": "libcloudsc_hostemu.so", "glibc": "libcloudsc_hostemu_glibc.so",
-            "redo": "libcloudsc_hostemu_redo.so"}[libm]
+            "redo": "libcloudsc_hostemu_redo.so", "window": "libcloudsc_hostemu_window.so"}[libm]
     path = os.path.join(here, name)
     if not os.path.exists(path):
         import subprocess
@@ -90,6 +90,9 @@ def run_hostemu(p, arrs, nproma, ngpblks, ngptot, precision=0, libm="plibm", kle
         *[out[n].ctypes.data for n, *_ in fields.BATCHED_FIELDS])
     nw = L.hostemu_batched(ctypes.byref(p), int(nproma), int(klev), int(ngpblks), int(ngptot),
                            ctypes.c_double(PTSPHY), ptrs, int(precision))
+    if libm == "window":
+        L.hostemu_window_violations.restype = ctypes.c_ulonglong
+        return out, nw, L.hostemu_window_violations()
     return out, nw
 
 
