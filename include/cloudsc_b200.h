@@ -602,6 +602,17 @@ int cloudsc_b200_division_check(const double *a, const double *b, int64_t n, dou
  */
 int cloudsc_b200_reciprocal_check(const double *b, int64_t n, double *y, int32_t *bad, void *stream);
 
+/*
+ * The column kernels' square root on n values (a self-check, no reference
+ * counterpart): where bad[i] = 0, y[i] = IEEE sqrt(x[i]) bit for bit; the
+ * columns whose root cannot be confirmed (bad[i] = 1: the rounding check
+ * failed or the significand of x[i] is all ones) run again with IEEE
+ * operations.  x inside 2^-200 <= x < 2^200 or not positive.  Device
+ * pointers; stream may be NULL.  CLOUDSC_E_SHAPE for n < 0, CLOUDSC_E_NULL for
+ * a NULL array with n > 0.
+ */
+int cloudsc_b200_sqrt_check(const double *x, int64_t n, double *y, int32_t *bad, void *stream);
+
 /* Last CUDA error string recorded by this library on the calling thread. */
 const char *cloudsc_b200_last_error(void);
 

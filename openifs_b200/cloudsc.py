@@ -87,6 +87,8 @@ def lib():
         L.cloudsc_b200_division_check.restype = ctypes.c_int
         L.cloudsc_b200_reciprocal_check.argtypes = [vp, ctypes.c_int64, vp, vp, vp]
         L.cloudsc_b200_reciprocal_check.restype = ctypes.c_int
+        L.cloudsc_b200_sqrt_check.argtypes = [vp, ctypes.c_int64, vp, vp, vp]
+        L.cloudsc_b200_sqrt_check.restype = ctypes.c_int
         L.cloudsc_b200_last_error.restype = ctypes.c_char_p
         L.cloudsc_b200_version.restype = ctypes.c_char_p
         L.cloudsc_b200_params_size.restype = ctypes.c_size_t
@@ -474,4 +476,19 @@ def reciprocal_check(b, stream=None):
     bad = torch.empty(b.shape, dtype=torch.int32, device=b.device)
     st = stream.cuda_stream if stream is not None else None
     _check(lib().cloudsc_b200_reciprocal_check(_ptr(b), b.numel(), _ptr(y), _ptr(bad), st))
+    return y, bad
+
+
+def sqrt_check(x, stream=None):
+    """The column kernels' square root on a float64 CUDA tensor: returns
+    (y, bad), the roots and an int32 flag, 1 where the kernels would run the
+    column again; elsewhere y equals IEEE sqrt(x) bit for bit."""
+    import torch
+    if x.dtype != torch.float64 or not x.is_cuda:
+        raise CloudscError(-2, "sqrt_check wants a float64 CUDA tensor")
+    x = x.contiguous()
+    y = torch.empty_like(x)
+    bad = torch.empty(x.shape, dtype=torch.int32, device=x.device)
+    st = stream.cuda_stream if stream is not None else None
+    _check(lib().cloudsc_b200_sqrt_check(_ptr(x), x.numel(), _ptr(y), _ptr(bad), st))
     return y, bad

@@ -13,6 +13,20 @@
 #ifndef CSC_LEVEL_SYNC
 #define CSC_LEVEL_SYNC()
 #endif
+// Hides how an offset was computed, so that the compiler keeps the few offsets
+// of a level and not a running pointer per array.
+#ifndef CSC_OPAQUE
+#define CSC_OPAQUE(X)
+#endif
+// L2 prefetch of the next level's inputs (nothing on the host).
+#ifndef CSC_PREFETCH
+#define CSC_PREFETCH_SETUP()
+#define CSC_PREFETCH(C, OFF)
+#endif
+// Whether any column of the warp has C (the column alone on the host).
+#ifndef CSC_ANY
+#define CSC_ANY(C) (C)
+#endif
 
 // Every division of the column code: the branch-free division when FAST_ (the
 // fast pass; with CHK_ recording its operands in divbad_), IEEE division
@@ -75,13 +89,7 @@ CSC_DEV double sink_sum(int jo, const QA &q) {
   }
 #define SCL1(F, A) \
   if (F) A = A * zr;
-template <bool FAST_, bool CHK_>
-CSC_DEV void scale_row(int jo, QA &q, const double qx[5], DivCheck &divbad_) {
-  const double zepsec = 1.E-14;
-  const double ss = sink_sum(jo, q);
-  const double zmm = mx(qx[jo], zepsec);
-  if (!(ss > zmm)) return;
-  const double zr = DIV(zmm, ss);
+CSC_DEV void scale_entries(int jo, QA &q, double zr) {
   switch (jo) {
     case L: {
       bool fLL = q.LL < 0.0, fLI = q.LI < 0.0, fLV = q.LV < 0.0;
@@ -105,8 +113,82 @@ CSC_DEV void scale_row(int jo, QA &q, const double qx[5], DivCheck &divbad_) {
     } break;
   }
 }
+template <bool FAST_, bool CHK_>
+CSC_DEV void scale_row(int jo, QA &q, const double qx[5], DivCheck &divbad_) {
+  const double zepsec = 1.E-14;
+  const double ss = sink_sum(jo, q);
+  const double zmm = mx(qx[jo], zepsec);
+  if (!(ss > zmm)) return;
+  scale_entries(jo, q, DIV(zmm, ss));
+}
 #undef SCL1
 #undef SCL2
+
+// The sink truncation of one column (cloudsc.F90:3455-3536): the rows rescaled
+// in the order of their ratios ZMM/MAX(ZSINKSUM,ZMM), ties in species order.
+// Only a row whose sinks exceed its amount has a ratio below 1; the other
+// rows' ratios are all exactly 1, so they come last, in species order, and
+// need no division.  Rows below 1 (none for most points, rarely more than
+// one) are taken smallest ratio first; their ratios are formed only where a
+// column of the warp has two of them to order.  The same rows are rescaled by
+// the same factors in the same order as with the full sort.
+template <bool CHK_>
+CSC_DEV void truncate_sinks(QA &q, const double qx[5], DivCheck &divbad_) {
+  constexpr bool FAST_ = true;
+  const double zepsec = 1.E-14;
+  double z[5], ss[5];
+  unsigned over = 0u;
+#pragma unroll
+  for (int jm = 0; jm < 5; ++jm) {
+    z[jm] = mx(qx[jm], zepsec);
+    ss[jm] = sink_sum(jm, q);
+    over |= ss[jm] > z[jm] ? 1u << jm : 0u;
+  }
+  if (!CSC_ANY(over != 0u)) return;
+  unsigned order = 0u;  // the species of the rows below 1, 3 bits each, first row lowest
+  {
+    const bool several = (over & (over - 1u)) != 0u;
+    if (CSC_ANY(several)) {
+      double r[5];
+#pragma unroll
+      for (int jm = 0; jm < 5; ++jm) r[jm] = DIV(z[jm], mx(ss[jm], z[jm]));
+      // a row's place: how many come before it (a smaller ratio, or an equal
+      // one of a lower species)
+      unsigned place[5] = {0u, 0u, 0u, 0u, 0u};
+#pragma unroll
+      for (int jm = 1; jm < 5; ++jm)
+#pragma unroll
+        for (int jn = 0; jn < jm; ++jn) {
+          const bool before = r[jn] <= r[jm];
+          place[jm] += before ? 3u : 0u;
+          place[jn] += before ? 0u : 3u;
+        }
+#pragma unroll
+      for (int jm = 0; jm < 5; ++jm) order |= (unsigned)jm << place[jm];
+    } else {
+#pragma unroll
+      for (int jm = 1; jm < 5; ++jm) order = (over >> jm) & 1u ? (unsigned)jm : order;
+    }
+  }
+  unsigned left = over;
+#pragma unroll 1
+  while (CSC_ANY(left != 0u)) {
+    if (left != 0u) {
+      const int jo = (int)(order & 7u);
+      order >>= 3;
+      left &= ~(1u << jo);
+      scale_row<FAST_, CHK_>(jo, q, qx, divbad_);
+    }
+  }
+#pragma unroll
+  for (int jm = 0; jm < 5; ++jm) {
+    const double s = sink_sum(jm, q);
+    const bool c = !((over >> jm) & 1u) && s > z[jm];
+    if (CSC_ANY(c)) {
+      if (c) scale_entries(jm, q, DIV(z[jm], s));
+    }
+  }
+}
 
 // ZRATIO for every species from the current ZSOLQA (cloudsc.F90:3455-3474).
 template <bool FAST_, bool CHK_>
@@ -349,6 +431,47 @@ CSC_DEV void write_budgets(const Fields &F, const KParams<Real> &P, const double
 }
 
 // ---------------------------------------------------------------------------
+// A value that waits long between its uses: a register (PARK = 0), or slot I
+// of the thread's own column of shared memory, PARK threads wide (the CTA's
+// compiled maximum), so that a warp's accesses are conflict-free.  The level
+// code keeps about 50 such values alive -- the state carried down the column,
+// the level's inputs and sources its last lines need again -- which is more
+// than the registers of 12 or more warps per SM hold; left to the compiler
+// they are spilled to local memory, whose lines the level's loads and stores
+// push out of L1.
+// ---------------------------------------------------------------------------
+constexpr int kParkSlots = 54;
+template <typename T, int PARK, int I>
+struct Parked {
+#if defined(__CUDA_ARCH__)
+  CSC_DEV static unsigned addr() { return park_base() + (unsigned)(I * PARK * 8); }
+  T v;
+  CSC_DEV explicit Parked(T x) { set(x); }
+  CSC_DEV void set(T x) {
+    if constexpr (PARK > 0) {
+      asm volatile("st.shared.f64 [%0], %1;" ::"r"(addr()), "d"((double)x));
+    } else {
+      v = x;
+    }
+  }
+  CSC_DEV T get() const {
+    if constexpr (PARK > 0) {
+      double x;
+      asm volatile("ld.shared.f64 %0, [%1];" : "=d"(x) : "r"(addr()));
+      return (T)x;
+    } else {
+      return v;
+    }
+  }
+#else
+  T v;
+  explicit Parked(T x) : v(x) {}
+  void set(T x) { v = x; }
+  T get() const { return v; }
+#endif
+};
+
+// ---------------------------------------------------------------------------
 // The column body.
 // ---------------------------------------------------------------------------
 // `active` false: the thread only keeps a CTA's per-level barrier company
@@ -383,7 +506,7 @@ CSC_DEV void write_budgets(const Fields &F, const KParams<Real> &P, const double
 // levels from *kbud on.  Every slot then receives IEEE's terms once each, in
 // level order, as in one IEEE run.
 template <typename Real, bool F32M, bool BUD = false, bool OPT = false, typename FT = Fields, bool GEN = false,
-          int PASS = kPassPlain>
+          int PASS = kPassPlain, int PARK = 0>
 CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool active = true, bool *bad = nullptr,
                             double *plude_in = nullptr, int *kbud = nullptr) {
   const KParams<Real> &P = KP<Real>();
@@ -394,7 +517,14 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
   // the optional forms' factors and inputs are not among the level's input
   // checks: their divisions check their own operands
   constexpr bool CHK_ = OPT;
+  // PARK < 0: the build with registers to spare, where the processes of a
+  // group form one block; otherwise each sits behind its own vote
+  constexpr bool WIDE = PARK < 0;
   DivCheck divbad_;
+  const auto root = [&](Real x) -> Real {
+    if constexpr (std::is_same<Real, double>::value) return csqrt<FAST_>(x, divbad_);
+    else return xsqrt(x);
+  };
   if constexpr (FAST_) {
     if (P.rcp_force) divbad_.acc = ~0u;  // a parameter outside the fast pass's ranges: rerun
 #if defined(CLOUDSC_HOST_WINDOW_CHECK) && !defined(__CUDA_ARCH__)
@@ -417,10 +547,10 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
   const Real zrdtgdp_f = C(1.0) / (rdt * P.rg);
 
   // per-column inputs
-  const Real plsm = Real(ld(F.plsm + o1));
+  const bool land = Real(ld(F.plsm + o1)) > C(0.5);
   const bool ldcum = ld(F.ldcum + o1) != 0;
   const int ktype = ld(F.ktype + o1);
-  const Real peis = Real(ld(F.peis + o1));
+  const bool shallow = ktype >= 2 && Real(ld(F.peis + o1)) < C(10.0);
   const D paph_surf = ld(F.paph + o2h + (size_t)klev * np);
   // reciprocals of the column's constant divisors (time step, surface
   // pressure), taken once
@@ -429,12 +559,10 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
     see_pos(dt, -10, divbad_);
     see_pos(paph_surf, -8, divbad_);
   }
-  Real zadvw = C(1.0), zadvwd = C(1.0);
-  if (ktype == 1 && P.rmfadvw > C(0.0)) {
-    zadvw = C(1.0) - P.rmfadvw;
-    zadvwd = C(1.0) - P.rmfadvw * P.rmfadvwdd;
-  }
-  const Real zconstpow = plsm > C(0.5) ? P.zconst_pow_land : P.zconst_pow_sea;
+  // mass-flux factors of the vertical advection (ZADVW, ZADVWD)
+  const bool advw = ktype == 1 && P.rmfadvw > C(0.0);
+#define ZADVW (advw ? C(1.0) - P.rmfadvw : C(1.0))
+#define ZADVWD (advw ? C(1.0) - P.rmfadvw * P.rmfadvwdd : C(1.0))
 
   // SPP: the factors EXP(MU + XMAG*PGP2DSPP(JL,MP)) of this column, one per
   // perturbation (CLOUDINHOM: two, fields MP and MP+1); grid-box length and
@@ -460,15 +588,35 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
   }
 
   // state carried between levels
+  // (Parked: in shared memory between uses when PARK, see there)
   D paph_k = ld(F.paph + o2h);
-  Real pmfu_k = Real(ld(F.pmfu + o2)), pmfd_k = Real(ld(F.pmfd + o2));
-  Real za_prev = C(0.0), qr_prev = C(0.0), qs_prev = C(0.0), t_prev = C(0.0), pap_prev = C(0.0);
-  Real qxnm1_l = C(0.0), qxnm1_i = C(0.0), qxnm1_r = C(0.0), qxnm1_s = C(0.0);
-  Real zanewm1 = C(0.0), zcovptot = C(0.0), zcovpmax = C(0.0), zcldtopdist = C(0.0);
+  Parked<Real, PARK, 0> p_pmfu(Real(ld(F.pmfu + o2)));
+  Parked<Real, PARK, 1> p_pmfd(Real(ld(F.pmfd + o2)));
+  Parked<Real, PARK, 2> p_za(C(0.0));
+  Parked<Real, PARK, 3> p_qr(C(0.0));
+  Parked<Real, PARK, 4> p_qs(C(0.0));
+  Parked<Real, PARK, 5> p_t(C(0.0));
+  Parked<Real, PARK, 6> p_pap(C(0.0));
+  Parked<Real, PARK, 7> p_xl(C(0.0));  // ZQXNM1
+  Parked<Real, PARK, 8> p_xi(C(0.0));
+  Parked<Real, PARK, 9> p_xr(C(0.0));
+  Parked<Real, PARK, 10> p_anew(C(0.0));
+  Parked<Real, PARK, 11> p_cov(C(0.0));
+  Parked<Real, PARK, 12> p_covmax(C(0.0));
+  Parked<Real, PARK, 13> p_ctd(C(0.0));
+  Parked<Real, PARK, 14> p_frac(C(0.0));
+  Parked<Real, PARK, 15> p_fli(C(0.0));  // ZPFPLSX(JK)
+  Parked<Real, PARK, 16> p_flr(C(0.0));
+  Parked<Real, PARK, 17> p_fls(C(0.0));
+  Parked<D, PARK, 18> p_fsqlf(0.0);
+  Parked<D, PARK, 19> p_fsqif(0.0);
+  Parked<D, PARK, 20> p_fcqlng(0.0);
+  Parked<D, PARK, 21> p_fcqnng(0.0);
+  Parked<D, PARK, 22> p_fsqltur(0.0);
+  Parked<D, PARK, 23> p_fsqitur(0.0);
+  Parked<Real, PARK, 24> p_rpsurf(rpsurf);
+  Parked<D, PARK, 25> p_psurf(paph_surf);
   bool llrainliq = true;
-  Real prainfrac = C(0.0);
-  Real pfplsx_i = C(0.0), pfplsx_r = C(0.0), pfplsx_s = C(0.0);  // ZPFPLSX(JK)
-  D fsqlf = 0.0, fsqif = 0.0, fcqlng = 0.0, fcqnng = 0.0, fsqltur = 0.0, fsqitur = 0.0;
   unsigned nwarn = 0;
   // first level whose budget terms the fast pass leaves to the redo pass
   int kbud_l = klev;
@@ -483,9 +631,17 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
 
   // (KLON,KLEV,N) arrays: the block stride is N*KLON*KLEV, species m at +m*KLON*KLEV
   const size_t o5 = (size_t)ib * 5 * s2 + jl, o4 = (size_t)ib * 4 * s2 + jl, o2s = (size_t)ib * 2 * s2 + jl;
+  // this lane's share of the warp's input lines
+  CSC_PREFETCH_SETUP();
   for (int k = 0; k < klev; ++k) {
-    const size_t ok = o2 + (size_t)k * np;
-    const size_t ok5 = o5 + (size_t)k * np, ok4 = o4 + (size_t)k * np, ok2s = o2s + (size_t)k * np;
+    size_t ok = o2 + (size_t)k * np;
+    size_t ok5 = o5 + (size_t)k * np, ok4 = o4 + (size_t)k * np, ok2s = o2s + (size_t)k * np;
+    size_t oh = o2h + (size_t)k * np;
+    CSC_OPAQUE(ok);
+    CSC_OPAQUE(ok5);
+    CSC_OPAQUE(ok4);
+    CSC_OPAQUE(ok2s);
+    CSC_OPAQUE(oh);
     // ---------------- loads for level k ----------------
     const D pt_k = ld(F.pt + ok), pq_k = ld(F.pq + ok), pa_k = ld(F.pa + ok);
     const D cml_t = ld(F.cml_t + ok), cml_q = ld(F.cml_q + ok), cml_a = ld(F.cml_a + ok);
@@ -494,7 +650,7 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
     const D pc_l = ld(F.pclv + ok5), pc_i = ld(F.pclv + ok5 + s2), pc_r = ld(F.pclv + ok5 + 2 * s2),
             pc_s = ld(F.pclv + ok5 + 3 * s2);
     const D pap_kd = ld(F.pap + ok);
-    const D paph_k1 = ld(F.paph + o2h + (size_t)(k + 1) * np);
+    const D paph_k1 = ld(F.paph + oh + np);
     const D pvfl = ld(F.pvfl + ok), pvfi = ld(F.pvfi + ok);
     const D pludeli1 = ld(F.pludeli + ok4), pludeli2 = ld(F.pludeli + ok4 + s2);
     const bool last = (k == klev - 1);
@@ -514,6 +670,16 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
       if constexpr (PASS == kPassFast) plude_in[k] = plude_k;
     }
     const Real pap_k = Real(pap_kd);
+    Parked<D, PARK, 26> p_pt(pt_k);
+    Parked<D, PARK, 27> p_pq(pq_k);
+    Parked<D, PARK, 28> p_pa(pa_k);
+    Parked<D, PARK, 29> p_ct(cml_t);
+    Parked<D, PARK, 30> p_cq(cml_q);
+    Parked<D, PARK, 31> p_ca(cml_a);
+    Parked<D, PARK, 32> p_dl(pludeli1);
+    Parked<D, PARK, 33> p_di(pludeli2);
+    Parked<D, PARK, 52> p_vfl(pvfl);
+    Parked<D, PARK, 53> p_vfi(pvfi);
 
     // ---------------- first guess (:982-1002) ----------------
     // The state is kept in double in both kernels (tendencies are small
@@ -522,9 +688,12 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
     D qvD = pq_k + dt * cml_q;
     D aD = pa_k + dt * cml_a;
     const D aorig = aD;
-    const D q0_l = pc_l + dt * cl_l, q0_i = pc_i + dt * cl_i, q0_r = pc_r + dt * cl_r,
-            q0_s = pc_s + dt * cl_s;
-    D qlD = q0_l, qiD = q0_i, qrD = q0_r, qsD = q0_s;
+    D qlD = pc_l + dt * cl_l, qiD = pc_i + dt * cl_i, qrD = pc_r + dt * cl_r, qsD = pc_s + dt * cl_s;
+    Parked<D, PARK, 34> p_q0l(qlD);
+    Parked<D, PARK, 35> p_q0i(qiD);
+    Parked<D, PARK, 36> p_q0r(qrD);
+    Parked<D, PARK, 37> p_q0s(qsD);
+    Parked<D, PARK, 38> p_aorig(aorig);
     const Real t = Real(tD);
 
     // ---------------- saturation (:1087-1115) ----------------
@@ -623,6 +792,12 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
     TIDY(qsD, lneg_s, ralsdcp)
 #undef TIDY
     aD = mx(0.0, mn(1.0, aD));
+    Parked<D, PARK, 39> p_negl(lneg_l);
+    Parked<D, PARK, 40> p_negi(lneg_i);
+    Parked<D, PARK, 41> p_negr(lneg_r);
+    Parked<D, PARK, 42> p_negs(lneg_s);
+    Parked<D, PARK, 43> p_loct(loc_t);
+    Parked<D, PARK, 44> p_locq(loc_q);
     if constexpr (FAST_) {
       if (k >= ncldtop0) {
         see(qvD, divbad_);
@@ -640,9 +815,11 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
     const Real ql = Real(qlD), qi = Real(qiD), qr = Real(qrD), qs = Real(qsD);
     const Real zli = ql + qi;
     Real liqfrac = C(0.0), icefrac = C(0.0);
-    if (zli > P.rlmin) {
-      liqfrac = DIV(ql, zli);
-      icefrac = C(1.0) - liqfrac;
+    {
+      const bool c = zli > P.rlmin;
+      const Real f = DIV(ql, c ? zli : C(1.0));
+      liqfrac = c ? f : C(0.0);
+      icefrac = c ? C(1.0) - f : C(0.0);
     }
 
     // FSD bookkeeping of this level (ZLFSD, ZANEWP, ZRATFSD, ZICEF, ZLIQF;
@@ -743,20 +920,21 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
       // 3.2 detrainment (:1362-1398)
       if (!last) {
         plude_k = plude_k * D(zdtgdp);
-        if (ldcum && Real(plude_k) > zepsec && plu_k1 > zepsec) {
-          solac = solac + DIV(Real(plude_k), plu_k1);
-          convsrce_l = Real(pludeli1) * zdtgdp;
-          convsrce_i = Real(pludeli2) * zdtgdp;
-          QADD(LL, convsrce_l);
-          QADD(II, convsrce_i);
-          if constexpr (BUD) {  // :1378-1380
+        const bool c = ldcum && Real(plude_k) > zepsec && plu_k1 > zepsec;
+        const Real dcov = DIV(Real(plude_k), c ? plu_k1 : C(1.0));
+        solac = c ? solac + dcov : solac;
+        convsrce_l = c ? Real(pludeli1) * zdtgdp : C(0.0);
+        convsrce_i = c ? Real(pludeli2) * zdtgdp : C(0.0);
+        QADD(LL, convsrce_l);
+        QADD(II, convsrce_i);
+        if constexpr (BUD) {  // :1378-1380
+          if (c) {
             bd.l[3] = convsrce_l * zqtmst;
             bd.i[3] = convsrce_i * zqtmst;
             bd.cc[3] = DIV(zqtmst * plude_k, plu_k1);
           }
-        } else {
-          plude_k = 0.0;
         }
+        plude_k = c ? plude_k : 0.0;
         if (P.lmfdsnow) {
           const D psnde_r = ld(F.psnde + ok2s), psnde_s = ld(F.psnde + ok2s + s2);
           if constexpr (FAST_) {
@@ -773,14 +951,15 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
 
       // 3.3 subsidence source and evaporation (:1419-1492)
       if (k > ncldtop0) {
-        Real zmf = mx(C(0.0), (pmfu_k * zadvw + pmfd_k * zadvwd) * zdtgdp);
+        const Real pmfu_k = p_pmfu.get(), pmfd_k = p_pmfd.get(), zanewm1 = p_anew.get();
+        Real zmf = mx(C(0.0), (pmfu_k * ZADVW + pmfd_k * ZADVWD) * zdtgdp);
         Real zacust = zmf * zanewm1;
-        Real lcust_l = zmf * qxnm1_l;
-        Real lcust_i = zmf * qxnm1_i;
+        Real lcust_l = zmf * p_xl.get();
+        Real lcust_i = zmf * p_xi.get();
         convsrce_l = convsrce_l + lcust_l;
         convsrce_i = convsrce_i + lcust_i;
-        Real zdtdp = DIV(P.zrdcp * C(0.5) * (t_prev + t), Real(paph_k));
-        Real zwtot = mn(P.rg * (pmfu_k * zadvw + pmfd_k * zadvwd), DIVY((pap_k - pap_prev), rdt, rrdt));
+        Real zdtdp = DIV(P.zrdcp * C(0.5) * (p_t.get() + t), Real(paph_k));
+        Real zwtot = mn(P.rg * (pmfu_k * ZADVW + pmfd_k * ZADVWD), DIVY((pap_k - p_pap.get()), rdt, rrdt));
         Real zdtforc = zdtdp * rdt * zwtot;
         Real zdqs = zanewm1 * zdtforc * zdqsmixdt;
         Real lfinalsum = C(0.0);
@@ -810,15 +989,16 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
         }
         solac = solac + zacust;
         if constexpr (BUD) bd.cc[4] = zacust * zqtmst;  // :1484
-        if (lfinalsum < zepsec) {
-          solac = solac - zacust;
-          if constexpr (BUD) bd.cc[5] = -zacust * zqtmst;  // :1488
+        const bool none = lfinalsum < zepsec;
+        solac = none ? solac - zacust : solac;
+        if constexpr (BUD) {  // :1488
+          if (none) bd.cc[5] = -zacust * zqtmst;
         }
       }
 
       // subsidence sink (:1499-1514)
       if (!last) {
-        Real zmfdn = mx(C(0.0), (pmfu_k1 * zadvw + pmfd_k1 * zadvwd) * zdtgdp);
+        Real zmfdn = mx(C(0.0), (pmfu_k1 * ZADVW + pmfd_k1 * ZADVWD) * zdtgdp);
         solab = solab + zmfdn;
         qb_ll = qb_ll + zmfdn;
         qb_ii = qb_ii + zmfdn;
@@ -831,22 +1011,24 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
         Real zldifdt = P.rcldiff * rdt;
         if (spp && P.spp_on[CLOUDSC_SPP_RCLDIFF]) zldifdt = P.rcldiff * rdt * Real(sppf[CLOUDSC_SPP_RCLDIFF]);
         Real pl = Real(plude_k);
-        if (ktype >= 2 && pl > zepsec && peis < C(10.0)) {
+        if (shallow && pl > zepsec) {
           zldifdt = C(20.0) * P.rcldiff_convi * zldifdt;
         } else if (ktype == 1 && pl > zepsec) {
           zldifdt = C(2.0) * P.rcldiff_convi * zldifdt;
         }
-        if (zli > zepsec) {
-          Real zqe = DIVY((qv - a * zqsmix), d1ma, r1ma);
-          Real ze = mx(zqsmix - zqe, C(0.0));
-          Real zleros = C(0.333) * a * (C(1.) - a) * zldifdt * ze;
-          zleros = mn(zleros, zevaplimmix);
-          zleros = mn(zleros, zli);
-          Real zaeros = DIV(C(0.5) * zleros, zlicld);
-          solac = solac - zaeros;
-          QSUB(LV, liqfrac * zleros);  // (V,L) +=, (L,V) -=
-          QSUB(IV, icefrac * zleros);  // (V,I) +=, (I,V) -=
-          if constexpr (BUD) {  // :1749-1751
+        const bool c = zli > zepsec;
+        Real zqe = DIVY((qv - a * zqsmix), d1ma, r1ma);
+        Real ze = mx(zqsmix - zqe, C(0.0));
+        Real zleros = C(0.333) * a * (C(1.) - a) * zldifdt * ze;
+        zleros = mn(zleros, zevaplimmix);
+        zleros = mn(zleros, zli);
+        zleros = c ? zleros : C(0.0);
+        Real zaeros = DIV(C(0.5) * zleros, c ? zlicld : C(1.0));
+        solac = solac - zaeros;
+        QSUB(LV, liqfrac * zleros);  // (V,L) +=, (L,V) -=
+        QSUB(IV, icefrac * zleros);  // (V,I) +=, (I,V) -=
+        if constexpr (BUD) {  // :1749-1751
+          if (c) {
             bd.l[7] = -liqfrac * zleros * zqtmst;
             bd.i[7] = -icefrac * zleros * zqtmst;
             bd.cc[7] = -zaeros * zqtmst;
@@ -863,59 +1045,79 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
       const Real fs_i = (spp && P.spp_on[CLOUDSC_SPP_FALLSPEED]) ? fs_i0 * Real(sppf[CLOUDSC_SPP_FALLSPEED])
                                                                  : fs_i0;  // :1806-1808
       const Real fs_s = P.rvsnow;
+      // (the rain fall speed is computed with the rain processes below)
       Real fs_r = C(0.0);
-      {
-        Real ztemp = C(0.5) * (qr + qxnm1_r);
-        if (ztemp != C(0.0)) {
-          Real zfallcorr = fallcorr_r;
-          Real zrlambda = mpowp<F32M, GEN, FAST_>(DIVP(zrho * ztemp, P.rcl_lam1r, P.rcp_rcl_lam1r), P.rcl_lam2r);
-          fs_r = P.rxfallspeedrain * zfallcorr * P.rcl_const7r * mpowp<F32M, GEN, FAST_>(zrlambda, P.rcl_dr);
-        }
-      }
+      const Real qr_mid = C(0.5) * (qr + p_xr.get());
       if (k > ncldtop0) {
-        fallsrce_i = pfplsx_i * zdtgdp;
+        fallsrce_i = p_fli.get() * zdtgdp;
         QADD(II, fallsrce_i);
         if constexpr (BUD) bd.i[12] = fallsrce_i * zqtmst;  // :1865
         qxfg_i = qxfg_i + fallsrce_i;
         qpretot = qpretot + qxfg_i;
-        fallsrce_r = pfplsx_r * zdtgdp;
+        fallsrce_r = p_flr.get() * zdtgdp;
         QADD(RR, fallsrce_r);
         qxfg_r = qxfg_r + fallsrce_r;
         qpretot = qpretot + qxfg_r;
-        fallsrce_s = pfplsx_s * zdtgdp;
+        fallsrce_s = p_fls.get() * zdtgdp;
         QADD(SS, fallsrce_s);
         qxfg_s = qxfg_s + fallsrce_s;
         qpretot = qpretot + qxfg_s;
       }
       const Real fallsink_i = zdtgdp * zrho * fs_i;
-      const Real fallsink_r = zdtgdp * zrho * fs_r;
       const Real fallsink_s = zdtgdp * zrho * fs_s;
 
       // 4.2 precipitation fraction (:1898-1919)
-      Real zcovpclr, zraincld, zraincldm1, zsnowcld;
-      if (qpretot > zepsec) {
-        zcovptot = C(1.0) - (DIV((C(1.0) - zcovptot) * (C(1.0) - mx(a, za_prev)), (C(1.0) - mn(za_prev, C(1.0) - C(1.E-06)))));
-        zcovptot = mx(zcovptot, P.rcovpmin);
-        zcovpclr = mx(C(0.0), zcovptot - a);
-        const Real rcov = RCP(zcovptot);
-        zraincld = DIVY(C(0.5) * (qr + qr_prev), zcovptot, rcov);
-        zraincldm1 = DIVY(C(0.5) * (qr + qxnm1_r), zcovptot, rcov);
-        zsnowcld = DIVY(C(0.5) * (qs + qs_prev), zcovptot, rcov);
-        zcovpmax = mx(zcovptot, zcovpmax);
-      } else {
-        zraincld = C(0.0);
-        zraincldm1 = C(0.0);
-        zsnowcld = C(0.0);
-        zcovptot = C(0.0);
-        zcovpclr = C(0.0);
-        zcovpmax = C(0.0);
+      Real zcovpclr = C(0.0), zraincld = C(0.0), zraincldm1 = C(0.0), zsnowcld = C(0.0);
+      Real zcovptot = C(0.0), zcovpmax = C(0.0);
+      const Real za_prev = p_za.get();
+      if (k > ncldtop0) {  // QPRETOT is zero at the first level
+        const bool c = qpretot > zepsec;
+        zcovptot = p_cov.get();
+        Real cov = C(1.0) - (DIV((C(1.0) - zcovptot) * (C(1.0) - mx(a, za_prev)), (C(1.0) - mn(za_prev, C(1.0) - C(1.E-06)))));
+        cov = mx(cov, P.rcovpmin);
+        const Real rcov = RCP(cov);
+        const Real rain = DIVY(C(0.5) * (qr + p_qr.get()), cov, rcov);
+        const Real rainm1 = DIVY(qr_mid, cov, rcov);
+        const Real snow = DIVY(C(0.5) * (qs + p_qs.get()), cov, rcov);
+        zcovptot = c ? cov : C(0.0);
+        zcovpclr = c ? mx(C(0.0), cov - a) : C(0.0);
+        zraincld = c ? rain : C(0.0);
+        zraincldm1 = c ? rainm1 : C(0.0);
+        zsnowcld = c ? snow : C(0.0);
+        zcovpmax = c ? mx(cov, p_covmax.get()) : C(0.0);
       }
 
       // 4.3 warm rain, IWARMRAIN=3, IRAINACC=1 (:1930-2259)
-      if (zliqcld > zepsec) {
-        const PowBase b_liq = mbase<F32M, FAST_>(zliqcld);
+      // 4.4's humidity limits (:2282-2300)
+      Real zzrh = P.rprecrhmax + DIVY((C(1.0) - P.rprecrhmax) * zcovpmax, d1ma, r1ma);
+      zzrh = mn(mx(zzrh, P.rprecrhmax), C(1.0));
+      const Real zrhmax = zzrh;
+      Real zxramid = P.ramid;
+      if (spp && P.spp_on[CLOUDSC_SPP_RAMID]) {  // :2282-2287
+        zxramid = P.ramid * Real(sppf[CLOUDSC_SPP_RAMID]);
+        if (P.spp_lramidlimit1) zxramid = mn(C(1.0), zxramid);
+      }
+      const Real zsigk = DIVY(pap_k, Real(p_psurf.get()), p_rpsurf.get());
+      {
+        const Real sg = DIVK((zsigk - C(0.8)), 0.2);
+        const Real zrhc = zsigk > C(0.8) ? zxramid + (C(1.0) - zxramid) * (sg * sg) : zxramid;
+        zzrh = mn(zrhc, zzrh);
+        zzrh = mn(C(0.9), zzrh);
+      }
+      const Real zqe_r = mx(C(0.0), mn(qv, zqsliq));
+      // The rain processes together: warm rain (4.3), the rain fall speed
+      // (4.1) and rain evaporation (4.4).  Their rates do not depend on one
+      // another; a lane without one of them computes it on a harmless operand
+      // and selects it away, so that the independent logs, exps and divisions
+      // form one block and overlap (a branch each, the walk down a column
+      // waited on one dependent chain after another).  Skipped when no lane
+      // of the warp needs any.
+      const bool wet = zliqcld > zepsec, accr = wet && zraincld > zepsec, falls = qr_mid != C(0.0);
+      const bool evap = zcovpclr > zepsec && zraincldm1 > zepsec && zqe_r < zzrh * zqsliq;
+      if (CSC_ANY(wet || falls || evap)) {
         Real zeaut = P.rcl_inhomogaut, zeacc = P.rcl_inhomogacc;
         if constexpr (OPT) {
+          if (wet) {
           double zcldraincorr = 0.0;
           if (P.lcloud_inhomog || P.lrad_cloud_inhomog) {  // :1937-1967
             const double zqtot = mn((qvD + qlD) * 1000.0, 30.0);
@@ -948,70 +1150,62 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
             zeaut = zeaut * Real(sppf[CLOUDSC_SPP_CLOUDINHOM]);
             zeacc = zeacc * Real(sppf[8]);
           }
+          }
         }
-        Real zrainaut = zeaut * rdt * P.rcl_kkaau * mpowbp<F32M, GEN, FAST_>(b_liq, P.kkbauq_m1) * zconstpow;
-        qb_rl = qb_rl + zrainaut;
-        Real zrainacc = C(0.0);
-        if (zraincld > zepsec) {
-          zrainacc = zeacc * rdt * P.rcl_kkaac * mpowbp<F32M, GEN, FAST_>(b_liq, P.kkbac_m1) *
-                     mpowp<F32M, GEN, FAST_>(zraincld, P.rcl_kkbac);
+        if (WIDE || CSC_ANY(wet)) {
+          const PowBase b_liq = mbase<F32M, FAST_>(wet ? zliqcld : C(1.0));
+          const PowBase b_rain = mbase<F32M, FAST_>(accr ? zraincld : C(1.0));
+          Real zrainaut = zeaut * rdt * P.rcl_kkaau * mpowbp<F32M, GEN, FAST_>(b_liq, P.kkbauq_m1) * (land ? P.zconst_pow_land : P.zconst_pow_sea);
+          zrainaut = wet ? zrainaut : C(0.0);
+          qb_rl = qb_rl + zrainaut;
+          Real zrainacc = zeacc * rdt * P.rcl_kkaac * mpowbp<F32M, GEN, FAST_>(b_liq, P.kkbac_m1) *
+                          mpowbp<F32M, GEN, FAST_>(b_rain, P.rcl_kkbac);
+          zrainacc = accr ? zrainacc : C(0.0);
+          qb_rl = qb_rl + zrainacc;
+          if constexpr (BUD) {
+            b_rainaut = zrainaut;
+            b_rainacc = zrainacc;
+          }
         }
-        qb_rl = qb_rl + zrainacc;
-        if constexpr (BUD) {
-          b_rainaut = zrainaut;
-          b_rainacc = zrainacc;
+        if (WIDE || CSC_ANY(falls)) {
+          const Real zrlambda = mpowp<F32M, GEN, FAST_>(DIVP(zrho * (falls ? qr_mid : C(1.0)), P.rcl_lam1r, P.rcp_rcl_lam1r), P.rcl_lam2r);
+          fs_r = P.rxfallspeedrain * fallcorr_r * P.rcl_const7r * mpowp<F32M, GEN, FAST_>(zrlambda, P.rcl_dr);
+          fs_r = falls ? fs_r : C(0.0);
         }
-      }
-
-      // 4.4 rain evaporation (:2271-2378)
-      {
-        Real zzrh = P.rprecrhmax + DIVY((C(1.0) - P.rprecrhmax) * zcovpmax, d1ma, r1ma);
-        zzrh = mn(mx(zzrh, P.rprecrhmax), C(1.0));
-        Real zxramid = P.ramid;
-        if (spp && P.spp_on[CLOUDSC_SPP_RAMID]) {  // :2282-2287
-          zxramid = P.ramid * Real(sppf[CLOUDSC_SPP_RAMID]);
-          if (P.spp_lramidlimit1) zxramid = mn(C(1.0), zxramid);
-        }
-        Real zrhc = zxramid;
-        Real zsigk = DIVY(pap_k, Real(paph_surf), rpsurf);
-        if (zsigk > C(0.8)) {
-          Real s = DIVK((zsigk - C(0.8)), 0.2);
-          zrhc = zxramid + (C(1.0) - zxramid) * (s * s);
-        }
-        zzrh = mn(zrhc, zzrh);
-        zzrh = mn(C(0.9), zzrh);
-        Real zqe = mx(C(0.0), mn(qv, zqsliq));
-        if (zcovpclr > zepsec && zraincldm1 > zepsec && zqe < zzrh * zqsliq) {
-          Real zpreclr = zraincldm1;
-          Real zfallcorr = fallcorr_f;
+        // rain evaporation (:2300-2378)
+        if (WIDE || CSC_ANY(evap)) {
+          const PowBase b_lam = mbase<F32M, FAST_>(mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1r, (zrho * (evap ? zraincldm1 : C(1.0)))), P.rcl_lam2r));
           Real zesatliq = P.rv_rd * (P.r2es * el_e);
-          Real zlambda = mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1r, (zrho * zpreclr)), P.rcl_lam2r);
-          const PowBase b_lam = mbase<F32M, FAST_>(zlambda);
           Real zevap_denom = P.rcl_cdenom1 * zesatliq - P.rcl_cdenom2 * t * zesatliq +
                              P.rcl_cdenom3 * mpow<F32M, FAST_>(t, C(3.0)) * pap_k;
-          Real zcorr2 = DIV(mpow<F32M, FAST_>(DIVK(t, 273.), C(1.5)) * C(393.), (t + C(120.)));
-          Real zsubsat = mx(zzrh * zqsliq - zqe, C(0.0));
+          Real zcorr2 = DIV(mroot3<F32M, FAST_>(DIVK(t, 273.), divbad_) * C(393.), (t + C(120.)));
+          Real zsubsat = mx(zzrh * zqsliq - zqe_r, C(0.0));
           Real zbeta = (DIV(C(0.15), zqsliq)) * (t * t) * zesatliq * P.rcl_const1r * (DIV(zcorr2, zevap_denom)) *
                        (DIV(C(0.78), (mpowbp<F32M, GEN, FAST_>(b_lam, P.rcl_const4r))) +
-                        DIV(P.rcl_const2r * mpow<F32M, FAST_>(zrho * zfallcorr, C(0.5)), (mpow<F32M, FAST_>(zcorr2, C(0.5)) * mpowbp<F32M, GEN, FAST_>(b_lam, P.rcl_const3r))));
+                        DIV(P.rcl_const2r * mroot<F32M, FAST_>(zrho * fallcorr_f, divbad_), (mroot<F32M, FAST_>(zcorr2, divbad_) * mpowbp<F32M, GEN, FAST_>(b_lam, P.rcl_const3r))));
           Real zdenom = C(1.0) + zbeta * rdt * zcorqsliq;
           Real zdpevap = DIV(zcovpclr * zbeta * rdt * zsubsat, zdenom);
           if (spp && P.spp_on[CLOUDSC_SPP_RAINEVAP]) zdpevap = zdpevap * Real(sppf[CLOUDSC_SPP_RAINEVAP]);
           D zevap = mn(D(zdpevap), qxfg_r);
+          zevap = evap ? zevap : 0.0;
           QSUB(RV, zevap);  // (V,R) += zevap, (R,V) -= zevap
-          if constexpr (BUD) bd.l[20] = -zevap * zqtmst;  // :2363
+          if constexpr (BUD) {  // :2363
+            if (evap) bd.l[20] = -zevap * zqtmst;
+          }
           qxfg_r = qxfg_r - zevap;
         }
       }
+      const Real fallsink_r = zdtgdp * zrho * fs_r;
 
+      // the next level's lines on their way while this level computes
+      CSC_PREFETCH(k + 2 < klev, (size_t)(k + 1) * np);
       // 4.5 ice deposition, IDEPICE=1 (:2404-2499)
       {
-        if (za_prev < P.rcldtopcf && a >= P.rcldtopcf) {
-          zcldtopdist = C(0.0);
-        } else {
-          zcldtopdist = zcldtopdist + DIV(zdp, (zrho * P.rg));
-        }
-        if (t < (P.rtt - C(5.)) && qxfg_l > P.rlmin) {
+        const Real deeper = p_ctd.get() + DIV(zdp, (zrho * P.rg));
+        const Real zcldtopdist = (za_prev < P.rcldtopcf && a >= P.rcldtopcf) ? C(0.0) : deeper;
+        p_ctd.set(zcldtopdist);
+        const bool dep = t < (P.rtt - C(5.)) && qxfg_l > P.rlmin;
+        if (CSC_ANY(dep)) {
           Real zsupersatice = DIV((zqsliq - zqsice), zqsice);
           Real zvpice = DIVP((P.r2es * ei_e) * P.rv, P.rd, P.rcp_rd);
           Real zicenuclei = C(1000.0) * mexp<F32M, FAST_>(C(12.96) * zsupersatice - C(0.639));
@@ -1019,19 +1213,23 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
           Real zbdd = DIV(P.rv * t * pap_k, (C(2.21) * zvpice));
           Real zcvds = DIV(C(7.8) * mpow<F32M, FAST_>(DIVY(zicenuclei, zrho, rrho), C(0.666)) * zsupersatice, (C(8.87) * (zadd + zbdd)));
           Real zice0 = mx(zicecld, DIVY(zicenuclei * P.riceinit, zrho, rrho));
-          Real zinew = mpow<F32M, FAST_>(C(0.666) * zcvds * rdt + mpow<F32M, FAST_>(zice0, C(0.666)), C(1.5));
+          const Real grown = C(0.666) * zcvds * rdt + mpow<F32M, FAST_>(zice0, C(0.666));
+          Real zinew = mroot3<F32M, FAST_>(dep ? grown : C(1.0), divbad_);
           D zdepos = D(mx(P.rcl_overlapliqice * a * (zinew - zice0), C(0.0)));
           zdepos = mn(zdepos, qxfg_l);
           Real zinfactor = mn(DIVK(zicenuclei, 15000.), C(1.0));
           zdepos = zdepos * D(mn(zinfactor + (C(1.0) - zinfactor) *
                                                (P.rdepliqrefrate + DIVP(zcldtopdist, P.rdepliqrefdepth, P.rcp_rdepliqrefdepth)),
                                C(1.0)));
+          zdepos = dep ? zdepos : 0.0;
           QSUB(LI, zdepos);  // (I,L) += zdepos, (L,I) -= zdepos
           qxfg_i = qxfg_i + zdepos;
           qxfg_l = qxfg_l - zdepos;
           if constexpr (BUD) {  // :2495-2496
-            bd.l[11] = -zdepos * zqtmst;
-            bd.i[11] = zdepos * zqtmst;
+            if (dep) {
+              bd.l[11] = -zdepos * zqtmst;
+              bd.i[11] = zdepos * zqtmst;
+            }
           }
         }
       }
@@ -1039,30 +1237,45 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
       // 4.7 snow deposition, IDEPSNOW=1 (:2698-2745)
       {
         Real zsupersatice = mx(DIV((qv - zqsmix), zqsmix), C(0.0));
-        if (t < P.rtt && zsnowcld > zepsec && zsupersatice > C(0.0)) {
-          Real zvpice = DIVP((P.r2es * ei_e) * P.rv, P.rd, P.rcp_rd);
-          Real zaplusb = P.rcl_apb1 * zvpice - P.rcl_apb2 * zvpice * t + pap_k * P.rcl_apb3 * (t * t * t);
-          Real zcorrfac = mpow<F32M, FAST_>(rrho, C(0.5));
-          Real zcorrfac2 = (mpow<F32M, FAST_>(DIVK(t, 273.0), C(1.5))) * (DIV(C(393.0), (t + C(120.0))));
-          Real zpr02 = zrho * zsnowcld * P.rcl_const1s;
+        const bool dep = t < P.rtt && zsnowcld > zepsec && zsupersatice > C(0.0);
+        // revise in-cloud condensate (:2750-2754)
+        zliqcld = Real(qxfg_l) * ztmpa;
+        zicecld = Real(qxfg_i) * ztmpa;
+        // riming (4.9, :2973-3017) raises the same base to its own power
+        const bool rime = t <= P.rtt && zliqcld > zepsec && zsnowcld > zepsec && zcovptot > C(0.01);
+        if (CSC_ANY(dep || rime)) {
+          const Real zpr02 = zrho * (dep || rime ? zsnowcld : C(1.0)) * P.rcl_const1s;
           const PowBase b_pr02 = mbase<F32M, FAST_>(zpr02);
-          Real zterm1 = DIV(zsupersatice * (t * t) * zvpice * zcorrfac2 * P.rcl_const2s, (zrho * zaplusb));
-          Real zterm2 = C(0.65) * P.rcl_const6s * mpowbp<F32M, GEN, FAST_>(b_pr02, P.rcl_const4s) +
-                        DIV(P.rcl_const3s * mpow<F32M, FAST_>(zcorrfac, C(0.5)) * mpow<F32M, FAST_>(zrho, C(0.5)) *
-                            mpowbp<F32M, GEN, FAST_>(b_pr02, P.rcl_const5s), mpow<F32M, FAST_>(zcorrfac2, C(0.5)));
-          Real zpsdep = mx(zcovptot * zterm1 * zterm2 * rdt, C(0.0));
-          zpsdep = DIVY(mn(zpsdep, qv - zqsmix), zcorqsmix, rcqsmix);
-          QADD(SV, zpsdep);  // (S,V) += zpsdep, (V,S) -= zpsdep
-          if constexpr (BUD) b_psdep = zpsdep;
+          if (WIDE || CSC_ANY(dep)) {
+            Real zvpice = DIVP((P.r2es * ei_e) * P.rv, P.rd, P.rcp_rd);
+            Real zaplusb = P.rcl_apb1 * zvpice - P.rcl_apb2 * zvpice * t + pap_k * P.rcl_apb3 * (t * t * t);
+            if (!dep) zaplusb = C(1.0);
+            Real zcorrfac = mroot<F32M, FAST_>(rrho, divbad_);
+            Real zcorrfac2 = (mroot3<F32M, FAST_>(DIVK(t, 273.0), divbad_)) * (DIV(C(393.0), (t + C(120.0))));
+            Real zterm1 = DIV(zsupersatice * (t * t) * zvpice * zcorrfac2 * P.rcl_const2s, (zrho * zaplusb));
+            Real zterm2 = C(0.65) * P.rcl_const6s * mpowbp<F32M, GEN, FAST_>(b_pr02, P.rcl_const4s) +
+                          DIV(P.rcl_const3s * mroot<F32M, FAST_>(zcorrfac, divbad_) * mroot<F32M, FAST_>(zrho, divbad_) *
+                              mpowbp<F32M, GEN, FAST_>(b_pr02, P.rcl_const5s), mroot<F32M, FAST_>(zcorrfac2, divbad_));
+            Real zpsdep = mx(zcovptot * zterm1 * zterm2 * rdt, C(0.0));
+            zpsdep = DIVY(mn(zpsdep, qv - zqsmix), zcorqsmix, rcqsmix);
+            zpsdep = dep ? zpsdep : C(0.0);
+            QADD(SV, zpsdep);  // (S,V) += zpsdep, (V,S) -= zpsdep
+            if constexpr (BUD) b_psdep = zpsdep;
+          }
+          if (WIDE || CSC_ANY(rime)) {
+            Real zsnowrime = P.rcl_effrime * zcovptot * rdt * P.rcl_const7s * fallcorr_f *
+                             mpowbp<F32M, GEN, FAST_>(b_pr02, P.rcl_const8s);
+            zsnowrime = mn(zsnowrime, C(1.0));
+            zsnowrime = rime ? zsnowrime : C(0.0);
+            qb_sl = qb_sl + zsnowrime;
+            if constexpr (BUD) b_snowrime = zsnowrime;
+          }
         }
       }
 
-      // revise in-cloud condensate (:2750-2754)
-      zliqcld = Real(qxfg_l) * ztmpa;
-      zicecld = Real(qxfg_i) * ztmpa;
-
       // 4.8 ice -> snow autoconversion (:2769-2800)
-      if (t <= P.rtt && zicecld > zepsec) {
+      const bool autoc = t <= P.rtt && zicecld > zepsec;
+      if (CSC_ANY(autoc)) {
         Real zzco = rdt * P.rsnowlin1 * mexp<F32M, FAST_>(P.rsnowlin2 * (t - P.rtt));
         Real zlcrit = P.rlcritsnow;
         bool aer = false;
@@ -1070,148 +1283,160 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
           // LAERICEAUTO: the aerosol's critical ice amount, the rate scaled by
           // (RNICE/PNICE)**0.333 (:2776-2779)
           if (P.laericeauto) {
-            zlcrit = Real(ld(F.picrit_aer + ok));
-            zzco = zzco * mpow<F32M, FAST_>(DIV(P.rnice, Real(ld(F.pnice + ok))), C(0.333));
+            zlcrit = autoc ? Real(ld(F.picrit_aer + ok)) : C(1.0);
+            zzco = zzco * mpow<F32M>(DIV(P.rnice, autoc ? Real(ld(F.pnice + ok)) : C(1.0)), C(0.333));
             aer = true;
           }
         }
         if (!aer && spp && P.spp_on[CLOUDSC_SPP_RLCRITSNOW])
           zlcrit = P.rlcritsnow * Real(sppf[CLOUDSC_SPP_RLCRITSNOW]);
-        Real r = DIV(zicecld, zlcrit);
+        Real r = DIV(autoc ? zicecld : C(0.0), zlcrit);
         Real ztemp = C(-1.) * (r * r);
         // 1 - exp(x) is 1 for every x <= -100: the bound changes nothing and
         // keeps the argument in the fast exp's window
         if (FAST_ && !F32M) ztemp = mx(ztemp, C(-100.0));
         Real zsnowaut = (ztemp < C(50.0)) ? zzco * (C(1.0) - mexp<F32M, FAST_>(ztemp)) : zzco;
+        zsnowaut = autoc ? zsnowaut : C(0.0);
         qb_si = qb_si + zsnowaut;
         if constexpr (BUD) b_snowaut = zsnowaut;
       }
 
       // 4.12 melting (:2815-2862)
       {
-        D zicetot = qxfg_i + qxfg_s;
-        Real zmeltmax = C(0.0);
-        if (zicetot > zepsec && t > P.rtt) {
+        const D zicetot = qxfg_i + qxfg_s;
+        const bool warm = zicetot > zepsec && t > P.rtt;
+        if (CSC_ANY(warm)) {
           Real zsubsat = mx(zqsice - qv, C(0.0));
           Real ztdmtw0 = t - P.rtt -
                          zsubsat * (C(1329.31) + C(0.0074615) * (pap_k - C(0.85E5)) - C(40.637) * (t - C(275.0)));
           Real zcons1 = xabs(DIVP(rdt * (C(1.0) + C(0.5) * ztdmtw0), P.rtaumel, P.rcp_rtaumel));
-          zmeltmax = mx(ztdmtw0 * zcons1 * P.zrldcp, C(0.0));
-        }
-        if (zmeltmax > zepsec && zicetot > zepsec) {
-          const D rit = RCP(D(zicetot));
-          D zalfa = DIVY(qxfg_i, D(zicetot), rit);
+          const Real zmeltmax = mx(ztdmtw0 * zcons1 * P.zrldcp, C(0.0));
+          const bool melt = warm && zmeltmax > zepsec;
+          const D tot = melt ? zicetot : 1.0;
+          const D rit = RCP(D(tot));
+          D zalfa = DIVY(qxfg_i, D(tot), rit);
           D zmelt = mn(qxfg_i, zalfa * D(zmeltmax));
+          zmelt = melt ? zmelt : 0.0;
+          zalfa = DIVY(qxfg_s, D(tot), rit);
           qxfg_i = qxfg_i - zmelt;
           qxfg_r = qxfg_r + zmelt;
           QSUB(IR, zmelt);  // (R,I) += zmelt, (I,R) -= zmelt
           if constexpr (BUD) {  // :2856-2857
-            bd.i[15] = -zmelt * zqtmst;
-            bd.l[17] = zmelt * zqtmst;
+            if (melt) {
+              bd.i[15] = -zmelt * zqtmst;
+              bd.l[17] = zmelt * zqtmst;
+            }
           }
-          zalfa = DIVY(qxfg_s, D(zicetot), rit);
           zmelt = mn(qxfg_s, zalfa * D(zmeltmax));
+          zmelt = melt ? zmelt : 0.0;
           qxfg_s = qxfg_s - zmelt;
           qxfg_r = qxfg_r + zmelt;
           QADD(RS, zmelt);  // (R,S) += zmelt, (S,R) -= zmelt
-          if constexpr (BUD) bd.i[16] = -zmelt * zqtmst;  // :2858
+          if constexpr (BUD) {  // :2858
+            if (melt) bd.i[16] = -zmelt * zqtmst;
+          }
         }
       }
 
       // 4.13 rain freezing (:2877-2933)
-      if (qr > zepsec) {
-        if (t <= P.rtt && t_prev > P.rtt) {
-          Real zqpre = mx(qs + qr, zepsec);
-          prainfrac = DIV(qr, zqpre);
-          llrainliq = prainfrac > P.flt_0p8;
+      const bool rainy = qr > zepsec;
+      Real prainfrac = p_frac.get();
+      {
+        const bool top = rainy && t <= P.rtt && p_t.get() > P.rtt;
+        const Real zqpre = mx(qs + qr, zepsec);
+        const Real f = DIV(qr, top ? zqpre : C(1.0));
+        prainfrac = top ? f : prainfrac;
+        llrainliq = top ? prainfrac > P.flt_0p8 : llrainliq;
+        p_frac.set(prainfrac);
+      }
+      const bool freeze = rainy && t < P.rtt;
+      // PSD slopes (:3026-3069), PSACR (:3084-3115), PIACR (:3171-3198)
+      const bool coll = t <= P.rtt && prainfrac < zepsec && zraincld > zepsec;
+      const bool coll_s = coll && zsnowcld > zepsec, coll_i = coll && zicecld > zepsec;
+      Real zpsacr = C(0.0), zpiacr = C(0.0);
+      // freezing and the two collections together, as the rain processes
+      if (CSC_ANY(freeze || coll_s || coll_i)) {
+        if (WIDE || CSC_ANY(freeze)) {
+          const bool liq = freeze && llrainliq;
+          const Real zlambda = mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1r, (zrho * (liq ? qr : C(1.0)))), P.rcl_lam2r);
+          Real ztemp = mn(P.rcl_fzrab * (t - P.rtt), C(50.));
+          Real zrate = rdt * (DIVY(P.rcl_const5r, zrho, rrho)) * (mexp<F32M, FAST_>(ztemp) - C(1.)) * mpowp<F32M, GEN, FAST_>(zlambda, P.rcl_const6r);
+          Real zcons1 = xabs(DIVP(rdt * (C(1.0) + C(0.5) * (P.rtt - t)), P.rtaumel, P.rcp_rtaumel));
+          const Real zfrzmax = llrainliq ? mx(zrate, C(0.0)) : mx((P.rtt - t) * zcons1 * P.zrldcp, C(0.0));
+          const bool c = freeze && zfrzmax > zepsec;
+          D zfrz = mn(qrD, D(zfrzmax));
+          zfrz = c ? zfrz : 0.0;
+          QSUB(RS, zfrz);  // (S,R) += zfrz, (R,S) -= zfrz
+          if constexpr (BUD) {  // :2927
+            if (c) bd.l[18] = -zfrz * zqtmst;
+          }
         }
-        if (t < P.rtt) {
-          Real zfrzmax;
-          if (llrainliq) {
-            Real zlambda = mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1r, (zrho * qr)), P.rcl_lam2r);
-            Real ztemp = mn(P.rcl_fzrab * (t - P.rtt), C(50.));
-            Real zfrz = rdt * (DIVY(P.rcl_const5r, zrho, rrho)) * (mexp<F32M, FAST_>(ztemp) - C(1.)) * mpowp<F32M, GEN, FAST_>(zlambda, P.rcl_const6r);
-            zfrzmax = mx(zfrz, C(0.0));
-          } else {
-            Real zcons1 = xabs(DIVP(rdt * (C(1.0) + C(0.5) * (P.rtt - t)), P.rtaumel, P.rcp_rtaumel));
-            zfrzmax = mx((P.rtt - t) * zcons1 * P.zrldcp, C(0.0));
+        if (WIDE || CSC_ANY(coll_s || coll_i)) {
+          const Real zlamr = mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1r, (zrho * (coll ? zraincld : C(1.0)))), P.rcl_lam2r);
+          Real zn0r = P.rcl_x1r * mpowp<F32M, GEN, FAST_>(zlamr, P.rcl_x2r);
+          Real zlamr3 = zlamr * zlamr * zlamr;
+          if (WIDE || CSC_ANY(coll_s)) {
+            const Real zlams = mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1s, (zrho * (coll_s ? zsnowcld : C(1.0)))), P.rcl_lam2s);
+            Real zn0s = P.rcl_x1s;
+            Real zfalldiff = mx(xabs(fs_r - fs_s), DIV2((fs_r + fs_s), C(8.)));
+            Real zfac = DIV(P.rpi * P.rpi * P.rdenswat * zrho * zn0r * zn0s, (zlams * zlamr3));
+            Real zrat = DIV(zlamr, zlams);
+            zpsacr = DIV(zcovptot * rdt * zfac * zfalldiff * ((C(0.5) * zrat + C(2.)) * zrat + C(5.)), zlamr3);
+            zpsacr = coll_s ? zpsacr : C(0.0);
           }
-          if (zfrzmax > zepsec) {
-            D zfrz = mn(qrD, D(zfrzmax));
-            QSUB(RS, zfrz);  // (S,R) += zfrz, (R,S) -= zfrz
-            if constexpr (BUD) bd.l[18] = -zfrz * zqtmst;  // :2927
+          if (WIDE || CSC_ANY(coll_i)) {
+            const Real zlami = mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1s, (zrho * (coll_i ? zicecld : C(1.0)))), P.rcl_lam2s);
+            Real zn0i = P.rcl_x1s;
+            Real zfalldiff = mx(xabs(fs_r - fs_i), DIV2((fs_r + fs_i), C(8.)));
+            Real zfac = DIV(P.rpi * P.rpi * P.rdenswat * C(0.1) * zrho * zn0r * zn0i, (zlami * zlamr3));
+            Real zrat = DIV(zlamr, zlami);
+            zpiacr = DIV(zcovptot * rdt * zfac * zfalldiff * ((C(0.5) * zrat + C(2.)) * zrat + C(5.)), zlamr3);
+            zpiacr = coll_i ? zpiacr : C(0.0);
           }
+        }
+        QSUB(RS, zpsacr);  // (S,R) += zpsacr, (R,S) -= zpsacr
+        QADD(IR, zpiacr);  // (I,R) += zpiacr, (R,I) -= zpiacr
+        if constexpr (BUD) {
+          b_psacr = zpsacr;
+          b_piacr = zpiacr;
         }
       }
 
       // 4.14 homogeneous freezing of cloud liquid (:2948-2960)
       {
         Real zfrzmax = mx((P.rthomo - t) * P.zrldcp, C(0.0));
-        if (zfrzmax > zepsec && qxfg_l > zepsec) {
-          D zfrz = mn(qxfg_l, D(zfrzmax));
-          QSUB(LI, zfrz);  // (I,L) += zfrz, (L,I) -= zfrz
-          if constexpr (BUD) bd.l[19] = -zfrz * zqtmst;  // :2958
-        }
-      }
-
-      // 4.9 riming (:2973-3017)
-      if (t <= P.rtt && zliqcld > zepsec && zsnowcld > zepsec && zcovptot > C(0.01)) {
-        Real zfallcorr = fallcorr_f;
-        Real zsnowrime = P.rcl_effrime * zcovptot * rdt * P.rcl_const7s * zfallcorr *
-                         mpowp<F32M, GEN, FAST_>(zrho * zsnowcld * P.rcl_const1s, P.rcl_const8s);
-        zsnowrime = mn(zsnowrime, C(1.0));
-        qb_sl = qb_sl + zsnowrime;
-        if constexpr (BUD) b_snowrime = zsnowrime;
-      }
-
-      // PSD slopes (:3026-3069), PSACR (:3084-3115), PIACR (:3171-3198)
-      if (t <= P.rtt && prainfrac < zepsec && zraincld > zepsec) {
-        Real zlamr = mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1r, (zrho * zraincld)), P.rcl_lam2r);
-        Real zn0r = P.rcl_x1r * mpowp<F32M, GEN, FAST_>(zlamr, P.rcl_x2r);
-        Real zlamr3 = zlamr * zlamr * zlamr;
-        if (zsnowcld > zepsec) {
-          Real zlams = mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1s, (zrho * zsnowcld)), P.rcl_lam2s);
-          Real zn0s = P.rcl_x1s;
-          Real zfalldiff = mx(xabs(fs_r - fs_s), DIV2((fs_r + fs_s), C(8.)));
-          Real zfac = DIV(P.rpi * P.rpi * P.rdenswat * zrho * zn0r * zn0s, (zlams * zlamr3));
-          Real zrat = DIV(zlamr, zlams);
-          Real zpsacr =
-              DIV(zcovptot * rdt * zfac * zfalldiff * ((C(0.5) * zrat + C(2.)) * zrat + C(5.)), zlamr3);
-          QSUB(RS, zpsacr);  // (S,R) += zpsacr, (R,S) -= zpsacr
-          if constexpr (BUD) b_psacr = zpsacr;
-        }
-        if (zicecld > zepsec) {
-          Real zlami = mpowp<F32M, GEN, FAST_>(DIV(P.rcl_lam1s, (zrho * zicecld)), P.rcl_lam2s);
-          Real zn0i = P.rcl_x1s;
-          Real zfalldiff = mx(xabs(fs_r - fs_i), DIV2((fs_r + fs_i), C(8.)));
-          Real zfac = DIV(P.rpi * P.rpi * P.rdenswat * C(0.1) * zrho * zn0r * zn0i, (zlami * zlamr3));
-          Real zrat = DIV(zlamr, zlami);
-          Real zpiacr =
-              DIV(zcovptot * rdt * zfac * zfalldiff * ((C(0.5) * zrat + C(2.)) * zrat + C(5.)), zlamr3);
-          QADD(IR, zpiacr);  // (I,R) += zpiacr, (R,I) -= zpiacr
-          if constexpr (BUD) b_piacr = zpiacr;
+        const bool c = zfrzmax > zepsec && qxfg_l > zepsec;
+        D zfrz = mn(qxfg_l, D(zfrzmax));
+        zfrz = c ? zfrz : 0.0;
+        QSUB(LI, zfrz);  // (I,L) += zfrz, (L,I) -= zfrz
+        if constexpr (BUD) {  // :2958
+          if (c) bd.l[19] = -zfrz * zqtmst;
         }
       }
 
       // 4.15 snow sublimation, ISUBLSNOW=1 (:3254-3318)
       {
-        Real zzrh = P.rprecrhmax + DIVY((C(1.0) - P.rprecrhmax) * zcovpmax, d1ma, r1ma);
-        zzrh = mn(mx(zzrh, P.rprecrhmax), C(1.0));
         Real zqe = DIVY((qv - a * zqsice), d1ma, r1ma);
         zqe = mx(C(0.0), mn(zqe, zqsice));
-        if (zcovpclr > zepsec && qxfg_s > zepsec && zqe < zzrh * zqsice) {
+        const bool subl = zcovpclr > zepsec && qxfg_s > zepsec && zqe < zrhmax * zqsice;
+        if (CSC_ANY(subl)) {
+          const D qs_div = subl ? qxfg_s : 1.0;
           Real aa = zcovptot * zdtgdp;
-          Real zpreclr = DIV(Real(qxfg_s) * zcovpclr, xsign(mx(xabs(aa), zepsilon), aa));
-          Real zbeta1 = DIV(DIVP(xsqrt(DIVY(pap_k, Real(paph_surf), rpsurf)), P.rvrfactor, P.rcp_rvrfactor) * zpreclr, mx(zcovpclr, zepsec));
+          Real zpreclr = DIV(Real(qs_div) * (subl ? zcovpclr : C(1.0)), xsign(mx(xabs(aa), zepsilon), aa));
+          Real zbeta1 = DIV(DIVP(root(zsigk), P.rvrfactor, P.rcp_rvrfactor) * zpreclr, mx(zcovpclr, zepsec));
           Real zbeta = P.rg * P.rpecons * mpow<F32M, FAST_>(zbeta1, C(0.5777));
           Real zdenom = C(1.0) + zbeta * rdt * zcorqsice;
           Real zdpr = DIV(zcovpclr * zbeta * (zqsice - zqe), zdenom) * zdp * P.zrg_r;
           Real zdpevap = zdpr * zdtgdp;
           if (spp && P.spp_on[CLOUDSC_SPP_SNOWSUBLIM]) zdpevap = zdpevap * Real(sppf[CLOUDSC_SPP_SNOWSUBLIM]);
           D zevap = mn(D(zdpevap), qxfg_s);
+          zevap = subl ? zevap : 0.0;
           QSUB(SV, zevap);  // (V,S) += zevap, (S,V) -= zevap
-          if constexpr (BUD) bd.i[17] = -zevap * zqtmst;  // :3304
-          zcovptot = mx(P.rcovpmin, zcovptot - mx(C(0.0), Real(DIV(D(zcovptot - a) * zevap, qxfg_s))));
+          if constexpr (BUD) {  // :3304
+            if (subl) bd.i[17] = -zevap * zqtmst;
+          }
+          const Real cov = mx(P.rcovpmin, zcovptot - mx(C(0.0), Real(DIV(D(zcovptot - a) * zevap, qs_div))));
+          zcovptot = subl ? cov : zcovptot;
           qxfg_s = qxfg_s - zevap;
         }
       }
@@ -1223,20 +1448,32 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
 #undef QADD
 #undef QSUB
 
+      // the sources wait for the tendencies
+      Parked<Real, PARK, 45> p_srcl(convsrce_l);
+      Parked<Real, PARK, 46> p_srci(convsrce_i);
+      Parked<Real, PARK, 47> p_srcr(convsrce_r);
+      Parked<Real, PARK, 48> p_srcs(convsrce_s);
+      Parked<Real, PARK, 49> p_falli(fallsrce_i);
+      Parked<Real, PARK, 50> p_fallr(fallsrce_r);
+      Parked<Real, PARK, 51> p_falls(fallsrce_s);
       // 5.1 cloud cover (:3429-3438)
       D zda;
+      Real zanew_b = C(0.0);
       {
         Real zanew = DIV((a + solac), (C(1.0) + solab));
         zanew = mn(zanew, C(1.0));
         if (zanew < P.ramin) zanew = C(0.0);
-        zda = D(zanew) - aorig;
-        zanewm1 = zanew;
+        zda = D(zanew) - p_aorig.get();
+        p_anew.set(zanew);
+        if constexpr (BUD) zanew_b = zanew;
       }
 
       // 5.2.1 sink truncation (:3455-3536), double: ratios, insertion sort
       // (IORDV, stable for ties), rows rescaled in sorted order
       const double qx[5] = {qlD, qiD, qrD, qsD, qvD};
-      {
+      if constexpr (FAST_) {
+        truncate_sinks<CHK_>(q, qx, divbad_);
+      } else {
         double ratio[5];
         sink_ratios<FAST_, CHK_>(q, qx, ratio, divbad_);
         double sr[5];
@@ -1303,10 +1540,9 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
         if (x_s < zepsecd) { x_v = x_v + x_s; x_s = 0.0; }
       }
       if constexpr (FAST_) REPORT_IF(!(x_l + x_i + x_r + x_s < 16.0));
-      qxnm1_l = Real(x_l);
-      qxnm1_i = Real(x_i);
-      qxnm1_r = Real(x_r);
-      qxnm1_s = Real(x_s);
+      p_xl.set(Real(x_l));
+      p_xi.set(Real(x_i));
+      p_xr.set(Real(x_r));
       qxn2d_l = x_l; qxn2d_i = x_i; qxn2d_r = x_r; qxn2d_s = x_s;
 
       // 5.3 fluxes to next level (:3658-3672)
@@ -1314,11 +1550,13 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
       pfplsx_r_n = Real(double(fallsink_r) * x_r * double(zrdtgdp));
       pfplsx_s_n = Real(double(fallsink_s) * x_s * double(zrdtgdp));
       if (pfplsx_s_n + pfplsx_r_n < zepsec) zcovptot = C(0.0);
+      p_cov.set(zcovptot);
+      p_covmax.set(zcovpmax);
 
       if constexpr (BUD) {  // diagnosed implicit rates (:3675-3699)
         bd.l[14] = -b_rainaut * x_l * zqtmst;
         bd.l[15] = -b_rainacc * x_l * zqtmst;
-        bd.cc[6] = -convsink_l * zanewm1 * zqtmst;
+        bd.cc[6] = -convsink_l * zanew_b * zqtmst;
         bd.l[6] = -convsink_l * x_l * zqtmst;
         bd.i[6] = -convsink_i * x_i * zqtmst;
         bd.i[13] = -fallsink_i * x_i * zqtmst;
@@ -1329,26 +1567,28 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
       // 6.1-6.3 tendencies (:3713-3769), double
       {
         D fq;
-        fq = D(convsrce_l) + 0.0 - (0.0 + D(convsink_l)) * x_l;
+        loc_t = p_loct.get();
+        loc_q = p_locq.get();
+        fq = D(p_srcl.get()) + 0.0 - (0.0 + D(convsink_l)) * x_l;
         loc_t = loc_t + PD.ralvdcp * (x_l - qlD - fq) * zqtmst;
-        loc_cl = 0.0 + (x_l - q0_l) * zqtmst;
-        fq = D(convsrce_i) + D(fallsrce_i) - (D(fallsink_i) + D(convsink_i)) * x_i;
+        loc_cl = 0.0 + (x_l - p_q0l.get()) * zqtmst;
+        fq = D(p_srci.get()) + D(p_falli.get()) - (D(fallsink_i) + D(convsink_i)) * x_i;
         loc_t = loc_t + PD.ralsdcp * (x_i - qiD - fq) * zqtmst;
-        loc_ci = 0.0 + (x_i - q0_i) * zqtmst;
-        fq = D(convsrce_r) + D(fallsrce_r) - (D(fallsink_r) + 0.0) * x_r;
+        loc_ci = 0.0 + (x_i - p_q0i.get()) * zqtmst;
+        fq = D(p_srcr.get()) + D(p_fallr.get()) - (D(fallsink_r) + 0.0) * x_r;
         loc_t = loc_t + PD.ralvdcp * (x_r - qrD - fq) * zqtmst;
-        loc_cr = 0.0 + (x_r - q0_r) * zqtmst;
-        fq = D(convsrce_s) + D(fallsrce_s) - (D(fallsink_s) + 0.0) * x_s;
+        loc_cr = 0.0 + (x_r - p_q0r.get()) * zqtmst;
+        fq = D(p_srcs.get()) + D(p_falls.get()) - (D(fallsink_s) + 0.0) * x_s;
         loc_t = loc_t + PD.ralsdcp * (x_s - qsD - fq) * zqtmst;
-        loc_cs = 0.0 + (x_s - q0_s) * zqtmst;
+        loc_cs = 0.0 + (x_s - p_q0s.get()) * zqtmst;
         loc_q = loc_q + (x_v - qvD) * zqtmst;
         loc_a = 0.0 + zda * zqtmst;
       }
       // 6.4 supersaturation check (:3765-3809), double
       {
-        D q_upd = pq_k + dt * (loc_q + cml_q);
-        D t_upd = pt_k + dt * (loc_t + cml_t);
-        D a_upd = pa_k + dt * (loc_a + cml_a);
+        D q_upd = p_pq.get() + dt * (loc_q + p_cq.get());
+        D t_upd = p_pt.get() + dt * (loc_t + p_ct.get());
+        D a_upd = p_pa.get() + dt * (loc_a + p_ca.get());
         if constexpr (FAST_) REPORT_IF(!(t_upd < 1024.0 && xabs(q_upd) < 16.0));
         D t_adj, q_adj, a_adj, l_adj, i_adj;
         supersatcheck<FAST_, CHK_>(t_upd, q_upd, a_upd, pap_kd, t_adj, q_adj, a_adj, l_adj, i_adj, divbad_);
@@ -1362,14 +1602,14 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
           bd.l[2] = l_adj * zqtmst;
           bd.i[2] = i_adj * zqtmst;
         }
-        D zl_adj = q0_l + loc_cl * dt;
+        D zl_adj = p_q0l.get() + loc_cl * dt;
         if (zl_adj < -PD.rlmin) nwarn++;
         if (zl_adj < 0.0) {
           loc_cl = loc_cl - zl_adj * zqtmst;
           loc_q = loc_q + zl_adj * zqtmst;
           loc_t = loc_t - PD.ralvdcp * zl_adj * zqtmst;
         }
-        D zi_adj = q0_i + loc_ci * dt;
+        D zi_adj = p_q0i.get() + loc_ci * dt;
         if (zi_adj < -PD.rlmin) nwarn++;
         if (zi_adj < 0.0) {
           loc_ci = loc_ci - zi_adj * zqtmst;
@@ -1380,7 +1620,8 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
       covp_out = zcovptot;
       if constexpr (OPT) {
         if (P.lrad_cloud_inhomog) {
-          const double pda = pa_k + zda;  // :3819-3823
+          const double q0_l = p_q0l.get(), q0_i = p_q0i.get();
+          const double pda = p_pa.get() + zda;  // :3819-3823
           if (pda > 0.001) anewp = mx(mx(pda, double(covp_out)), 0.1);
           if (q0_l + q0_i + plude_k > double(P.rlmin)) {  // :4112-4125
             ratfsd = DIV(plude_k, (plude_k + q0_l + q0_i));
@@ -1404,10 +1645,10 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
         if constexpr (PASS == kPassRedo) wr = wr && k >= kbud_l;
         if (wr)
           write_budgets(F, P, bd.cc, bd.l, bd.i, (size_t)ib * np * klev * F.kfldx + jl, np, klev, k, dt,
-                        zqtmst, double(zdp), double(zrho), opt(F.pvfa), opt(F.pdyna), double(pvfl),
-                        opt(F.pdynl), double(pvfi), opt(F.pdyni), opt(F.pdyns), opt(F.phrsw), opt(F.phrlw),
+                        zqtmst, double(zdp), double(zrho), opt(F.pvfa), opt(F.pdyna), p_vfl.get(),
+                        opt(F.pdynl), p_vfi.get(), opt(F.pdyni), opt(F.pdyns), opt(F.phrsw), opt(F.phrlw),
                         x_l, x_i, double(b_psdep), double(b_psacr), double(b_piacr), double(prainfrac), ktype,
-                        opti(F.kpbltype), opti(F.kctop), double(peis));
+                        opti(F.kpbltype), opti(F.kctop), ld(F.peis + o1));
       }
     }  // k >= ncldtop0
 
@@ -1451,8 +1692,7 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
 
     // precipitation fluxes at half level k (:4218-4224, 4297-4303)
     {
-      const size_t oh = o2h + (size_t)k * np;
-      const D fl = D(pfplsx_r) + 0.0, fn = D(pfplsx_s) + D(pfplsx_i);
+      const D fl = D(p_flr.get()) + 0.0, fn = D(p_fls.get()) + D(p_fli.get());
       if (active) {
         F.pfplsl[oh] = fl;
         F.pfplsn[oh] = fn;
@@ -1462,18 +1702,26 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
     }
     // DDH flux recurrences to half level k+1 (:4244-4292)
     {
-      const size_t oh1 = o2h + (size_t)(k + 1) * np;
+      const size_t oh1 = oh + np;
       const D zgdph_r = -PD.zrg_r * (paph_k1 - paph_k) * zqtmst;
-      const D sqrf = fsqlf + (qxn2d_r - q0_r) * zgdph_r;
-      const D cqrng = fcqlng + lneg_r * zgdph_r;
-      const D sqsf = fsqif + (qxn2d_s - q0_s) * zgdph_r;
-      const D cqsng = fcqnng + lneg_s * zgdph_r;
-      fsqlf = fsqlf + (qxn2d_l - q0_l + pvfl * dt) * zgdph_r + pludeli1;
-      fcqlng = fcqlng + lneg_l * zgdph_r;
-      fsqltur = fsqltur + pvfl * dt * zgdph_r;
-      fsqif = fsqif + (qxn2d_i - q0_i + pvfi * dt) * zgdph_r + pludeli2;
-      fcqnng = fcqnng + lneg_i * zgdph_r;
-      fsqitur = fsqitur + pvfi * dt * zgdph_r;
+      const D vfl = p_vfl.get(), vfi = p_vfi.get();
+      D fsqlf = p_fsqlf.get(), fsqif = p_fsqif.get(), fcqlng = p_fcqlng.get(), fcqnng = p_fcqnng.get();
+      const D sqrf = fsqlf + (qxn2d_r - p_q0r.get()) * zgdph_r;
+      const D cqrng = fcqlng + p_negr.get() * zgdph_r;
+      const D sqsf = fsqif + (qxn2d_s - p_q0s.get()) * zgdph_r;
+      const D cqsng = fcqnng + p_negs.get() * zgdph_r;
+      fsqlf = fsqlf + (qxn2d_l - p_q0l.get() + vfl * dt) * zgdph_r + p_dl.get();
+      fcqlng = fcqlng + p_negl.get() * zgdph_r;
+      const D fsqltur = p_fsqltur.get() + vfl * dt * zgdph_r;
+      fsqif = fsqif + (qxn2d_i - p_q0i.get() + vfi * dt) * zgdph_r + p_di.get();
+      fcqnng = fcqnng + p_negi.get() * zgdph_r;
+      const D fsqitur = p_fsqitur.get() + vfi * dt * zgdph_r;
+      p_fsqlf.set(fsqlf);
+      p_fsqif.set(fsqif);
+      p_fcqlng.set(fcqlng);
+      p_fcqnng.set(fcqnng);
+      p_fsqltur.set(fsqltur);
+      p_fsqitur.set(fsqitur);
       if (active) {
         F.pfsqlf[oh1] = fsqlf;
         F.pfsqif[oh1] = fsqif;
@@ -1489,23 +1737,23 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
     }
 
     // carry to level k+1
-    za_prev = a;
-    qr_prev = qr;
-    qs_prev = qs;
-    t_prev = t;
-    pap_prev = pap_k;
+    p_za.set(a);
+    p_qr.set(qr);
+    p_qs.set(qs);
+    p_t.set(t);
+    p_pap.set(pap_k);
     paph_k = paph_k1;
-    pmfu_k = pmfu_k1;
-    pmfd_k = pmfd_k1;
-    pfplsx_i = pfplsx_i_n;
-    pfplsx_r = pfplsx_r_n;
-    pfplsx_s = pfplsx_s_n;
+    p_pmfu.set(pmfu_k1);
+    p_pmfd.set(pmfd_k1);
+    p_fli.set(pfplsx_i_n);
+    p_flr.set(pfplsx_r_n);
+    p_fls.set(pfplsx_s_n);
     CSC_LEVEL_SYNC();
   }
   // precipitation fluxes at the surface half level KLEV+1
   {
     const size_t oh = o2h + (size_t)klev * np;
-    const D fl = D(pfplsx_r) + 0.0, fn = D(pfplsx_s) + D(pfplsx_i);
+    const D fl = D(p_flr.get()) + 0.0, fn = D(p_fls.get()) + D(p_fli.get());
     if (active) {
       F.pfplsl[oh] = fl;
       F.pfplsn[oh] = fn;
@@ -1513,7 +1761,7 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
       F.pfhpsn[oh] = -PD.rlstt * fn;
     }
   }
-  if (active) F.prainfrac_toprfz[o1] = D(prainfrac);
+  if (active) F.prainfrac_toprfz[o1] = D(p_frac.get());
   if (active && nwarn && F.ncounters && !(FAST_ && divbad_.bad())) atomic_add(F.ncounters, nwarn);
   if constexpr (FAST_) *bad = active && divbad_.bad();
   if constexpr (FAST_ && BUD) *kbud = kbud_l;
@@ -1527,5 +1775,7 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
 #undef RCP
 #undef DIVY
 #undef REPORT_IF
+#undef ZADVW
+#undef ZADVWD
 
 }  // namespace cloudsc

@@ -28,7 +28,9 @@ int num_variants();
 int default_variant();
 void variant_bounds(int v, int *maxt, int *minb);
 cudaError_t variant_attributes(int precision, int v, int *regs, int *local_bytes);
-cudaError_t max_local_bytes(size_t *out);
+cudaError_t prepare_kernels(size_t *max_local);
+int kernel_max_threads(int precision, int v, bool gen, int klev, bool sp);
+void pick_schedule(int precision, bool gen, int klev, bool sp, long long ncols, int sms, int *variant, int *threads);
 cudaError_t launch(int precision, int v, const Fields &f, const Shape &sh, int threads, int grid,
                    cudaStream_t stream, bool gen);
 bool params_allow_gen(const cloudsc_params &p, const Derived &d);
@@ -38,6 +40,7 @@ cudaError_t launch_state_increment(const IncFields &f, const Shape &sh, cudaStre
 cudaError_t launch_division_check(const double *a, const double *b, long long n, double *q, int *bad,
                                   cudaStream_t stream);
 cudaError_t launch_reciprocal_check(const double *b, long long n, double *y, int *bad, cudaStream_t stream);
+cudaError_t launch_sqrt_check(const double *x, long long n, double *y, int *bad, cudaStream_t stream);
 cudaError_t launch_sp(int precision, int v, const FieldsSP &f, const Shape &sh, int threads, int grid,
                       cudaStream_t stream, bool gen);
 }  // namespace cloudsc
@@ -56,9 +59,11 @@ unsigned long long g_gen_count = 0;  // parameter uploads so far
 constexpr int kMaxDev = 64;
 unsigned long long g_dev_gen[kMaxDev] = {0};
 // Launch schedule per precision (0 FP64, 1 FP32-mixed, 2 FP32 physics): compiled variant,
-// columns per CTA, persistent CTAs per SM (0: one CTA per column tile).
+// columns per CTA, persistent CTAs per SM (0: one CTA per column tile).  Until
+// one is set, each call takes the one pick_schedule gives for its size.
 struct Schedule {
   int variant, threads, ctas_per_sm;
+  bool set = false;
 };
 Schedule g_sched[3] = {{default_variant(), 448, 0}, {default_variant(), 448, 0}, {default_variant(), 448, 0}};
 
@@ -177,8 +182,8 @@ int ensure_params(int *dev_out) {
     // the device can hold (about half a GB on a B200 for a 2.6 KB frame), so
     // raise the stack limit to the largest kernel's frame (never lower it).
     size_t need = 0, cur = 0;
-    e = max_local_bytes(&need);
-    if (e != cudaSuccess) return fail(CLOUDSC_E_CUDA, "cudaFuncGetAttributes(column kernels)", e);
+    e = prepare_kernels(&need);
+    if (e != cudaSuccess) return fail(CLOUDSC_E_CUDA, "attributes of the column kernels", e);
     e = cudaDeviceGetLimit(&cur, cudaLimitStackSize);
     if (e != cudaSuccess) return fail(CLOUDSC_E_CUDA, "cudaDeviceGetLimit(stack size)", e);
     if (cur < need) {
@@ -458,7 +463,7 @@ int cloudsc_b200_set_schedule(int32_t precision, int32_t variant, int32_t thread
                                  "the variant's compiled limit");
   if (ctas_per_sm < 0 || ctas_per_sm > 32) return fail(CLOUDSC_E_SHAPE, "ctas_per_sm must be in [0,32]");
   std::lock_guard<std::mutex> lk(g_mu);
-  g_sched[precision] = {variant, threads_per_cta, ctas_per_sm};
+  g_sched[precision] = {variant, threads_per_cta, ctas_per_sm, true};
   return CLOUDSC_OK;
 }
 
@@ -491,6 +496,24 @@ int cloudsc_b200_set_launch(int32_t precision, int32_t threads_per_cta, int32_t 
     return fail(CLOUDSC_E_SHAPE, "threads_per_cta must be a multiple of 32, at least 32 and at most "
                                  "the largest compiled limit");
   return cloudsc_b200_set_schedule(precision, best, threads_per_cta, ctas_per_sm);
+}
+
+// The schedule of one call: the caller's, its CTA cut to what the kernel that
+// will run takes (parameters that rule out the GEN kernels, more than
+// kMaxLevFast levels and some forms have fewer builds), or pick_schedule's.
+static Schedule resolve_schedule(Schedule sc, int form, bool gen, const Shape &sh, bool sp, int *grid) {
+  const long long cols = (long long)sh.ngpblks * sh.nproma;
+  if (!sc.set) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    pick_schedule(form, gen, sh.klev, sp, cols, sms, &sc.variant, &sc.threads);
+    sc.ctas_per_sm = 0;
+  }
+  const int maxt = kernel_max_threads(form, sc.variant, gen, sh.klev, sp);
+  if (sc.threads > maxt) sc.threads = maxt;
+  *grid = grid_for(sc.ctas_per_sm, (int)((cols + sc.threads - 1) / sc.threads));
+  return sc;
 }
 
 // With the budget diagnostics on, the FP64 form that writes PEXTRA (kernel
@@ -531,13 +554,9 @@ static int launch_checked(int precision, const Fields &f, const Shape &sh, cudaS
                                          "arrays: use cloudsc_b200_batched_diag or cloudsc_b200_block");
     form = bud && opt ? 5 : (opt ? 4 : 3);
   }
-  // parameters that rule out the GEN kernels, more than kMaxLevFast levels
-  // and forms 3-5: a (448, 1) kernel, at most 448 columns per CTA
-  const bool small = !gen || sh.klev > kMaxLevFast || form > 2;
-  const int threads = (small && sc.threads > 448) ? 448 : sc.threads;
-  const int tiles = (int)(((long long)sh.ngpblks * sh.nproma + threads - 1) / threads);
-  const int grid = grid_for(sc.ctas_per_sm, tiles);
-  cudaError_t e = launch(form, sc.variant, f, sh, threads, grid, stream, gen);
+  int grid = 0;
+  const Schedule run = resolve_schedule(sc, form, gen, sh, false, &grid);
+  cudaError_t e = launch(form, run.variant, f, sh, run.threads, grid, stream, gen);
   if (e != cudaSuccess) return fail(CLOUDSC_E_CUDA, "kernel launch", e);
   return CLOUDSC_OK;
 }
@@ -854,11 +873,9 @@ int launch_sp_checked(int precision, const FieldsSP &f, const Shape &sh, cudaStr
     sc = g_sched[precision];
     gen = g_gen;
   }
-  int threads = sc.threads;
-  if ((sc.variant != 0 || !gen || sh.klev > kMaxLevFast) && threads > 448) threads = 448;
-  const int tiles = (int)(((long long)sh.ngpblks * sh.nproma + threads - 1) / threads);
-  const int grid = grid_for(sc.ctas_per_sm, tiles);
-  cudaError_t e = launch_sp(precision, sc.variant, f, sh, threads, grid, stream, gen);
+  int grid = 0;
+  const Schedule run = resolve_schedule(sc, precision, gen, sh, true, &grid);
+  cudaError_t e = launch_sp(precision, run.variant, f, sh, run.threads, grid, stream, gen);
   if (e != cudaSuccess) return fail(CLOUDSC_E_CUDA, "kernel launch", e);
   return CLOUDSC_OK;
 }
@@ -1538,6 +1555,15 @@ int cloudsc_b200_reciprocal_check(const double *b, int64_t n, double *y, int32_t
   if (n == 0) return CLOUDSC_OK;
   if (!b || !y || !bad) return fail(CLOUDSC_E_NULL, "a required array pointer is NULL");
   cudaError_t e = launch_reciprocal_check(b, (long long)n, y, bad, (cudaStream_t)stream);
+  if (e != cudaSuccess) return fail(CLOUDSC_E_CUDA, "kernel launch", e);
+  return CLOUDSC_OK;
+}
+
+int cloudsc_b200_sqrt_check(const double *x, int64_t n, double *y, int32_t *bad, void *stream) {
+  if (n < 0) return fail(CLOUDSC_E_SHAPE, "n < 0");
+  if (n == 0) return CLOUDSC_OK;
+  if (!x || !y || !bad) return fail(CLOUDSC_E_NULL, "a required array pointer is NULL");
+  cudaError_t e = launch_sqrt_check(x, (long long)n, y, bad, (cudaStream_t)stream);
   if (e != cudaSuccess) return fail(CLOUDSC_E_CUDA, "kernel launch", e);
   return CLOUDSC_OK;
 }

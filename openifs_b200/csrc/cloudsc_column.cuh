@@ -142,6 +142,42 @@ CSC_DEV double fast_quot(double a, double b, double y) {
 // All ones exactly for a divisor with an all-ones significand.
 CSC_DEV unsigned ones_word(double b) { return (hi_word(b) | 0xfff00000u) & lo_word(b); }
 
+// Branch-free correctly rounded square root for 2^-200 <= x < 2^200: the
+// estimate rsqrt.approx.ftz.f64 refined by two Goldschmidt steps on
+// g ~ sqrt(x), h ~ 1/(2 sqrt(x)) and one residual correction (Markstein 1990;
+// Handbook of Floating-Point Arithmetic, ch. 5).  That g is RN(sqrt(x)) is
+// then checked, not assumed: with u = ulp(g), sqrt(x) lies within u/2 of g
+// exactly when the residual x - g^2, exact in one fused multiply-add, is below
+// g u in magnitude (g u is a multiple of the residual's unit, so there is no
+// tie).  The one exception, x just below a power of 4 with g a power of two
+// (whose lower neighbour is only u/2 away), has an all-ones significand.
+// Both are reported to the rerun.
+template <bool FAST>
+CSC_DEV double csqrt(double x, DivCheck &dc) {
+#if defined(__CUDA_ARCH__)
+  if constexpr (FAST) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double g = __dmul_rn(x, y), h = __dmul_rn(0.5, y);
+    double r = __fma_rn(-g, h, 0.5);
+    g = __fma_rn(g, r, g);
+    h = __fma_rn(h, r, h);
+    r = __fma_rn(-g, h, 0.5);
+    g = __fma_rn(g, r, g);
+    h = __fma_rn(h, r, h);
+    g = __fma_rn(__fma_rn(-g, g, x), h, g);
+    const double d = __fma_rn(-g, g, x);
+    const double gu = __dmul_rn(g, __hiloint2double((__double2hiint(g) & 0x7ff00000) - (52 << 20), 0));
+    dc.pos |= fabs(d) < gu ? 0u : kPosRange;
+    const unsigned o = ones_word(x);
+    dc.ones = dc.ones > o ? dc.ones : o;
+    return g;
+  }
+#endif
+  (void)dc;
+  return sqrt(x);
+}
+
 // The two halves as one self-contained division with its own checks (the
 // division and reciprocal check entries): an all-ones divisor's reciprocal
 // gets its low significand bit set (which gives RN(1/b) = 2^(-E-1)(1 + 2^-52);
@@ -342,6 +378,32 @@ CSC_DEV double mpowb(const PowBase &b, double y) {
   if (WIN) return plibm_pow_with_log_win(b.x, y, b.lhi, b.llo);
   return plibm_pow_with_log(b.x, y, b.lhi, b.llo);
 #endif
+}
+// pow with the exponent 0.5 or 1.5 in the column code: in the FP64 fast pass
+// from csqrt (x^1.5 as plibm_pow1p5, for bases inside its range).
+template <bool F32, bool WIN>
+CSC_DEV double mroot(double x, DivCheck &dc) {
+#if !CSC_GLIBC
+  if (!F32 && WIN) return csqrt<WIN>(x, dc);
+#endif
+  (void)dc;
+  if (F32) return (double)xpow((float)x, 0.5f);
+  return xpow(x, 0.5);
+}
+template <bool F32, bool WIN>
+CSC_DEV double mroot3(double x, DivCheck &dc) {
+#if !CSC_GLIBC
+  if (!F32 && WIN) {
+    const double s = csqrt<WIN>(x, dc);
+    const double e = plibm_fma(-s, s, x);
+    const double p = x * s;
+    const double pe = plibm_fma(x, s, -p);
+    return p + (pe + (e * s) * 0.5);
+  }
+#endif
+  (void)dc;
+  if (F32) return (double)xpow((float)x, 1.5f);
+  return xpow(x, 1.5);
 }
 template <bool F32, bool WIN = false>
 CSC_DEV double mpow(double x, double y) {

@@ -18,6 +18,20 @@
 // warps of the CTA run the same stretch of the (very long) level code at the
 // same time and share the instruction cache.
 #define CSC_LEVEL_SYNC() __syncthreads()
+#define CSC_OPAQUE(X) asm volatile("" : "+l"(X))
+#define CSC_ANY(C) __any_sync(0xffffffffu, (C))
+// Next level's inputs into L2 while the level computes: the warps of a CTA
+// start a level together and all wait for its loads, so a DRAM round trip
+// shows in full.  Lane i owns input i: it prefetches the line of the warp's
+// first and last column (32 columns of a field are two lines), one
+// instruction each for all inputs together; both are addresses of elements
+// the warp reads.  FP64 at 262,144 columns, 384 columns per CTA: 9.83 -> 9.19
+// ms; one warp per SM 1.27 -> 1.22 ms (prefetching by every thread, 24
+// instructions a level, had been slower than none).
+#define CSC_PREFETCH_SETUP() \
+  PrefetchLines<FT, FAST_> pf_(F, ib, jl, s2, s2h, (size_t)np)
+#define CSC_PREFETCH(C, OFF) \
+  if (C) pf_.level(OFF)
 #include <type_traits>
 
 #include "cloudsc_column.cuh"
@@ -39,11 +53,65 @@ __device__ __forceinline__ const KParams<float> &KP<float>() { return c_kpf; }
 
 template <typename T>
 __device__ __forceinline__ T ld(const T *p) { return __ldg(p); }
+// This thread's column of the parking slots (Parked, cloudsc_body.cuh).
+extern __shared__ double csc_park[];
+__device__ __forceinline__ unsigned park_base() {
+  return (unsigned)__cvta_generic_to_shared(csc_park) + threadIdx.x * 8u;
+}
 __device__ __forceinline__ void atomic_add(uint32_t *p, uint32_t v) { atomicAdd(p, v); }
 __device__ __forceinline__ double xabs(double x) { return fabs(x); }
 __device__ __forceinline__ float xabs(float x) { return fabsf(x); }
 __device__ __forceinline__ double xsign(double a, double b) { return copysign(a, b); }
 __device__ __forceinline__ float xsign(float a, float b) { return copysignf(a, b); }
+
+template <typename FT, bool ON>
+struct PrefetchLines {
+  __device__ __forceinline__ PrefetchLines(const FT &, int, int, size_t, size_t, size_t) {}
+  __device__ __forceinline__ void level(size_t) const {}
+};
+template <typename FT>
+struct PrefetchLines<FT, true> {
+  static constexpr size_t ES = sizeof(*FT::pt);
+  const char *first, *last;  // element of level 0's successor, of the warp's first and last column
+  __device__ __forceinline__ PrefetchLines(const FT &F, int ib, int jl, size_t s2, size_t s2h, size_t np) {
+    const int lane = threadIdx.x & 31;
+    const void *b = nullptr;
+    size_t n = 1, m = 0, up = 0;  // species of the array, this lane's, extra levels down
+    switch (lane) {
+      case 0: b = F.pt; break;
+      case 1: b = F.pq; break;
+      case 2: b = F.pa; break;
+      case 3: b = F.cml_t; break;
+      case 4: b = F.cml_q; break;
+      case 5: b = F.cml_a; break;
+      case 6: case 7: case 8: case 9: b = F.cml_cld; n = 5; m = lane - 6; break;
+      case 10: case 11: case 12: case 13: b = F.pclv; n = 5; m = lane - 10; break;
+      case 14: b = F.pap; break;
+      case 15: b = F.paph; up = 1; break;
+      case 16: b = F.pvfl; break;
+      case 17: b = F.pvfi; break;
+      case 18: case 19: b = F.pludeli; n = 4; m = lane - 18; break;
+      case 20: b = F.pmfu; up = 1; break;  // read one level ahead
+      case 21: b = F.pmfd; up = 1; break;
+      case 22: b = F.plu; up = 1; break;
+      case 23: b = F.plude; break;
+      case 24: case 25: b = F.psnde; n = 2; m = lane - 24; break;
+      default: break;
+    }
+    const int ib0 = __shfl_sync(0xffffffffu, ib, 0), jl0 = __shfl_sync(0xffffffffu, jl, 0);
+    const int ib1 = __shfl_sync(0xffffffffu, ib, 31), jl1 = __shfl_sync(0xffffffffu, jl, 31);
+    const size_t sp = lane == 15 ? s2h : s2;
+    first = b ? (const char *)b + ES * (((size_t)ib0 * n + m) * sp + jl0 + up * np) : nullptr;
+    last = b ? (const char *)b + ES * (((size_t)ib1 * n + m) * sp + jl1 + up * np) : nullptr;
+  }
+  // off: (level) * NPROMA of the level to fetch
+  __device__ __forceinline__ void level(size_t off) const {
+    if (first) {
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(first + off * ES));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(last + off * ES));
+    }
+  }
+};
 
 }  // namespace cloudsc
 
@@ -51,6 +119,23 @@ __device__ __forceinline__ float xsign(float a, float b) { return copysignf(a, b
 #include "satadj_point.cuh"
 
 namespace cloudsc {
+
+// Where a kernel's long-lived values wait (Parked, cloudsc_body.cuh): in
+// shared memory for the 384- and 448-thread builds of the double-precision
+// forms, at most kParkSlots * 8 * 448 = 194 KB of the SM's 227; in registers
+// for the 256-thread build, whose 255 registers hold them (-1, which also
+// merges the processes of a group into one block), and for the others.
+// Parking against leaving them to the compiler's local-memory spills, FP64 at
+// 262,144 columns: 10.69 -> 10.00 ms (448 threads), 10.58 -> 10.0 (384);
+// FP32-mixed 8.51 -> 7.80.
+constexpr int park_threads(int form, int maxt, int minb, bool fast) {
+  if (!fast || form == 2 || minb != 1) return 0;
+  return maxt == 256 ? -1 : (maxt == 384 || maxt == 448 ? maxt : 0);
+}
+constexpr size_t park_bytes(int form, int maxt, int minb, bool fast) {
+  const int p = park_threads(form, maxt, minb, fast);
+  return p > 0 ? (size_t)p * 8 * kParkSlots : 0;
+}
 
 // Columns are numbered g = ib * NPROMA + jl over all blocks and dealt to CTAs
 // in tiles of blockDim.x consecutive columns (a warp reads 32 neighbouring
@@ -81,11 +166,12 @@ namespace cloudsc {
 // split PEXTRA's levels between them: cloudsc_column, kbud).
 template <int FORM, int MAXT, int MINB, typename FT = Fields, bool GEN = false, bool FAST = false>
 __global__ void __launch_bounds__(MAXT, MINB) cloudsc_kernel(FT F, Shape sh) {
-  // Let ptxas place part of the register spills in shared memory instead of
+  // Without parking: let ptxas place part of the register spills in shared memory instead of
   // local memory (a PTX pragma; the spill slots it moves no longer go
   // through L1/L2).  With the shared-memory tables, FP64: 15.29 ms vs
   // 15.75 ms; FP32-mixed: 11.28 ms vs 11.72 ms.
-  asm volatile(".pragma \"enable_smem_spilling\";");
+  constexpr int PARK = park_threads(FORM, MAXT, MINB, FAST);
+  if constexpr (PARK <= 0) asm volatile(".pragma \"enable_smem_spilling\";");
   plibm_load_tables();
   const long long ncols = (long long)sh.ngpblks * sh.nproma;
   const long long ntiles = (ncols + blockDim.x - 1) / blockDim.x;
@@ -105,7 +191,7 @@ __global__ void __launch_bounds__(MAXT, MINB) cloudsc_kernel(FT F, Shape sh) {
         double plude_in[kMaxLevFast];
         bool bad = false;
         int kbud = sh.klev;
-        cloudsc_column<double, false, BUD, OPT, FT, GEN, kPassFast>(F, sh, ib, jl, active, &bad, plude_in, &kbud);
+        cloudsc_column<double, false, BUD, OPT, FT, GEN, kPassFast, PARK>(F, sh, ib, jl, active, &bad, plude_in, &kbud);
         if (__syncthreads_or(bad))
           cloudsc_column<double, false, BUD, OPT, FT, GEN, kPassRedo>(F, sh, ib, jl, bad, nullptr, plude_in,
                                                                        &kbud);
@@ -116,7 +202,7 @@ __global__ void __launch_bounds__(MAXT, MINB) cloudsc_kernel(FT F, Shape sh) {
       typedef std::conditional_t<FORM == 2, float, double> Real;
       double plude_in[kMaxLevFast];
       bool bad = false;
-      cloudsc_column<Real, FORM != 0, false, false, FT, GEN, kPassFast>(F, sh, ib, jl, active, &bad, plude_in);
+      cloudsc_column<Real, FORM != 0, false, false, FT, GEN, kPassFast, PARK>(F, sh, ib, jl, active, &bad, plude_in);
       // The rerun takes the whole CTA (the column code holds a CTA barrier
       // at every level); only the columns that reported store anything.
       if (__syncthreads_or(bad))
@@ -288,6 +374,15 @@ __global__ void __launch_bounds__(kSatadjThreads) reciprocal_check_kernel(const 
   }
 }
 
+// csqrt of the fast pass on n values, and its report.
+__global__ void __launch_bounds__(kSatadjThreads) sqrt_check_kernel(const double *x, long long n, double *y, int *bad) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    DivCheck dc;
+    y[i] = csqrt<true>(x[i], dc);
+    bad[i] = dc.bad() ? 1 : 0;
+  }
+}
+
 }  // namespace cloudsc
 
 // ---------------------------------------------------------------------------
@@ -340,148 +435,197 @@ void variant_bounds(int v, int *maxt, int *minb) {
   *minb = kVariants[v].minb;
 }
 
-template <int FORM, bool GEN, bool FAST>
-static const void *kernel_ptr_form(int v) {
+// A compiled column kernel: its function, the largest CTA it takes and the
+// dynamic shared memory of its parking slots.
+struct ColumnKernel {
+  const void *f;
+  int maxt;
+  size_t smem;
+};
+template <int FORM, int MAXT, int MINB, typename FT, bool GEN, bool FAST>
+static ColumnKernel column_kernel() {
+  return {(const void *)cloudsc_kernel<FORM, MAXT, MINB, FT, GEN, FAST>, MAXT, park_bytes(FORM, MAXT, MINB, FAST)};
+}
+template <int FORM>
+static ColumnKernel kernel_form(int v) {
   switch (v) {
-    case 0: return (const void *)cloudsc_kernel<FORM, kVariants[0].maxt, kVariants[0].minb, Fields, GEN, FAST>;
-    case 1: return (const void *)cloudsc_kernel<FORM, kVariants[1].maxt, kVariants[1].minb, Fields, GEN, FAST>;
-    case 2: return (const void *)cloudsc_kernel<FORM, kVariants[2].maxt, kVariants[2].minb, Fields, GEN, FAST>;
-    case 3: return (const void *)cloudsc_kernel<FORM, kVariants[3].maxt, kVariants[3].minb, Fields, GEN, FAST>;
-    case 4: return (const void *)cloudsc_kernel<FORM, kVariants[4].maxt, kVariants[4].minb, Fields, GEN, FAST>;
-    case 5: return (const void *)cloudsc_kernel<FORM, kVariants[5].maxt, kVariants[5].minb, Fields, GEN, FAST>;
-    default: return nullptr;
+    case 0: return column_kernel<FORM, kVariants[0].maxt, kVariants[0].minb, Fields, true, true>();
+    case 1: return column_kernel<FORM, kVariants[1].maxt, kVariants[1].minb, Fields, true, true>();
+    case 2: return column_kernel<FORM, kVariants[2].maxt, kVariants[2].minb, Fields, true, true>();
+    case 3: return column_kernel<FORM, kVariants[3].maxt, kVariants[3].minb, Fields, true, true>();
+    case 4: return column_kernel<FORM, kVariants[4].maxt, kVariants[4].minb, Fields, true, true>();
+    default: return column_kernel<FORM, kVariants[5].maxt, kVariants[5].minb, Fields, true, true>();
   }
 }
-static_assert(kNumVariants == 6, "kernel_ptr_form lists every variant");
+static_assert(kNumVariants == 6, "kernel_form lists every variant");
 // Forms 0-2 exist in every variant with GEN and FAST (the parameters of every
 // known configuration allow GEN); for parameters that do not, in the (448, 1)
 // variant with FAST only; for KLEV above kMaxLevFast, in the (448, 1) variant
-// without either (`launch` then runs that one, at most 448 columns per CTA).
-// Forms 3-5 (budgets, SPP, inhomogeneity, aerosols) exist in the (448, 1)
-// variant only, in the same three builds; every variant maps to it.
-template <int FORM>
-static const void *kernel_ptr_opt_form(bool gen, bool fast) {
-  if (!fast) return (const void *)cloudsc_kernel<FORM, 448, 1, Fields, false, false>;
-  if (!gen) return (const void *)cloudsc_kernel<FORM, 448, 1, Fields, false, true>;
-  return (const void *)cloudsc_kernel<FORM, 448, 1, Fields, true, true>;
+// without either.  Forms 3-5 (budgets, SPP, inhomogeneity, aerosols) and the
+// single-precision interface exist in fewer variants with GEN and FAST; the
+// others map to the (448, 1) one.
+template <int FORM, typename FT>
+static ColumnKernel kernel_general(bool fast) {
+  return fast ? column_kernel<FORM, 448, 1, FT, false, true>() : column_kernel<FORM, 448, 1, FT, false, false>();
 }
-static const void *kernel_ptr(int precision, int v, bool gen, bool fast) {
-  if (precision <= 2 && !fast) {
+template <int FORM>
+static ColumnKernel kernel_opt_form(int v, bool gen, bool fast) {
+  if (!fast || !gen) return kernel_general<FORM, Fields>(fast);
+  if (v == 3) return column_kernel<FORM, 256, 1, Fields, true, true>();
+  return column_kernel<FORM, 448, 1, Fields, true, true>();
+}
+template <int FORM>
+static ColumnKernel kernel_sp_form(int v, bool gen, bool fast) {
+  if (!fast || !gen) return kernel_general<FORM, FieldsSP>(fast);
+  if (v == 0) return column_kernel<FORM, 640, 1, FieldsSP, true, true>();
+  if (v == 2) return column_kernel<FORM, 384, 1, FieldsSP, true, true>();
+  if (v == 3) return column_kernel<FORM, 256, 1, FieldsSP, true, true>();
+  return column_kernel<FORM, 448, 1, FieldsSP, true, true>();
+}
+static ColumnKernel find_kernel(int precision, int v, bool gen, bool fast) {
+  if (precision <= 2 && (!gen || !fast)) {
     switch (precision) {
-      case 0: return (const void *)cloudsc_kernel<0, 448, 1, Fields, false, false>;
-      case 1: return (const void *)cloudsc_kernel<1, 448, 1, Fields, false, false>;
-      case 2: return (const void *)cloudsc_kernel<2, 448, 1, Fields, false, false>;
-    }
-  }
-  if (!gen && precision <= 2) {
-    switch (precision) {
-      case 0: return (const void *)cloudsc_kernel<0, 448, 1, Fields, false, true>;
-      case 1: return (const void *)cloudsc_kernel<1, 448, 1, Fields, false, true>;
-      case 2: return (const void *)cloudsc_kernel<2, 448, 1, Fields, false, true>;
+      case 0: return kernel_general<0, Fields>(fast);
+      case 1: return kernel_general<1, Fields>(fast);
+      default: return kernel_general<2, Fields>(fast);
     }
   }
   switch (precision) {
-    case 0: return kernel_ptr_form<0, true, true>(v);
-    case 1: return kernel_ptr_form<1, true, true>(v);
-    case 2: return kernel_ptr_form<2, true, true>(v);
-    case 3: return kernel_ptr_opt_form<3>(gen, fast);
-    case 4: return kernel_ptr_opt_form<4>(gen, fast);
-    case 5: return kernel_ptr_opt_form<5>(gen, fast);
-    default: return nullptr;
+    case 0: return kernel_form<0>(v);
+    case 1: return kernel_form<1>(v);
+    case 2: return kernel_form<2>(v);
+    case 3: return kernel_opt_form<3>(v, gen, fast);
+    case 4: return kernel_opt_form<4>(v, gen, fast);
+    case 5: return kernel_opt_form<5>(v, gen, fast);
+    default: return {nullptr, 0, 0};
+  }
+}
+static ColumnKernel find_kernel_sp(int precision, int v, bool gen, bool fast) {
+  switch (precision) {
+    case 0: return kernel_sp_form<0>(v, gen, fast);
+    case 1: return kernel_sp_form<1>(v, gen, fast);
+    case 2: return kernel_sp_form<2>(v, gen, fast);
+    default: return {nullptr, 0, 0};
   }
 }
 
-// The single-precision interface's kernels: forms 0-2 in the two variants
-// the tuned schedules use, (640, 1) and (448, 1), with GEN and FAST; in the
-// (448, 1) variant with FAST only, and without either for KLEV above
-// kMaxLevFast.  Other variants map to the (448, 1) kernel (see launch_sp).
-template <int FORM>
-static const void *kernel_ptr_sp_form(int v, bool gen, bool fast) {
-  if (!fast) return (const void *)cloudsc_kernel<FORM, 448, 1, FieldsSP, false, false>;
-  if (!gen) return (const void *)cloudsc_kernel<FORM, 448, 1, FieldsSP, false, true>;
-  if (v == 0) return (const void *)cloudsc_kernel<FORM, 640, 1, FieldsSP, true, true>;
-  return (const void *)cloudsc_kernel<FORM, 448, 1, FieldsSP, true, true>;
+// The largest CTA of the kernel a call runs with variant v.
+int kernel_max_threads(int precision, int v, bool gen, int klev, bool sp) {
+  const bool fast = klev <= kMaxLevFast;
+  return (sp ? find_kernel_sp(precision, v, gen, fast) : find_kernel(precision, v, gen, fast)).maxt;
 }
-static const void *kernel_ptr_sp(int precision, int v, bool gen, bool fast) {
-  switch (precision) {
-    case 0: return kernel_ptr_sp_form<0>(v, gen, fast);
-    case 1: return kernel_ptr_sp_form<1>(v, gen, fast);
-    case 2: return kernel_ptr_sp_form<2>(v, gen, fast);
-    default: return nullptr;
+
+// Variant and CTA size for a call of ncols columns when the caller has set no
+// schedule.  A launch is one CTA per SM at a time in every variant, its CTAs
+// run in waves, and the time of a wave grows little with the columns in it
+// (one warp alone is bound by the latency of its own chain): so the columns
+// are spread evenly over the SMs and the waves, and the variant is the one
+// with the smallest waves * (time of a wave of that CTA).  The wave times are
+// those measured at 137 levels, in microseconds as base + slope per warp
+// (FP64; the other forms follow the same order):
+//   (256, 1), 255 registers:  2 warps 1230, 4 1273, 8 1428
+//   (384, 1), 168 registers:  2 warps 1362, 4 1472, 8 1681, 12 1926
+//   (448, 1), 128 registers:  2 warps 1554, 4 1678, 8 1873, 12 2122, 14 2415
+// The lines cross where the 255-register build runs out of threads: below 257
+// columns per SM it is the fastest at every size, above that one wave of more
+// warps beats two of it.  3,200 columns: CTAs of 32 on 100 SMs, 1.21 ms,
+// where 448 per CTA on 8 SMs took 2.0; 262,144: 5 waves of 384, 9.4 ms, against
+// 4 of 448, 9.7, and 7 of 256, 10.0.
+void pick_schedule(int precision, bool gen, int klev, bool sp, long long ncols, int sms, int *variant, int *threads) {
+  struct Cost {
+    int v;
+    double base, slope;
+  };
+  static const Cost costs[] = {{3, 1165.0, 32.0}, {2, 1250.0, 56.0}, {1, 1420.0, 68.0}};
+  double best = 0.0;
+  *variant = kDefaultVariant;
+  *threads = 0;
+  for (const Cost &c : costs) {
+    const int maxt = kernel_max_threads(precision, c.v, gen, klev, sp);
+    if (maxt != kVariants[c.v].maxt) continue;  // this form has no such build
+    const long long per_wave = (long long)sms * maxt;
+    const long long waves = (ncols + per_wave - 1) / per_wave;
+    const long long ctas = waves * sms;
+    int t = (int)((ncols + ctas - 1) / ctas);
+    t = (t + 31) / 32 * 32;
+    const double cost = (double)waves * (c.base + c.slope * (t / 32));
+    if (*threads == 0 || cost < best) {
+      best = cost;
+      *variant = c.v;
+      *threads = t;
+    }
   }
 }
 
 // Registers and local (spill) bytes per thread of variant v (needs a device).
 cudaError_t variant_attributes(int precision, int v, int *regs, int *local_bytes) {
-  const void *k = kernel_ptr(precision, v, true, true);
-  if (!k) return cudaErrorInvalidValue;
+  const ColumnKernel k = find_kernel(precision, v, true, true);
+  if (!k.f) return cudaErrorInvalidValue;
   cudaFuncAttributes a;
-  cudaError_t e = cudaFuncGetAttributes(&a, k);
+  cudaError_t e = cudaFuncGetAttributes(&a, k.f);
   if (e != cudaSuccess) return e;
   *regs = a.numRegs;
   *local_bytes = (int)a.localSizeBytes;
   return cudaSuccess;
 }
 
-// The largest local memory (stack frame) per thread of any column kernel:
-// the spill slots and the fast pass's copy of the PLUDE inputs.
-cudaError_t max_local_bytes(size_t *out) {
+// Once per device: allow every column kernel its parking slots, and find the
+// largest local memory (stack frame) per thread of any of them: the spill
+// slots and the fast pass's copy of the PLUDE inputs.
+cudaError_t prepare_kernels(size_t *max_local) {
   size_t m = 0;
-  auto see = [&](const void *k) -> cudaError_t {
-    if (!k) return cudaSuccess;
+  auto see = [&](const ColumnKernel &k) -> cudaError_t {
+    if (!k.f) return cudaSuccess;
     cudaFuncAttributes a;
-    cudaError_t e = cudaFuncGetAttributes(&a, k);
+    cudaError_t e = cudaFuncGetAttributes(&a, k.f);
     if (e == cudaSuccess && a.localSizeBytes > m) m = a.localSizeBytes;
+    if (e == cudaSuccess && k.smem)
+      e = cudaFuncSetAttribute(k.f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
     return e;
   };
   for (int v = 0; v < kNumVariants; ++v)
     for (int g = 0; g < 2; ++g)
       for (int f = 0; f < 2; ++f) {
         for (int prec = 0; prec <= 5; ++prec) {
-          cudaError_t e = see(kernel_ptr(prec, v, g != 0, f != 0));
+          cudaError_t e = see(find_kernel(prec, v, g != 0, f != 0));
           if (e != cudaSuccess) return e;
         }
         for (int prec = 0; prec <= 2; ++prec) {
-          cudaError_t e = see(kernel_ptr_sp(prec, v, g != 0, f != 0));
+          cudaError_t e = see(find_kernel_sp(prec, v, g != 0, f != 0));
           if (e != cudaSuccess) return e;
         }
       }
-  *out = m;
+  *max_local = m;
   return cudaSuccess;
 }
 
 // Launch variant v of the kernel: precision 0 = FP64, 1 = FP32-mixed,
 // 2 = FP32 physics, 3-5 the FP64 forms with budgets / SPP and inhomogeneity;
-// gen: the parameters allow the GEN kernels (forms 0-2 otherwise run the
-// (448, 1) kernel without GEN, at most 448 columns per CTA, as they do for
-// KLEV above kMaxLevFast; forms 3-5 always run a (448, 1) kernel).
+// gen: the parameters allow the GEN kernels.  threads: at most
+// kernel_max_threads.
 cudaError_t launch(int precision, int v, const Fields &f, const Shape &sh, int threads, int grid,
                    cudaStream_t stream, bool gen) {
-  const bool fast = sh.klev <= kMaxLevFast;
-  if (v < 0 || v >= kNumVariants || threads > kVariants[v].maxt) return cudaErrorInvalidConfiguration;
-  if ((!gen || !fast || precision > 2) && threads > 448) return cudaErrorInvalidConfiguration;
-  const void *k = kernel_ptr(precision, v, gen, fast);
-  if (!k) return cudaErrorInvalidValue;
+  if (v < 0 || v >= kNumVariants) return cudaErrorInvalidConfiguration;
+  const ColumnKernel k = find_kernel(precision, v, gen, sh.klev <= kMaxLevFast);
+  if (!k.f) return cudaErrorInvalidValue;
+  if (threads > k.maxt) return cudaErrorInvalidConfiguration;
   Fields fa = f;
   Shape sa = sh;
   void *args[] = {&fa, &sa};
-  return cudaLaunchKernel(k, dim3(grid), dim3(threads), args, 0, stream);
+  return cudaLaunchKernel(k.f, dim3(grid), dim3(threads), args, k.smem, stream);
 }
 
-// Launch form `precision` (0-2) of the single-precision interface with the
-// schedule of variant v: variant 0 keeps its (640, 1) kernel; every other
-// variant runs the (448, 1) kernel with at most 448 columns per CTA.
+// The same for form `precision` (0-2) of the single-precision interface.
 cudaError_t launch_sp(int precision, int v, const FieldsSP &f, const Shape &sh, int threads, int grid,
                       cudaStream_t stream, bool gen) {
-  const bool fast = sh.klev <= kMaxLevFast;
-  if (v < 0 || v >= kNumVariants || threads > kVariants[v].maxt) return cudaErrorInvalidConfiguration;
-  if ((v != 0 || !gen || !fast) && threads > 448) return cudaErrorInvalidConfiguration;
-  const void *k = kernel_ptr_sp(precision, v, gen, fast);
-  if (!k) return cudaErrorInvalidValue;
+  if (v < 0 || v >= kNumVariants) return cudaErrorInvalidConfiguration;
+  const ColumnKernel k = find_kernel_sp(precision, v, gen, sh.klev <= kMaxLevFast);
+  if (!k.f) return cudaErrorInvalidValue;
+  if (threads > k.maxt) return cudaErrorInvalidConfiguration;
   FieldsSP fa = f;
   Shape sa = sh;
   void *args[] = {&fa, &sa};
-  return cudaLaunchKernel(k, dim3(grid), dim3(threads), args, 0, stream);
+  return cudaLaunchKernel(k.f, dim3(grid), dim3(threads), args, k.smem, stream);
 }
 
 // Launch CLOUD_SATADJ over every point of the batched arrays: a grid of
@@ -545,6 +689,14 @@ cudaError_t launch_reciprocal_check(const double *b, long long n, double *y, int
   if (blocks > 148LL * 16) blocks = 148LL * 16;
   if (blocks < 1) blocks = 1;
   reciprocal_check_kernel<<<(unsigned)blocks, kSatadjThreads, 0, stream>>>(b, n, y, bad);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_sqrt_check(const double *x, long long n, double *y, int *bad, cudaStream_t stream) {
+  long long blocks = (n + kSatadjThreads - 1) / kSatadjThreads;
+  if (blocks > 148LL * 16) blocks = 148LL * 16;
+  if (blocks < 1) blocks = 1;
+  sqrt_check_kernel<<<(unsigned)blocks, kSatadjThreads, 0, stream>>>(x, n, y, bad);
   return cudaGetLastError();
 }
 
