@@ -372,30 +372,46 @@ __global__ void adamw_kernel(float *p, float *g, float *m, float *v, int taps, i
 }
 
 // ---------------------------------------------------------------- guard
-// One thread per column.  Pass 1 over the levels: de-normalise, refill
-// condensates the step would drive negative (from vapour, with the latent
-// heat), write the outputs, accumulate the budgets and the guard quantities.
-// Pass 2: the column-constant LOC_Q and LOC_T shifts that close the water and
-// enthalpy budgets with the predicted surface precipitation, and the enthalpy
-// fluxes.
-// 64 registers (8 CTAs of 128 per SM) with a small spill, against 96
-// registers and 5 CTAs per SM uncapped.
-__global__ void __launch_bounds__(128, 8) post_kernel(Cols C, const float *__restrict__ y, int nheads, cs_guard gd,
-                                                     int *nflagged, int *flagged, float4 *diag) {
+// A CTA takes 32 neighbouring columns, one per lane, and its warps share the
+// levels (a contiguous run each): one thread per column left 49,152 columns
+// on three warps per scheduler, each walking 137 levels of dependent loads.
+// Pass 1: de-normalise, refill condensates the step would drive negative
+// (from vapour, with the latent heat), write the outputs, accumulate the
+// budgets and the guard quantities of the warp's levels; the partial sums meet
+// in shared memory in level order.  Pass 2: the column-constant LOC_Q and LOC_T
+// shifts that close the water and enthalpy budgets with the predicted surface
+// precipitation; LOC_Q and LOC_T wait for them in shared memory (KEEP; for more
+// levels than fit, in their own arrays).
+constexpr int PW = 8;     // warps per CTA
+constexpr int PSUM = 12;  // partial sums per column
+constexpr size_t post_smem(int klev, bool keep) {
+  return (size_t)PSUM * PW * 32 * 8 + 4 * 32 * 8 + (keep ? (size_t)klev * 32 * 2 * 8 : 0);
+}
+constexpr size_t POST_SMEM_MAX = 160 * 1024;
+
+template <bool KEEP>
+__global__ void __launch_bounds__(32 * PW) post_kernel(Cols C, const float *__restrict__ y, int nheads, cs_guard gd,
+                                                       int *nflagged, int *flagged, float4 *diag) {
+  extern __shared__ double psm[];
+  double *part = psm;                      // [PSUM][PW][32]
+  double *tot = psm + PSUM * PW * 32;      // qshift, tshift, pr, ps [4][32]
+  double *kq = tot + 4 * 32, *kt = kq + (size_t)C.c.klev * 32;
   const int ys = 64;
   const int ncol = C.c.nproma * C.c.ngpblks, lp = C.c.lp, klev = C.c.klev;
   const int k0 = gd.ncldtop - 1;  // first level of CLOUDSC's level loop
   const double dt = gd.ptsphy, rg = gd.rg;
   const double ral[4] = {gd.ralvdcp, gd.ralsdcp, gd.ralvdcp, gd.ralsdcp};  // l, i, r, s
-  for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < ncol; col += gridDim.x * blockDim.x) {
-    const cs_columns &c = C.c;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int ka = klev * w / PW, kb = klev * (w + 1) / PW;
+  const cs_columns &c = C.c;
+  for (int col0 = blockIdx.x * 32; col0 < ncol; col0 += gridDim.x * 32) {
+    const int col = col0 + lane;
+    const bool on = col < ncol;
     double w_lhs = 0.0, w_abs = 0.0, e_lhs = 0.0, e_abs = 0.0;
     double s_l = 0.0, s_i = 0.0, s_r = 0.0, s_s = 0.0, mass = 0.0, spread2 = 0.0;
     double refill = 0.0, cond = 0.0;
-    int spread_n = 0;
-    const bool ldcum = c.ldcum[C.o1(col)] != 0;
-    double pr = 0.0, ps = 0.0;
-    for (int k = 0; k < klev; ++k) {
+    const bool ldcum = on && c.ldcum[C.o1(col)] != 0;
+    for (int k = ka; on && k < kb; ++k) {
       const size_t r = (size_t)col * lp + 2 + k;
       // channels 0..11 of each head as three 16-byte loads (rows are 256 bytes)
       __align__(16) float ya[12], yb[12];
@@ -412,10 +428,7 @@ __global__ void __launch_bounds__(128, 8) post_kernel(Cols C, const float *__res
         float a = ya[i];
         if (nheads == 2) {
           const float b = yb[i];
-          if (i < 7) {
-            spread2 += (double)(a - b) * (double)(a - b);
-            ++spread_n;
-          }
+          if (i < 7) spread2 += (double)(a - b) * (double)(a - b);
           a = 0.5f * (a + b);
         }
         yv[i] = a * gd.out_scale[i];
@@ -442,14 +455,29 @@ __global__ void __launch_bounds__(128, 8) post_kernel(Cols C, const float *__res
       c.loc_a[o] = la;
 #pragma unroll
       for (int m = 0; m < 4; ++m) c.loc_cld[C.o3(col, m, 5, k)] = lc[m];
-      c.loc_q[o] = lq;
-      c.loc_t[o] = lt;
-      if (k + 1 < klev) {
-        c.pfplsl[C.oh(col, k + 1)] = fmax((double)yv[7], 0.0);
-        c.pfplsn[C.oh(col, k + 1)] = fmax((double)yv[8], 0.0);
+      if (KEEP) {
+        kq[k * 32 + lane] = lq;
+        kt[k * 32 + lane] = lt;
       } else {
-        pr = fmax((double)yv[7], 0.0);
-        ps = fmax((double)yv[8], 0.0);
+        c.loc_q[o] = lq;
+        c.loc_t[o] = lt;
+      }
+      const double fl = fmax((double)yv[7], 0.0), fn = fmax((double)yv[8], 0.0);
+      const size_t o1 = C.oh(col, k + 1);
+      c.pfplsl[o1] = fl;
+      c.pfplsn[o1] = fn;
+      c.pfhpsl[o1] = -gd.rlvtt * fl;
+      c.pfhpsn[o1] = -gd.rlstt * fn;
+      if (k + 1 == klev) {
+        tot[2 * 32 + lane] = fl;
+        tot[3 * 32 + lane] = fn;
+      }
+      if (k == 0) {
+        const size_t o0 = C.oh(col, 0);
+        c.pfplsl[o0] = 0.0;
+        c.pfplsn[o0] = 0.0;
+        c.pfhpsl[o0] = -gd.rlvtt * 0.0;
+        c.pfhpsn[o0] = -gd.rlstt * 0.0;
       }
       // convective detrainment exactly as CLOUDSC applies it (cloudsc.F90:1362-1398)
       if (k >= k0 && k + 1 < klev) {
@@ -472,39 +500,50 @@ __global__ void __launch_bounds__(128, 8) post_kernel(Cols C, const float *__res
       e_abs += fabs(dpg * lt);
       mass += dpg;
     }
-    // water: shift LOC_Q so that sum dp/g (q + condensates) = S - P
-    const double w_rhs = (s_l + s_i + s_r + s_s) - (pr + ps);
-    const double w_res = w_lhs - w_rhs;
-    const double w_raw = fabs(w_res) / (w_abs + fabs(w_rhs) + 1e-30);
-    const double qshift = w_res / mass;
-    // enthalpy: shift LOC_T (the LOC_Q shift does not enter this budget)
-    const double e_rhs = gd.ralvdcp * (pr - s_l - s_r) + gd.ralsdcp * (ps - s_i - s_s);
-    const double e_res = e_lhs - e_rhs;
-    const double e_raw = fabs(e_res) / (e_abs + fabs(e_rhs) + 1e-30);
-    const double tshift = e_res / mass;
-    for (int k = 0; k < klev; ++k) {
-      const size_t o = C.o2(col, k);
-      c.loc_q[o] = c.loc_q[o] - qshift;
-      c.loc_t[o] = c.loc_t[o] - tshift;
+    {
+      const double v[PSUM] = {w_lhs, w_abs, e_lhs, e_abs, s_l, s_i, s_r, s_s, mass, spread2, refill, cond};
+#pragma unroll
+      for (int i = 0; i < PSUM; ++i) part[(i * PW + w) * 32 + lane] = v[i];
     }
-    c.pfplsl[C.oh(col, klev)] = pr;
-    c.pfplsn[C.oh(col, klev)] = ps;
-    c.pfplsl[C.oh(col, 0)] = 0.0;
-    c.pfplsn[C.oh(col, 0)] = 0.0;
-    for (int k = 0; k <= klev; ++k) {
-      const size_t oo = C.oh(col, k);
-      c.pfhpsl[oo] = -gd.rlvtt * c.pfplsl[oo];
-      c.pfhpsn[oo] = -gd.rlstt * c.pfplsn[oo];
+    __syncthreads();
+    if (w == 0 && on) {
+      double v[PSUM];
+#pragma unroll
+      for (int i = 0; i < PSUM; ++i) {
+        v[i] = part[i * PW * 32 + lane];
+        for (int q = 1; q < PW; ++q) v[i] += part[(i * PW + q) * 32 + lane];
+      }
+      const double pr = tot[2 * 32 + lane], ps = tot[3 * 32 + lane];
+      // water: shift LOC_Q so that sum dp/g (q + condensates) = S - P
+      const double w_rhs = (v[4] + v[5] + v[6] + v[7]) - (pr + ps);
+      const double w_res = v[0] - w_rhs;
+      const double w_raw = fabs(w_res) / (v[1] + fabs(w_rhs) + 1e-30);
+      tot[lane] = w_res / v[8];
+      // enthalpy: shift LOC_T (the LOC_Q shift does not enter this budget)
+      const double e_rhs = gd.ralvdcp * (pr - v[4] - v[6]) + gd.ralsdcp * (ps - v[5] - v[7]);
+      const double e_res = v[2] - e_rhs;
+      const double e_raw = fabs(e_res) / (v[3] + fabs(e_rhs) + 1e-30);
+      tot[32 + lane] = e_res / v[8];
+      const double spread = nheads == 2 ? sqrt(v[9] / (7 * klev)) : 0.0;
+      const double refill_rel = v[10] / (v[11] + 1e-12);
+      const bool flag = refill_rel > gd.neg_tol || w_raw > gd.closure_tol || e_raw > gd.closure_tol ||
+                        (nheads == 2 && spread > gd.spread_tol);
+      if (diag) diag[col] = make_float4((float)w_raw, (float)e_raw, (float)spread, (float)refill_rel);
+      if (flag) {
+        const int slot = atomicAdd(nflagged, 1);
+        if (slot < gd.capacity) flagged[slot] = col;
+      }
     }
-    const double spread = spread_n ? sqrt(spread2 / spread_n) : 0.0;
-    const double refill_rel = refill / (cond + 1e-12);
-    const bool flag = refill_rel > gd.neg_tol || w_raw > gd.closure_tol || e_raw > gd.closure_tol ||
-                      (nheads == 2 && spread > gd.spread_tol);
-    if (diag) diag[col] = make_float4((float)w_raw, (float)e_raw, (float)spread, (float)refill_rel);
-    if (flag) {
-      const int slot = atomicAdd(nflagged, 1);
-      if (slot < gd.capacity) flagged[slot] = col;
+    __syncthreads();
+    {
+      const double qshift = tot[lane], tshift = tot[32 + lane];
+      for (int k = ka; on && k < kb; ++k) {
+        const size_t o = C.o2(col, k);
+        c.loc_q[o] = (KEEP ? kq[k * 32 + lane] : c.loc_q[o]) - qshift;
+        c.loc_t[o] = (KEEP ? kt[k * 32 + lane] : c.loc_t[o]) - tshift;
+      }
     }
+    __syncthreads();
   }
 }
 
@@ -650,9 +689,21 @@ int cs_post(const cs_columns *c, const float *y, int32_t nheads, const cs_guard 
     return CS_E_ARG;
   Cols C{*c};
   const int ncol = c->nproma * c->ngpblks;
-  post_kernel<<<grid_1d(ncol, 128), 128, 0, (cudaStream_t)stream>>>(C, y, nheads, *g, nflagged, flagged,
-                                                                      (float4 *)diag);
-  return cudaGetLastError() == cudaSuccess ? CS_OK : CS_E_CUDA;
+  const bool keep = post_smem(c->klev, true) <= POST_SMEM_MAX;
+  const size_t smem = post_smem(c->klev, keep);
+  const int tiles = (ncol + 31) / 32;
+  const int grid = tiles < 148 * 16 ? tiles : 148 * 16;
+  cudaError_t e = cudaSuccess;
+  if (keep) {
+    e = cudaFuncSetAttribute(post_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)
+      post_kernel<true><<<grid, 32 * PW, smem, (cudaStream_t)stream>>>(C, y, nheads, *g, nflagged, flagged,
+                                                                        (float4 *)diag);
+  } else {
+    post_kernel<false><<<grid, 32 * PW, smem, (cudaStream_t)stream>>>(C, y, nheads, *g, nflagged, flagged,
+                                                                       (float4 *)diag);
+  }
+  return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? CS_OK : CS_E_CUDA;
 }
 
 int cs_move_columns(const cs_colarray *arrays, int32_t narr, int32_t nproma_src, int32_t nproma_dst,
