@@ -24,8 +24,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # contraction anywhere, so the kernels, the host-side constant set-up and
 # plibm.h evaluate exactly the operations written.
 NVCC_FLAGS = ["-O3", "-lineinfo", "--fmad=false", "-std=c++17", "-Xcompiler", "-fPIC",
-              "-Xcompiler", "-O2", "-Xcompiler", "-ffp-contract=off", "--expt-relaxed-constexpr",
-              "-split-compile=8"]  # the many column-kernel builds of one file, in parallel
+              "-Xcompiler", "-O2", "-Xcompiler", "-ffp-contract=off", "--expt-relaxed-constexpr"]
 
 
 def _nvcc():

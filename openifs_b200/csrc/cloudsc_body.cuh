@@ -1,5 +1,5 @@
 // Per-column CLOUDSC body (device code), shared by the GPU kernels
-// (cloudsc_kernels.cu) and by the host build of the same code that the tests
+// (cloudsc_kernels.cuh) and by the host build of the same code that the tests
 // compare against the oracle (tests/hostemu).  The including file provides:
 //   CSC_DEV           function qualifiers (__device__ __forceinline__ on the GPU)
 //   KP<Real>()        the KParams<Real> block, c_kd the KParamsD block

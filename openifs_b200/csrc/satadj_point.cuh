@@ -15,9 +15,22 @@
 // Quantities the reference forms but never uses at this configuration
 // (ZQSLIQ, ZCORQSLIQ, ZEVAPLIMMIX, ZQSLIM, the _UPD liquid/ice/Koop values,
 // ZRDTGDP, ZRHO, ZDZ, in-cloud condensate) are not computed.
+//
+// FAST_ (the kernel's first pass): the branch-free divisions and the windowed
+// exponentials of the column kernels (cloudsc_column.cuh).  The point's own
+// checks bound their operands -- every temperature in [128, 1024) K, the
+// pressures, the layer thickness, the humidities and the amounts, and the
+// parameters by fast_pass_params_ok -- and a point that fails one is computed
+// again with IEEE division and plibm's full exponential, so the bits are the
+// same for every input.
 #pragma once
 
 namespace cloudsc {
+
+#define SDIV(A, B) cdiv<FAST_, false>(A, B, dc)
+#define SRCP(B) crcp<FAST_, false>(B, dc)
+#define SREPORT_IF(C) \
+  if constexpr (FAST_) dc.pos |= (C) ? kPosRange : 0u
 
 // Saturation pieces of fcttre.func.h at one temperature (both exponentials
 // evaluated once).
@@ -25,23 +38,26 @@ struct Sat {
   double el, ei, alfa;
   bool delta;
 };
-CSC_DEV Sat sat_at(const KParams<double> &k, double t) {
+template <bool FAST_>
+CSC_DEV Sat sat_at(const KParams<double> &k, double t, DivCheck &dc) {
   Sat s;
-  s.el = xexp(k.r3les * (t - k.rtt) / (t - k.r4les));
+  SREPORT_IF(!(t >= 128.0 && t < 1024.0));
+  s.el = mexp<false, FAST_>(SDIV(k.r3les * (t - k.rtt), t - k.r4les));
   const double x = (mx(k.rtice, mn(k.rtwat, t)) - k.rtice) * k.rtwat_rtice_r;
   s.alfa = mn(1.0, x * x);
   s.delta = copysign(1.0, t - k.rtt) > 0.0;
   s.ei = 0.0;
-  if (!s.delta || s.alfa < 1.0) s.ei = xexp(k.r3ies * (t - k.rtt) / (t - k.r4ies));
+  if (!s.delta || s.alfa < 1.0) s.ei = mexp<false, FAST_>(SDIV(k.r3ies * (t - k.rtt), t - k.r4ies));
   return s;
 }
 CSC_DEV double sat_foeewm(const KParams<double> &k, const Sat &s) {
   const double w = (s.alfa < 1.0) ? s.alfa * s.el + (1.0 - s.alfa) * s.ei : s.el;
   return k.r2es * w;
 }
-CSC_DEV double sat_foedem(const KParams<double> &k, const Sat &s, double t) {
+template <bool FAST_>
+CSC_DEV double sat_foedem(const KParams<double> &k, const Sat &s, double t, DivCheck &dc) {
   const double xl = t - k.r4les, xi = t - k.r4ies;
-  return s.alfa * k.r5alvcp * (1.0 / (xl * xl)) + (1.0 - s.alfa) * k.r5alscp * (1.0 / (xi * xi));
+  return s.alfa * k.r5alvcp * SRCP(xl * xl) + (1.0 - s.alfa) * k.r5alscp * SRCP(xi * xi);
 }
 CSC_DEV double sat_foeldcpm(const KParams<double> &k, const Sat &s) {
   return s.alfa * k.ralvdcp + (1.0 - s.alfa) * k.ralsdcp;
@@ -49,17 +65,18 @@ CSC_DEV double sat_foeldcpm(const KParams<double> &k, const Sat &s) {
 
 // QSATMIXADJ (cloud_satadj.F90:948-1017): two Newton steps towards the
 // mixed-phase saturation; returns the adjusted humidity.
-CSC_DEV double qsatmixadj(const KParams<double> &k, double pt, double pq, double pp) {
+template <bool FAST_>
+CSC_DEV double qsatmixadj(const KParams<double> &k, double pt, double pq, double pp, DivCheck &dc) {
   double zt = pt, zq = pq;
-  const double zp_r = 1.0 / pp;
+  const double zp_r = SRCP(pp);
 #pragma unroll 1
   for (int ji = 0; ji < 2; ++ji) {
-    const Sat s = sat_at(k, zt);
+    const Sat s = sat_at<FAST_>(k, zt, dc);
     const double zfoeet = mn(sat_foeewm(k, s) * zp_r, 0.5);
-    const double zcor = 1.0 / (1.0 - k.retv * zfoeet);
+    const double zcor = SRCP(1.0 - k.retv * zfoeet);
     const double zqsat = zfoeet * zcor;
-    const double zcorqs = 1.0 + zqsat * zcor * sat_foedem(k, s, zt);
-    const double zcond = (zq - zqsat) / zcorqs;
+    const double zcorqs = 1.0 + zqsat * zcor * sat_foedem<FAST_>(k, s, zt, dc);
+    const double zcond = SDIV(zq - zqsat, zcorqs);
     zt = zt + sat_foeldcpm(k, s) * zcond;
     zq = zq - zcond;
   }
@@ -69,23 +86,25 @@ CSC_DEV double qsatmixadj(const KParams<double> &k, double pt, double pq, double
 // CLOUD_SUPERSATCHECK with KFTLIQICE = 2 (cloud_supersatcheck.F90:111-223):
 // the condensate ZCOND = PL_ADJ + PI_ADJ and the cloud increase ZDA.  The
 // caller only needs their sum, which is ZCOND + 0 in either phase branch.
+template <bool FAST_>
 CSC_DEV void supersat_cond(const KParams<double> &k, double pt, double pq, double pa, double pp,
-                           double &cond, double &da) {
+                           double &cond, double &da, DivCheck &dc) {
+  SREPORT_IF(!(pt < 1024.0 && xabs(pq) < 16.0));
   const double zepsec = 1.E-14;
   double zda = 0.0;
   const double zt = mx(pt, 160.0);
   const double za = mx(mn(pa, 1.0), 0.0);
-  const double zp_r = 1.0 / pp;
-  const Sat s = sat_at(k, zt);
+  const double zp_r = SRCP(pp);
+  const Sat s = sat_at<FAST_>(k, zt, dc);
   const double zfoeeliq = mn((k.r2es * s.el) * zp_r, 0.5);
   const double foeew = s.delta ? k.r2es * s.el : k.r2es * s.ei;
   const double zfoeeice = mn(foeew * zp_r, 0.5);
   const double zfokoop = mn(zfoeeice * (k.rkoop1 - k.rkoop2 * zt), zfoeeliq);
-  double zqsliqk = zfokoop / (1.0 - k.retv * zfokoop);
+  double zqsliqk = SDIV(zfokoop, 1.0 - k.retv * zfokoop);
   const double zfoeemix = mn(sat_foeewm(k, s) * zp_r, 0.5);
-  const double zcor = 1.0 / (1.0 - k.retv * zfoeemix);
+  const double zcor = SRCP(1.0 - k.retv * zfoeemix);
   const double zqsmix = zfoeemix * zcor;
-  const double zcorqsmix = 1.0 + zqsmix * zcor * sat_foedem(k, s, zt);
+  const double zcorqsmix = 1.0 + zqsmix * zcor * sat_foedem<FAST_>(k, s, zt, dc);
   zqsliqk = 0.5 * (zqsliqk + zqsmix);
   double zqslim = za * zqsmix + (1.0 - za) * zqsliqk;
   double zcond = mx(pq - zqslim, 0.0);
@@ -94,7 +113,7 @@ CSC_DEV void supersat_cond(const KParams<double> &k, double pt, double pq, doubl
     zda = (1.0 - za) * zfaci;
     const double za_upd = za + zda;
     zqslim = za_upd * zqsmix + (1.0 - za_upd) * zqsliqk;
-    zcond = (pq - zqslim) / zcorqsmix;
+    zcond = SDIV(pq - zqslim, zcorqsmix);
   }
   const bool liquid = pt + sat_foeldcpm(k, s) * zcond >= k.rthomo;
   cond = (liquid ? zcond : 0.0) + (liquid ? 0.0 : zcond);
@@ -105,12 +124,14 @@ CSC_DEV void supersat_cond(const KParams<double> &k, double pt, double pq, doubl
 // all five adjustments, liquid and ice split by the mixed-phase fraction.
 CSC_DEV void supersatcheck_kft1(const KParams<double> &k, double pt, double pq, double pa, double pp,
                                 double &t_adj, double &q_adj, double &a_adj, double &l_adj, double &i_adj) {
+  constexpr bool FAST_ = false;
+  DivCheck dc;
   const double zepsec = 1.E-14;
   double zda = 0.0;
   const double zt = mx(pt, 160.0);
   const double za = mx(mn(pa, 1.0), 0.0);
   const double zp_r = 1.0 / pp;
-  const Sat s = sat_at(k, zt);
+  const Sat s = sat_at<FAST_>(k, zt, dc);
   const double zfoeeliq = mn((k.r2es * s.el) * zp_r, 0.5);
   const double foeew = s.delta ? k.r2es * s.el : k.r2es * s.ei;
   const double zfoeeice = mn(foeew * zp_r, 0.5);
@@ -119,7 +140,7 @@ CSC_DEV void supersatcheck_kft1(const KParams<double> &k, double pt, double pq, 
   const double zfoeemix = mn(sat_foeewm(k, s) * zp_r, 0.5);
   const double zcor = 1.0 / (1.0 - k.retv * zfoeemix);
   const double zqsmix = zfoeemix * zcor;
-  const double zcorqsmix = 1.0 + zqsmix * zcor * sat_foedem(k, s, zt);
+  const double zcorqsmix = 1.0 + zqsmix * zcor * sat_foedem<FAST_>(k, s, zt, dc);
   zqsliqk = 0.5 * (zqsliqk + zqsmix);
   double zqslim = za * zqsmix + (1.0 - za) * zqsliqk;
   double zcond = mx(pq - zqslim, 0.0);
@@ -141,12 +162,13 @@ CSC_DEV void supersatcheck_kft1(const KParams<double> &k, double pt, double pq, 
 // (arguments are that point's inputs; psurf = PAPH(KLEV+1)).  nwarn is
 // incremented for each negative-condensate warning the reference prints
 // (:828, :836).
-CSC_DEV void satadj_point(const KParams<double> &k, double dt, double zqtmst, double pap, double paph_k,
+template <bool FAST_>
+CSC_DEV void satadj_pass(const KParams<double> &k, double dt, double zqtmst, double pap, double paph_k,
                           double paph_k1, double psurf, double pt, double pq, double pa, double pl,
                           double pi, double cml_t, double cml_q, double cml_a, double cml_l,
                           double cml_i, double phrsw, double phrlw, double vdf_t, double vdf_q,
                           double pludeli3, double pludeli4, double pvervel, double &loc_t,
-                          double &loc_q, double &loc_a, double &loc_l, double &loc_i, int &nwarn) {
+                          double &loc_q, double &loc_a, double &loc_l, double &loc_i, int &nwarn, DivCheck &dc) {
   const double zepsec = 1.E-14;
   // updated state (:357-366)
   const double zt = pt + dt * cml_t;
@@ -157,9 +179,20 @@ CSC_DEV void satadj_point(const KParams<double> &k, double dt, double zqtmst, do
   za = mx(0.0, mn(1.0, za));
   // T and q forcing (:384-413)
   const double zdp = paph_k1 - paph_k;
-  const double zgdp = k.rg / zdp;
+  if constexpr (FAST_) {
+    if (k.rcp_force) dc.acc = ~0u;
+    see_pos(pap, -8, dc);
+    see_pos(psurf, -8, dc);
+    see_pos(zdp, -10, dc);
+    see(pq, dc);
+    see(pa, dc);
+    see(zl, dc);
+    SREPORT_IF(!(xabs(pq) + xabs(zq) + xabs(pa) + xabs(zl) + xabs(zi) < 16.0));
+  }
+  const double zgdp = SDIV(k.rg, zdp);
   const double zdtgdp = dt * zgdp;
-  const double zdtdp = k.zrdcp * pt / pap;
+  const double zp_r = SRCP(pap);
+  const double zdtdp = cdivk<FAST_, false>(k.zrdcp * pt, pap, zp_r, dc);
   const double zdpmxdt = zdp * zqtmst;
   const double zwtot = mn(zdpmxdt, mx(-zdpmxdt, pvervel));
   const double zzzdt = phrsw + phrlw;
@@ -170,46 +203,46 @@ CSC_DEV void satadj_point(const KParams<double> &k, double dt, double zqtmst, do
   const double zli = zl + zi;
   double zliqfrac = 0.0, zicefrac = 0.0;
   if (zli > k.rlmin) {
-    zliqfrac = zl / zli;
+    zliqfrac = SDIV(zl, zli);
     zicefrac = 1.0 - zliqfrac;
   }
   double zrhc = k.ramid;
-  const double zsigk = pap / psurf;
+  const double zsigk = SDIV(pap, psurf);
   if (zsigk > 0.8) {
-    const double x = (zsigk - 0.8) / 0.2;
+    const double x = cdivk<FAST_, false>(zsigk - 0.8, 0.2, 1.0 / 0.2, dc);
     zrhc = k.ramid + (1.0 - k.ramid) * (x * x);
   }
   // saturation of the start-of-step state (:474-501)
-  const double zp_r = 1.0 / pap;
-  const Sat s0 = sat_at(k, pt);
+  const Sat s0 = sat_at<FAST_>(k, pt, dc);
   const double zfoeeliq = mn((k.r2es * s0.el) * zp_r, 0.5);
   const double zfoeeice = mn((s0.delta ? k.r2es * s0.el : k.r2es * s0.ei) * zp_r, 0.5);
   const double zfokoop = mn(zfoeeice * (k.rkoop1 - k.rkoop2 * pt), zfoeeliq);
-  double zqsliqk = zfokoop / (1.0 - k.retv * zfokoop);
+  double zqsliqk = SDIV(zfokoop, 1.0 - k.retv * zfokoop);
   double zfoeemix = mn(sat_foeewm(k, s0) * zp_r, 0.5);
-  double zcor = 1.0 / (1.0 - k.retv * zfoeemix);
+  double zcor = SRCP(1.0 - k.retv * zfoeemix);
   const double zqsmix = zfoeemix * zcor;
   zqsliqk = 0.5 * (zqsliqk + zqsmix);
   // saturation of the updated state (:507-542): ZQSMIX_UPD, ZCORQSMIX_UPD
-  const Sat s1 = sat_at(k, zt);
+  const Sat s1 = sat_at<FAST_>(k, zt, dc);
   zfoeemix = mn(sat_foeewm(k, s1) * zp_r, 0.5);
-  zcor = 1.0 / (1.0 - k.retv * zfoeemix);
+  zcor = SRCP(1.0 - k.retv * zfoeemix);
   const double zqsmix_upd = zfoeemix * zcor;
-  const double zcorqsmix_upd = 1.0 + zqsmix_upd * zcor * sat_foedem(k, s1, zt);
+  const double zcorqsmix_upd = 1.0 + zqsmix_upd * zcor * sat_foedem<FAST_>(k, s1, zt, dc);
   // condensation/evaporation from dqsat/dt (:574-593)
   const double zttmp = mx(pt + zdtforce, 160.0);
   const double zqtmp = zqsmix + zdqforce;
-  const double zdqs = qsatmixadj(k, zttmp, zqtmp, pap) - zqtmp;
+  SREPORT_IF(!(xabs(zqtmp) < 16.0));
+  const double zdqs = qsatmixadj<FAST_>(k, zttmp, zqtmp, pap, dc) - zqtmp;
   // clear-air condensation, new cloud (:602-655)
   double env_l = 0.0, env_i = 0.0, zacond = 0.0;
   if (zdqs <= -k.rlmin && pa < 1.0 - zepsec) {
-    double zqe = (pq - pa * zqsmix) / mx(zepsec, 1.0 - pa);
+    double zqe = SDIV(pq - pa * zqsmix, mx(zepsec, 1.0 - pa));
     zqe = mx(0.0, zqe);
     if (zqe >= zrhc * zqsliqk && zqe < zqsliqk) {
-      zacond = -(1.0 - pa) * zdqs / mx(2.0 * (zqsliqk - zqe), zepsec);
+      zacond = SDIV(-(1.0 - pa) * zdqs, mx(2.0 * (zqsliqk - zqe), zepsec));
       zacond = mn(zacond, 1.0 - pa);
       double zlcond_env = -zdqs * 0.5 * zacond;
-      const double zzdl = 2.0 * (zqsliqk - zqe) / mx(zepsec, 1.0 - pa);
+      const double zzdl = SDIV(2.0 * (zqsliqk - zqe), mx(zepsec, 1.0 - pa));
       if (zdqs < -zzdl) {
         const double zlcondlim = (pa - 1.0) * zdqs - zqsliqk + pq;
         zlcond_env = mn(zlcond_env, zlcondlim);
@@ -228,7 +261,7 @@ CSC_DEV void satadj_point(const KParams<double> &k, double dt, double zqtmst, do
   double cld_l = 0.0, cld_i = 0.0;
   if (pa > zepsec && zdqs <= -k.rlmin) {
     double zlcond_cld = mx(-zdqs, 0.0);
-    const double zcdmax = mx((zq - zqsmix_upd) / zcorqsmix_upd, 0.0);
+    const double zcdmax = mx(SDIV(zq - zqsmix_upd, zcorqsmix_upd), 0.0);
     zlcond_cld = mn(zlcond_cld, zcdmax);
     zlcond_cld = pa * zlcond_cld;
     if (zlcond_cld < k.rlmin) zlcond_cld = 0.0;
@@ -251,7 +284,7 @@ CSC_DEV void satadj_point(const KParams<double> &k, double dt, double zqtmst, do
   if (zanew < k.ramin) zanew = 0.0;
   // supersaturation check (:767-793)
   double zcond, zsupsata;
-  supersat_cond(k, zt_upd, zq_upd, zanew, pap, zcond, zsupsata);
+  supersat_cond<FAST_>(k, zt_upd, zq_upd, zanew, pap, zcond, zsupsata, dc);
   double supl, supi;
   if (zt_upd > k.rthomo) {
     supl = zcond;
@@ -290,5 +323,21 @@ CSC_DEV void satadj_point(const KParams<double> &k, double dt, double zqtmst, do
   loc_l = tl;
   loc_i = ti;
 }
+
+// The point with IEEE division and plibm's full exponential.
+CSC_DEV void satadj_point(const KParams<double> &k, double dt, double zqtmst, double pap, double paph_k,
+                          double paph_k1, double psurf, double pt, double pq, double pa, double pl,
+                          double pi, double cml_t, double cml_q, double cml_a, double cml_l,
+                          double cml_i, double phrsw, double phrlw, double vdf_t, double vdf_q,
+                          double pludeli3, double pludeli4, double pvervel, double &loc_t,
+                          double &loc_q, double &loc_a, double &loc_l, double &loc_i, int &nwarn) {
+  DivCheck dc;
+  satadj_pass<false>(k, dt, zqtmst, pap, paph_k, paph_k1, psurf, pt, pq, pa, pl, pi, cml_t, cml_q, cml_a, cml_l, cml_i,
+                     phrsw, phrlw, vdf_t, vdf_q, pludeli3, pludeli4, pvervel, loc_t, loc_q, loc_a, loc_l, loc_i, nwarn, dc);
+}
+
+#undef SDIV
+#undef SRCP
+#undef SREPORT_IF
 
 }  // namespace cloudsc
