@@ -150,6 +150,16 @@ typedef struct cs_adam {
  * ([taps][k][n], taps reversed: the backward-data operand) when not NULL. */
 int cs_adamw(float *p, float *g, float *m, float *v, int32_t taps, int32_t n, int32_t k, const cs_adam *hp,
              void *w, void *wt, void *stream);
+/* The same step for `count` (at most CS_ADAM_MAX) tensors in one launch, each
+ * with its own weight decay (hp->weight_decay is not read). */
+#define CS_ADAM_MAX 16
+typedef struct cs_adam_tensor {
+  float *p, *g, *m, *v;
+  void *w, *wt;
+  int32_t taps, n, k;
+  float weight_decay;
+} cs_adam_tensor;
+int cs_adamw_tensors(const cs_adam_tensor *tensors, int32_t count, const cs_adam *hp, void *stream);
 
 /* Guard of the surrogate's output.  The small parameter structs (cs_norm,
  * cs_adam, cs_guard) and the w16 / scale16 arrays of the calls above and

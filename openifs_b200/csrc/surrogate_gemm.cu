@@ -20,6 +20,7 @@
 #include <stdint.h>
 #include <string.h>
 #include <mutex>
+#include <type_traits>
 #include "tc_gemm.cuh"
 #include "cloudsc_surrogate.h"
 
@@ -246,28 +247,88 @@ __device__ __forceinline__ void ld256_nc(const void *p, uint32_t *w) {
                : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
                : "l"(p));
 }
-// 32 bf16 of row-major storage as 2 x 32-byte loads.
-__device__ __forceinline__ void load_bf16x32(const __nv_bfloat16 *p, float (&f)[32]) {
+// 32 bf16 (64 bytes) of each lane's row, moved by lane pairs: rows r and r + 1
+// belong to lanes 2j and 2j + 1, and in each access the pair covers one row,
+// the even lane its first 32 bytes and the odd lane the other 32, so that a
+// warp touches 16 rows instead of 32 (the load/store pipe, at a line an
+// access, was the busiest unit).  Each lane exchanges the half it does not
+// move.  Used where an epilogue moves three arrays or more (training: 1.77 ->
+// 1.66 ms for four steps of 512 columns at width 128); with two the exchange
+// costs what it saves (inference: 7.79 against 7.85 ms for 49,152 columns),
+// and each lane moves its own row.  `even` is the pair's even row at the warp's columns, `ld` the row
+// length; every lane of the warp calls (ok_e, ok_o: the rows exist).
+__device__ __forceinline__ void load_bf16x32(const __nv_bfloat16 *even, size_t ld, bool odd, bool ok_e, bool ok_o,
+                                             float (&f)[32]) {
+  __align__(32) uint32_t a[8] = {0}, b[8] = {0}, t[16];
+  const int off = odd ? 16 : 0;
+  if (ok_e) ld256_nc(even + off, a);
+  if (ok_o) ld256_nc(even + ld + off, b);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? a[i] : b[i], 1);
+    t[i] = odd ? got : a[i];
+    t[8 + i] = odd ? b[i] : got;
+  }
+#pragma unroll
+  for (int i = 0; i < 32; ++i) f[i] = __bfloat162float(((const __nv_bfloat16 *)t)[i]);
+}
+// The same, each lane its own row.
+__device__ __forceinline__ void load_own32(const __nv_bfloat16 *p, float (&f)[32]) {
   __align__(32) __nv_bfloat16 t[32];
   ld256_nc(p, (uint32_t *)t);
   ld256_nc(p + 16, (uint32_t *)t + 8);
 #pragma unroll
   for (int i = 0; i < 32; ++i) f[i] = __bfloat162float(t[i]);
 }
-// 32 bf16 as 2 x 32-byte stores.
-__device__ __forceinline__ void store_bf16x32(__nv_bfloat16 *p, const __nv_bfloat16 (&h)[32]) {
+__device__ __forceinline__ void store_own32(__nv_bfloat16 *p, const __nv_bfloat16 (&h)[32]) {
   st256(p, (const uint32_t *)h);
   st256(p + 16, (const uint32_t *)h + 8);
 }
+__device__ __forceinline__ void store_bf16x32(__nv_bfloat16 *even, size_t ld, bool odd, bool ok_e, bool ok_o,
+                                              const __nv_bfloat16 (&h)[32]) {
+  const uint32_t *w = (const uint32_t *)h;
+  uint32_t a[8], b[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? w[i] : w[8 + i], 1);
+    a[i] = odd ? got : w[i];
+    b[i] = odd ? w[8 + i] : got;
+  }
+  const int off = odd ? 16 : 0;
+  if (ok_e) st256(even + off, a);
+  if (ok_o) st256(even + ld + off, b);
+}
 
-template <int BN, int EPI>
+// With PAIRS every lane of the warp calls (lane l holds row `row`, row - l a
+// multiple of 32), otherwise only lanes whose row exists.
+template <int BN, int EPI, bool PAIRS>
 __device__ __forceinline__ void epilogue32(const Args &a, const float (&v)[32], int row, bool valid, int c0,
                                            const float *bias) {
   const size_t o = (size_t)row * BN + c0;
+  if (EPI == CS_EPI_LINEAR_F32) {
+    float *d = a.outf + o;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      uint32_t w[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) w[j] = __float_as_uint(valid ? v[8 * i + j] + bias[c0 + 8 * i + j] : 0.0f);
+      st256(d + 8 * i, w);
+    }
+    return;
+  }
+  const bool odd = row & 1;
+  const int re = row & ~1;
+  const bool ok_e = re < a.rows, ok_o = re + 1 < a.rows;
+  const size_t oe = (size_t)re * BN + c0;
   if (EPI == CS_EPI_SILU) {
     float r[32];
-    if (a.resid) load_bf16x32(a.resid + o, r);
-    __align__(32) __nv_bfloat16 h[32], z[32];
+    if (a.resid) {
+      if constexpr (PAIRS)
+        load_bf16x32(a.resid + oe, BN, odd, ok_e, ok_o, r);
+      else
+        load_own32(a.resid + o, r);
+    }
+    __align__(32) __nv_bfloat16 h[32], z[PAIRS ? 32 : 1];
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
       float zz = v[i] + bias[c0 + i];
@@ -277,24 +338,19 @@ __device__ __forceinline__ void epilogue32(const Args &a, const float (&v)[32], 
         zz = 0.0f;
         hh = 0.0f;
       }
-      z[i] = __float2bfloat16(zz);
+      if constexpr (PAIRS) z[i] = __float2bfloat16(zz);
       h[i] = __float2bfloat16(hh);
     }
-    store_bf16x32(a.out + o, h);
-    if (a.out_pre) store_bf16x32(a.out_pre + o, z);
-  } else if (EPI == CS_EPI_LINEAR_F32) {
-    float *d = a.outf + o;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      uint32_t w[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) w[j] = __float_as_uint(valid ? v[8 * i + j] + bias[c0 + 8 * i + j] : 0.0f);
-      st256(d + 8 * i, w);
+    if constexpr (PAIRS) {
+      store_bf16x32(a.out + oe, BN, odd, ok_e, ok_o, h);
+      store_bf16x32(a.out_pre + oe, BN, odd, ok_e, ok_o, z);
+    } else {
+      store_own32(a.out + o, h);
     }
   } else {  // CS_EPI_BWD
     float r[32], zp[32];
-    if (a.resid) load_bf16x32(a.resid + o, r);
-    load_bf16x32(a.zprev + o, zp);
+    if (a.resid) load_bf16x32(a.resid + oe, BN, odd, ok_e, ok_o, r);
+    load_bf16x32(a.zprev + oe, BN, odd, ok_e, ok_o, zp);
     __align__(32) __nv_bfloat16 g[32], dz[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
@@ -308,8 +364,8 @@ __device__ __forceinline__ void epilogue32(const Args &a, const float (&v)[32], 
       g[i] = __float2bfloat16(gg);
       dz[i] = __float2bfloat16(d);
     }
-    store_bf16x32(a.out + o, dz);
-    if (a.gout) store_bf16x32(a.gout + o, g);
+    store_bf16x32(a.out + oe, BN, odd, ok_e, ok_o, dz);
+    if (a.gout) store_bf16x32(a.gout + oe, BN, odd, ok_e, ok_o, g);
   }
 }
 
@@ -327,7 +383,9 @@ constexpr int EPI_WARPS = 16;
 constexpr int WS_THREADS = 64 + 32 * EPI_WARPS;
 constexpr int WS_SMEM = 227 * 1024;
 
-template <int BN, int EPI, int TAPS>
+// PAIRS: the bf16 epilogue moves its arrays by lane pairs; for SiLU it then
+// also writes the pre-activation.
+template <int BN, int EPI, int TAPS, bool PAIRS>
 __global__ void __launch_bounds__(WS_THREADS, 1)
     conv_gemm_ws_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Args a,
                         int nst) {
@@ -466,7 +524,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
         const bool valid = in_range && (a.lp <= 0 || (pos >= 2 && pos < 2 + a.klev));
         float v[32];
         tcg::tmem_ld32(tmem + (uint32_t)(buf * BN) + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
-        if (in_range) epilogue32<BN, EPI>(a, v, row, valid, c0, sbias);
+        if (PAIRS || in_range) epilogue32<BN, EPI, PAIRS>(a, v, row, valid, c0, sbias);
       }
       tcg::tc_fence_before();
       __syncwarp();
@@ -770,7 +828,8 @@ constexpr int WG_RK = 64;                    // rows (K) per stage
 constexpr int WG_STAGES = 4;
 constexpr int WG_HALF = WG_RK * 128;         // one box of 64 features: 8 KB
 constexpr int WG_STAGE = 4 * WG_HALF;        // dZ (two halves) + X (two halves)
-constexpr int WG_SMEM = WG_STAGES * WG_STAGE + 1024 + 256;
+constexpr int WG_ONES = WG_STAGES * WG_STAGE;  // 64 rows x 64 ones (bf16), for the bias gradient
+constexpr int WG_SMEM = WG_ONES + WG_HALF + 1024 + 256;
 
 __device__ __forceinline__ uint64_t sdesc_mn_sw128(uint32_t saddr, uint32_t lbo) {
   return (uint64_t)((saddr >> 4) & 0x3FFFu)          // start address / 16
@@ -787,12 +846,13 @@ __device__ __forceinline__ void red_add_v4(float *p, float a, float b, float c, 
 template <int BN>
 __global__ void __launch_bounds__(128, 1)
     wgrad_tc_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmX, int rows,
-                    int chunk, int n, int taps, float *dw, unsigned *err) {
+                    int chunk, int n, int taps, float *dw, float *db, unsigned *err) {
   // transpose bits 15 and 16: both operands MN-major
   constexpr uint32_t IDESC = tcg::idesc_bf16_f32(128, BN) | (1u << 15) | (1u << 16);
+  constexpr uint32_t IDESC1 = tcg::idesc_bf16_f32(128, 16) | (1u << 15) | (1u << 16);
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t *bars = (uint64_t *)(smem + WG_STAGES * WG_STAGE);
+  uint64_t *bars = (uint64_t *)(smem + WG_ONES + WG_HALF);
   uint64_t *full = bars, *empty = bars + WG_STAGES, *tfull = empty + WG_STAGES, *drain = tfull + 1;
   uint32_t *tmem_slot = (uint32_t *)(drain + 1);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
@@ -805,6 +865,13 @@ __global__ void __launch_bounds__(128, 1)
   const int nkb = (r1 - r0 + WG_RK - 1) / WG_RK;
   const int nh = n / 64;
   constexpr int KH = BN / 64;
+  // the bias gradient, dZ's column sums: one more product with a matrix of
+  // ones (16 of its columns, the narrowest N), by the CTAs of the first tap
+  const bool bias = db != nullptr && t == 0;
+  if (bias) {
+    for (int i = tid; i < WG_HALF / 4; i += blockDim.x) reinterpret_cast<uint32_t *>(smem + WG_ONES)[i] = 0x3f803f80u;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
   // the dZ half TMA never writes (n = 64) stays zero: M is always 128
   if (nh == 1) {
     for (int i = tid; i < WG_STAGES * WG_HALF / 16; i += blockDim.x) {
@@ -828,7 +895,7 @@ __global__ void __launch_bounds__(128, 1)
     tcg::tma_prefetch_desc(&tmX);
   }
   if (warp == 1) {
-    tcg::tmem_alloc(tmem_slot, BN);
+    tcg::tmem_alloc(tmem_slot, 2 * BN);
     tcg::tmem_relinquish();
   }
   tcg::tc_fence_before();
@@ -862,11 +929,18 @@ __global__ void __launch_bounds__(128, 1)
       tcg::tc_fence_after();
       const uint32_t sa = tcg::smem_u32(smem + s * WG_STAGE);
       const uint64_t da = sdesc_mn_sw128(sa, WG_HALF);
-      const uint64_t db = sdesc_mn_sw128(sa + 2 * WG_HALF, WG_HALF);
+      const uint64_t dbx = sdesc_mn_sw128(sa + 2 * WG_HALF, WG_HALF);
 #pragma unroll
       for (int kk = 0; kk < WG_RK / 16; ++kk)  // 16 rows = two 1024-byte groups per instruction
-        tcg::mma_bf16(tmem, da + (uint64_t)(kk * (2048 >> 4)), db + (uint64_t)(kk * (2048 >> 4)), IDESC,
+        tcg::mma_bf16(tmem, da + (uint64_t)(kk * (2048 >> 4)), dbx + (uint64_t)(kk * (2048 >> 4)), IDESC,
                       (kb > 0 || kk > 0) ? 1u : 0u);
+      if (bias) {
+        const uint64_t d1 = sdesc_mn_sw128(tcg::smem_u32(smem + WG_ONES), WG_HALF);
+#pragma unroll
+        for (int kk = 0; kk < WG_RK / 16; ++kk)
+          tcg::mma_bf16(tmem + BN, da + (uint64_t)(kk * (2048 >> 4)), d1 + (uint64_t)(kk * (2048 >> 4)), IDESC1,
+                        (kb > 0 || kk > 0) ? 1u : 0u);
+      }
       tcg::mma_commit(&empty[s]);
       *consumed = (uint32_t)(kb + 1);
     }
@@ -894,6 +968,11 @@ __global__ void __launch_bounds__(128, 1)
 #pragma unroll
         for (int i = 0; i < 32; i += 4) red_add_v4(d + i, v[i], v[i + 1], v[i + 2], v[i + 3]);
       }
+      if (bias) {
+        float v[32];  // columns 0-15 hold the sums, all equal
+        tcg::tmem_ld32(tmem + ((uint32_t)m0 << 16) + (uint32_t)BN, v);
+        atomicAdd(db + m0 + lane, v[0]);
+      }
     }
   } else if (lane == 0) {
     flag(err, 2u);
@@ -912,7 +991,7 @@ __global__ void __launch_bounds__(128, 1)
   }
   tcg::tc_fence_before();
   __syncthreads();
-  if (warp == 1) tcg::tmem_dealloc(tmem, BN);
+  if (warp == 1) tcg::tmem_dealloc(tmem, 2 * BN);
 }
 
 // ------------------------------------------------------------------ host side
@@ -958,43 +1037,44 @@ cudaError_t launch_t(const CUtensorMap &ma, const CUtensorMap &mb, const Args &a
   return cudaGetLastError();
 }
 
-template <int BN, int EPI, int TAPS>
+template <int BN, int EPI, int TAPS, bool PAIRS>
 cudaError_t launch_ws_t(const CUtensorMap &ma, const CUtensorMap &mb, const Args &a, int grid, int nst,
                         cudaStream_t st) {
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(conv_gemm_ws_kernel<BN, EPI, TAPS>,
+    cudaError_t e = cudaFuncSetAttribute(conv_gemm_ws_kernel<BN, EPI, TAPS, PAIRS>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, WS_SMEM);
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  conv_gemm_ws_kernel<BN, EPI, TAPS><<<grid, WS_THREADS, WS_SMEM, st>>>(ma, mb, a, nst);
+  conv_gemm_ws_kernel<BN, EPI, TAPS, PAIRS><<<grid, WS_THREADS, WS_SMEM, st>>>(ma, mb, a, nst);
   return cudaGetLastError();
 }
 
 template <int BN>
 cudaError_t launch_ws_n(const CUtensorMap &ma, const CUtensorMap &mb, const Args &a, int grid, int nst,
                         cudaStream_t st) {
-  if (a.taps == 5) {
-    if (a.epi == CS_EPI_SILU) return launch_ws_t<BN, CS_EPI_SILU, 5>(ma, mb, a, grid, nst, st);
-    if (a.epi == CS_EPI_BWD) return launch_ws_t<BN, CS_EPI_BWD, 5>(ma, mb, a, grid, nst, st);
-    return launch_ws_t<BN, CS_EPI_LINEAR_F32, 5>(ma, mb, a, grid, nst, st);
-  }
-  if (a.epi == CS_EPI_SILU) return launch_ws_t<BN, CS_EPI_SILU, 1>(ma, mb, a, grid, nst, st);
-  if (a.epi == CS_EPI_BWD) return launch_ws_t<BN, CS_EPI_BWD, 1>(ma, mb, a, grid, nst, st);
-  return launch_ws_t<BN, CS_EPI_LINEAR_F32, 1>(ma, mb, a, grid, nst, st);
+  auto taps = [&](auto t) -> cudaError_t {
+    constexpr int T = decltype(t)::value;
+    if (a.epi == CS_EPI_SILU)
+      return a.out_pre ? launch_ws_t<BN, CS_EPI_SILU, T, true>(ma, mb, a, grid, nst, st)
+                       : launch_ws_t<BN, CS_EPI_SILU, T, false>(ma, mb, a, grid, nst, st);
+    if (a.epi == CS_EPI_BWD) return launch_ws_t<BN, CS_EPI_BWD, T, true>(ma, mb, a, grid, nst, st);
+    return launch_ws_t<BN, CS_EPI_LINEAR_F32, T, false>(ma, mb, a, grid, nst, st);
+  };
+  return a.taps == 5 ? taps(std::integral_constant<int, 5>()) : taps(std::integral_constant<int, 1>());
 }
 
 template <int BN>
 cudaError_t launch_wgrad_t(const CUtensorMap &md, const CUtensorMap &mx, int rows, int chunk, int nchunks, int n,
-                           int taps, float *dw, unsigned *err, cudaStream_t st) {
+                           int taps, float *dw, float *db, unsigned *err, cudaStream_t st) {
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(wgrad_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM);
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  wgrad_tc_kernel<BN><<<dim3(nchunks, taps), 128, WG_SMEM, st>>>(md, mx, rows, chunk, n, taps, dw, err);
+  wgrad_tc_kernel<BN><<<dim3(nchunks, taps), 128, WG_SMEM, st>>>(md, mx, rows, chunk, n, taps, dw, db, err);
   return cudaGetLastError();
 }
 
@@ -1094,8 +1174,9 @@ extern "C" int cs_conv_gemm(const cs_gemm_desc *g, void *stream) {
 
 // dW[t][n][k] += sum over rows of dZ[r][n] X[r + t - taps/2][k] on the tensor
 // cores (wgrad_tc_kernel): dZ [rows][n], X [rows][k] bf16 row-major, dW f32.
-extern "C" int cs_wgrad_tc(const void *dz, const void *x, int32_t rows, int32_t n, int32_t k, int32_t taps,
-                           float *dw, unsigned *err, void *stream) {
+// With db, the column sums of dZ are added to it (the bias gradient).
+int wgrad_tc(const void *dz, const void *x, int32_t rows, int32_t n, int32_t k, int32_t taps, float *dw, float *db,
+             unsigned *err, void *stream) {
   using namespace sg;
   if (!dz || !x || !dw || rows <= 0 || (n != 64 && n != 128) || (k != 64 && k != 128) || (taps != 1 && taps != 5))
     return CS_E_ARG;
@@ -1106,9 +1187,10 @@ extern "C" int cs_wgrad_tc(const void *dz, const void *x, int32_t rows, int32_t 
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // about two CTAs per SM over all taps, chunks of at least 512 rows (each
-  // chunk adds its n x k partial to dW)
-  int nchunks = (2 * sms + taps - 1) / taps;
+  // one CTA per SM (its ring and the ones fill the shared memory) over all
+  // taps, in one wave; chunks of at least 512 rows (each chunk adds its n x k
+  // partial to dW)
+  int nchunks = sms / taps;
   const int maxchunks = (rows + 511) / 512;
   if (nchunks > maxchunks) nchunks = maxchunks;
   if (nchunks < 1) nchunks = 1;
@@ -1116,9 +1198,13 @@ extern "C" int cs_wgrad_tc(const void *dz, const void *x, int32_t rows, int32_t 
   chunk = (chunk + WG_RK - 1) / WG_RK * WG_RK;
   nchunks = (rows + chunk - 1) / chunk;
   cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t e = k == 128 ? launch_wgrad_t<128>(md, mx, rows, chunk, nchunks, n, taps, dw, err, st)
-                           : launch_wgrad_t<64>(md, mx, rows, chunk, nchunks, n, taps, dw, err, st);
+  cudaError_t e = k == 128 ? launch_wgrad_t<128>(md, mx, rows, chunk, nchunks, n, taps, dw, db, err, st)
+                           : launch_wgrad_t<64>(md, mx, rows, chunk, nchunks, n, taps, dw, db, err, st);
   return e == cudaSuccess ? CS_OK : CS_E_CUDA;
+}
+extern "C" int cs_wgrad_tc(const void *dz, const void *x, int32_t rows, int32_t n, int32_t k, int32_t taps,
+                           float *dw, unsigned *err, void *stream) {
+  return wgrad_tc(dz, x, rows, n, k, taps, dw, nullptr, err, stream);
 }
 
 // The network's MLP layer and output head in one kernel (inference):

@@ -329,38 +329,28 @@ __global__ void loss_kernel(const float *__restrict__ y, const float *__restrict
   if (threadIdx.x == 0) atomicAdd(loss_sum, red[0]);
 }
 
-// ---------------------------------------------------------------- gradients
-// The weight gradients run on the tensor cores (cs_wgrad_tc, surrogate_gemm.cu);
-// the bias gradient is a column sum of dz over chunks of rows.
-constexpr int BG_CHUNK = 128;
-__global__ void bgrad_kernel(const __nv_bfloat16 *__restrict__ dz, int rows, int n, float *db) {
-  const int r0 = blockIdx.x * BG_CHUNK, r1 = min(rows, r0 + BG_CHUNK);
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // four independent sums: the loads overlap
-    int r = r0;
-    for (; r + 4 <= r1; r += 4) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) s[q] += __bfloat162float(dz[(size_t)(r + q) * n + j]);
-    }
-    for (; r < r1; ++r) s[0] += __bfloat162float(dz[(size_t)r * n + j]);
-    atomicAdd(&db[j], (s[0] + s[1]) + (s[2] + s[3]));
-  }
-}
-
 // ---------------------------------------------------------------- AdamW
-__global__ void adamw_kernel(float *p, float *g, float *m, float *v, int taps, int n, int k, cs_adam hp,
-                             __nv_bfloat16 *w, __nv_bfloat16 *wt) {
+// One launch for several tensors (blockIdx.y): a training step updates ten,
+// and a launch each took longer than the updates.
+struct AdamTensors {
+  cs_adam_tensor t[CS_ADAM_MAX];
+};
+__global__ void adamw_kernel(AdamTensors A, cs_adam hp) {
+  const cs_adam_tensor &T = A.t[blockIdx.y];
+  const int taps = T.taps, n = T.n, k = T.k;
+  __nv_bfloat16 *w = (__nv_bfloat16 *)T.w, *wt = (__nv_bfloat16 *)T.wt;
+  const float wd = T.weight_decay;
   const long long cnt = (long long)taps * n * k;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < cnt; i += (long long)gridDim.x * blockDim.x) {
-    const float gi = g[i];
-    const float mi = hp.beta1 * m[i] + (1.0f - hp.beta1) * gi;
-    const float vi = hp.beta2 * v[i] + (1.0f - hp.beta2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    g[i] = 0.0f;
-    float pi = p[i];
-    pi -= hp.lr * ((mi / hp.bc1) / (sqrtf(vi / hp.bc2) + hp.eps) + hp.weight_decay * pi);
-    p[i] = pi;
+    const float gi = T.g[i];
+    const float mi = hp.beta1 * T.m[i] + (1.0f - hp.beta1) * gi;
+    const float vi = hp.beta2 * T.v[i] + (1.0f - hp.beta2) * gi * gi;
+    T.m[i] = mi;
+    T.v[i] = vi;
+    T.g[i] = 0.0f;
+    float pi = T.p[i];
+    pi -= hp.lr * ((mi / hp.bc1) / (sqrtf(vi / hp.bc2) + hp.eps) + wd * pi);
+    T.p[i] = pi;
     if (w) w[i] = __float2bfloat16(pi);
     if (wt) {
       const int t = (int)(i / ((long long)n * k));
@@ -590,6 +580,10 @@ bool cols_ok(const cs_columns *c) {
 
 }  // namespace sk
 
+// The weight (and bias) gradient on the tensor cores (surrogate_gemm.cu).
+int wgrad_tc(const void *dz, const void *x, int32_t rows, int32_t n, int32_t k, int32_t taps, float *dw, float *db,
+             unsigned *err, void *stream);
+
 extern "C" {
 
 int cs_raw_features(const cs_columns *c, float *feat, void *stream) {
@@ -664,21 +658,30 @@ int cs_wgrad(const void *dz, const void *x, int32_t rows, int32_t n, int32_t k, 
   using namespace sk;
   if (!dz || !x || !dw || rows <= 0 || (n != 64 && n != 128) || (k != 64 && k != 128) || (taps != 1 && taps != 5))
     return CS_E_ARG;
-  const int rc = cs_wgrad_tc(dz, x, rows, n, k, taps, dw, nullptr, stream);
-  if (rc != CS_OK) return rc;
-  if (db) bgrad_kernel<<<(rows + BG_CHUNK - 1) / BG_CHUNK, 128, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16 *)dz, rows, n, db);
+  return wgrad_tc(dz, x, rows, n, k, taps, dw, db, nullptr, stream);
+}
+
+int cs_adamw_tensors(const cs_adam_tensor *t, int32_t count, const cs_adam *hp, void *stream) {
+  using namespace sk;
+  if (!t || !hp || count <= 0 || count > CS_ADAM_MAX) return CS_E_ARG;
+  AdamTensors A;
+  memset(&A, 0, sizeof(A));
+  long long most = 0;
+  for (int i = 0; i < count; ++i) {
+    if (!t[i].p || !t[i].g || !t[i].m || !t[i].v || t[i].taps <= 0 || t[i].n <= 0 || t[i].k <= 0) return CS_E_ARG;
+    A.t[i] = t[i];
+    const long long cnt = (long long)t[i].taps * t[i].n * t[i].k;
+    most = cnt > most ? cnt : most;
+  }
+  adamw_kernel<<<dim3(grid_1d(most, 256), count), 256, 0, (cudaStream_t)stream>>>(A, *hp);
   return cudaGetLastError() == cudaSuccess ? CS_OK : CS_E_CUDA;
 }
 
 int cs_adamw(float *p, float *g, float *m, float *v, int32_t taps, int32_t n, int32_t k, const cs_adam *hp, void *w,
              void *wt, void *stream) {
-  using namespace sk;
-  if (!p || !g || !m || !v || !hp || taps <= 0 || n <= 0 || k <= 0) return CS_E_ARG;
-  const long long cnt = (long long)taps * n * k;
-  adamw_kernel<<<grid_1d(cnt, 256), 256, 0, (cudaStream_t)stream>>>(p, g, m, v, taps, n, k, *hp,
-                                                                     (__nv_bfloat16 *)w, (__nv_bfloat16 *)wt);
-  return cudaGetLastError() == cudaSuccess ? CS_OK : CS_E_CUDA;
+  if (!hp) return CS_E_ARG;
+  const cs_adam_tensor t = {p, g, m, v, w, wt, taps, n, k, hp->weight_decay};
+  return cs_adamw_tensors(&t, 1, hp, stream);
 }
 
 int cs_post(const cs_columns *c, const float *y, int32_t nheads, const cs_guard *g, int32_t *nflagged,

@@ -76,6 +76,11 @@ class Adam(ctypes.Structure):
     _fields_ = [(n, ctypes.c_float) for n in ["lr", "beta1", "beta2", "eps", "weight_decay", "bc1", "bc2"]]
 
 
+class AdamTensor(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p) for n in ["p", "g", "m", "v", "w", "wt"]] + \
+               [(n, ctypes.c_int32) for n in ["taps", "n", "k"]] + [("weight_decay", ctypes.c_float)]
+
+
 class Guard(ctypes.Structure):
     _fields_ = [("out_scale", ctypes.c_float * 16), ("rg", ctypes.c_double), ("ralvdcp", ctypes.c_double),
                 ("ralsdcp", ctypes.c_double), ("rlvtt", ctypes.c_double), ("rlstt", ctypes.c_double),
@@ -106,10 +111,11 @@ def _lib():
         L.cs_wgrad.argtypes = [vp, vp, i32, i32, i32, i32, vp, vp, vp]
         L.cs_wgrad_tc.argtypes = [vp, vp, i32, i32, i32, i32, vp, vp, vp]
         L.cs_adamw.argtypes = [vp, vp, vp, vp, i32, i32, i32, ctypes.POINTER(Adam), vp, vp, vp]
+        L.cs_adamw_tensors.argtypes = [ctypes.POINTER(AdamTensor), i32, ctypes.POINTER(Adam), vp]
         L.cs_post.argtypes = [ctypes.POINTER(Columns), vp, i32, ctypes.POINTER(Guard), vp, vp, vp, vp]
         L.cs_move_columns.argtypes = [vp, i32, i32, i32, vp, vp, i32, i32, vp]
         for f in ["cs_raw_features", "cs_column_sums", "cs_prep_inputs", "cs_prep_targets", "cs_prep_batch", "cs_loss",
-                  "cs_wgrad", "cs_wgrad_tc", "cs_adamw", "cs_post", "cs_move_columns"]:
+                  "cs_wgrad", "cs_wgrad_tc", "cs_adamw", "cs_adamw_tensors", "cs_post", "cs_move_columns"]:
             getattr(L, f).restype = ctypes.c_int
         _L = L
     return _L
@@ -247,12 +253,12 @@ class Net:
         self.step_count += 1
         t = self.step_count
         hp = Adam(lr, beta1, beta2, eps, wd, 1 - beta1 ** t, 1 - beta2 ** t)
-        hpb = Adam(lr, beta1, beta2, eps, 0.0, 1 - beta1 ** t, 1 - beta2 ** t)
+        ts = []
         for i, (tp, n, k) in self.shapes.items():
-            _ok(L.cs_adamw(_p(self.p[i]), _p(self.g[i]), _p(self.m[i]), _p(self.v[i]), tp, n, k,
-                           ctypes.byref(hp), _p(self.wbf[i]), _p(self.wtbf[i]), s), "cs_adamw")
-            _ok(L.cs_adamw(_p(self.b[i]), _p(self.gb[i]), _p(self.mb[i]), _p(self.vb[i]), 1, n, 1,
-                           ctypes.byref(hpb), None, None, s), "cs_adamw")
+            ts.append(AdamTensor(_p(self.p[i]), _p(self.g[i]), _p(self.m[i]), _p(self.v[i]), _p(self.wbf[i]),
+                                 _p(self.wtbf[i]), tp, n, k, wd))
+            ts.append(AdamTensor(_p(self.b[i]), _p(self.gb[i]), _p(self.mb[i]), _p(self.vb[i]), None, None, 1, n, 1, 0.0))
+        _ok(L.cs_adamw_tensors((AdamTensor * len(ts))(*ts), len(ts), ctypes.byref(hp), s), "cs_adamw_tensors")
 
     # -- persistence
     def state(self):
