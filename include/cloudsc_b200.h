@@ -231,7 +231,8 @@ int cloudsc_b200_batched(
 /*
  * Batched call with HOST pointers (same arrays and order as
  * cloudsc_b200_batched): blocks are processed in chunks of chunk_blocks
- * (<= 0 selects 64), each chunk's host-to-device copy, kernel and
+ * (<= 0: as many as give the least estimated time, at most 8,192 columns a
+ * chunk), each chunk's host-to-device copy, kernel and
  * device-to-host copy pipelined on three streams over three device buffers,
  * so transfers overlap compute.  Host arrays should be page-locked for the
  * copies to run asynchronously.  Synchronous: returns when all outputs are

@@ -31,7 +31,7 @@
 // Every division of the column code: the branch-free division when FAST_ (the
 // fast pass; with CHK_ recording its operands in divbad_), IEEE division
 // otherwise (cdiv, cloudsc_column.cuh).
-#define DIV(...) cdiv<FAST_, CHK_>(__VA_ARGS__, divbad_)
+#define DIV(...) cdiv<FAST_, CHK_, SHORT_>(__VA_ARGS__, divbad_)
 // A literal divisor: its reciprocal folded at compile time (cdivk).
 #define DIVK(A, B) cdivk<FAST_, CHK_>(A, B, 1.0 / (B), divbad_)
 // A power-of-two literal divisor: multiplication by its exact reciprocal,
@@ -115,6 +115,7 @@ CSC_DEV void scale_entries(int jo, QA &q, double zr) {
 }
 template <bool FAST_, bool CHK_>
 CSC_DEV void scale_row(int jo, QA &q, const double qx[5], DivCheck &divbad_) {
+  constexpr bool SHORT_ = true;
   const double zepsec = 1.E-14;
   const double ss = sink_sum(jo, q);
   const double zmm = mx(qx[jo], zepsec);
@@ -134,6 +135,7 @@ CSC_DEV void scale_row(int jo, QA &q, const double qx[5], DivCheck &divbad_) {
 // the same factors in the same order as with the full sort.
 template <bool CHK_>
 CSC_DEV void truncate_sinks(QA &q, const double qx[5], DivCheck &divbad_) {
+  constexpr bool SHORT_ = true;
   constexpr bool FAST_ = true;
   const double zepsec = 1.E-14;
   double z[5], ss[5];
@@ -193,6 +195,7 @@ CSC_DEV void truncate_sinks(QA &q, const double qx[5], DivCheck &divbad_) {
 // ZRATIO for every species from the current ZSOLQA (cloudsc.F90:3455-3474).
 template <bool FAST_, bool CHK_>
 CSC_DEV void sink_ratios(const QA &q, const double qx[5], double r[5], DivCheck &divbad_) {
+  constexpr bool SHORT_ = true;
   const double zepsec = 1.E-14;
 #pragma unroll
   for (int jm = 0; jm < 5; ++jm) {
@@ -207,6 +210,7 @@ CSC_DEV void sink_ratios(const QA &q, const double qx[5], double r[5], DivCheck 
 template <bool FAST_, bool CHK_>
 CSC_DEV void supersatcheck(double pt, double pq, double pa, double pp, double &t_adj, double &q_adj,
                            double &a_adj, double &l_adj, double &i_adj, DivCheck &divbad_) {
+  constexpr bool SHORT_ = true;
   const KParamsD &k = c_kd;
   const double zepsec = 1.E-14;
   double zda = 0.0;
@@ -520,6 +524,7 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
   // PARK < 0: the build with registers to spare, where the processes of a
   // group form one block; otherwise each sits behind its own vote
   constexpr bool WIDE = PARK < 0;
+  constexpr bool SHORT_ = WIDE || F32M || OPT;  // fast_quot_rcp
   DivCheck divbad_;
   const auto root = [&](Real x) -> Real {
     if constexpr (std::is_same<Real, double>::value) return csqrt<FAST_>(x, divbad_);
