@@ -125,6 +125,15 @@ CSC_DEV void scale_row(int jo, QA &q, const double qx[5], DivCheck &divbad_) {
 #undef SCL1
 #undef SCL2
 
+// The position of the lowest set bit of a nonzero x.
+CSC_DEV int lowest_bit(unsigned x) {
+#if defined(__CUDA_ARCH__)
+  return __ffs((int)x) - 1;
+#else
+  return __builtin_ctz(x);
+#endif
+}
+
 // The sink truncation of one column (cloudsc.F90:3455-3536): the rows rescaled
 // in the order of their ratios ZMM/MAX(ZSINKSUM,ZMM), ties in species order.
 // Only a row whose sinks exceed its amount has a ratio below 1; the other
@@ -172,12 +181,18 @@ CSC_DEV void truncate_sinks(QA &q, const double qx[5], DivCheck &divbad_) {
       for (int jm = 1; jm < 5; ++jm) order = (over >> jm) & 1u ? (unsigned)jm : order;
     }
   }
+  // Every trip takes one row of `left`, whatever the bits of `order`: a NaN
+  // ratio (an infinite amount or sink sum, in a column the checks have reported
+  // and whose rerun decides the outputs) leaves `order` without being a
+  // permutation, and the row it names is then replaced by the lowest one left.
+  // So at most five trips, and each row at most once.
   unsigned left = over;
 #pragma unroll 1
-  while (CSC_ANY(left != 0u)) {
+  for (int trip = 0; trip < 5 && CSC_ANY(left != 0u); ++trip) {
     if (left != 0u) {
-      const int jo = (int)(order & 7u);
+      int jo = (int)(order & 7u);
       order >>= 3;
+      if (!((left >> jo) & 1u)) jo = lowest_bit(left);
       left &= ~(1u << jo);
       scale_row<FAST_, CHK_>(jo, q, qx, divbad_);
     }

@@ -81,6 +81,7 @@ struct DivCheck {
 #if defined(__CUDA_ARCH__)
 CSC_DEV unsigned hi_word(double x) { return (unsigned)__double2hiint(x); }
 CSC_DEV unsigned lo_word(double x) { return (unsigned)__double2loint(x); }
+CSC_DEV double from_words(unsigned hi, unsigned lo) { return __hiloint2double((int)hi, (int)lo); }
 #else
 inline unsigned hi_word(double x) {
   uint64_t u;
@@ -92,6 +93,45 @@ inline unsigned lo_word(double x) {
   std::memcpy(&u, &x, sizeof u);
   return (unsigned)u;
 }
+inline double from_words(unsigned hi, unsigned lo) {
+  const uint64_t u = (uint64_t)hi << 32 | lo;
+  double x;
+  std::memcpy(&x, &u, sizeof x);
+  return x;
+}
+#endif
+
+// The branch-free sequences below run on the GPU, and in host builds that ask
+// for them (CLOUDSC_HOST_SEQUENCES); other host builds divide and take roots
+// with IEEE operations.  Their estimates are rcp.approx.ftz.f64 and
+// rsqrt.approx.ftz.f64 on the GPU; on the host the values 1/x and 1/sqrt(x)
+// cut to 20 fraction bits, subnormals read and returned as zero.
+#if defined(__CUDA_ARCH__)
+#define CSC_SEQUENCES 1
+CSC_DEV double rcp_estimate(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+CSC_DEV double rsqrt_estimate(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+CSC_DEV double fmad(double a, double b, double c) { return __fma_rn(a, b, c); }
+CSC_DEV double muld(double a, double b) { return __dmul_rn(a, b); }
+#elif defined(CLOUDSC_HOST_SEQUENCES)
+#define CSC_SEQUENCES 1
+inline double no_subnormal(double x) { return std::fabs(x) < 0x1p-1022 ? std::copysign(0.0, x) : x; }
+inline double estimate_of(double y) {
+  return no_subnormal(std::isfinite(y) ? from_words(hi_word(y), 0u) : y);
+}
+inline double rcp_estimate(double x) { return estimate_of(1.0 / no_subnormal(x)); }
+inline double rsqrt_estimate(double x) { return estimate_of(1.0 / std::sqrt(no_subnormal(x))); }
+inline double fmad(double a, double b, double c) { return std::fma(a, b, c); }
+inline double muld(double a, double b) { return a * b; }
+#else
+#define CSC_SEQUENCES 0
 #endif
 // Record a value that must be zero or inside 2^-256 <= |x| < 2^256.
 CSC_DEV void see(double x, DivCheck &dc) { dc.acc |= x == 0.0 ? 0u : hi_word(x) * 2u - kDivBase; }
@@ -108,15 +148,14 @@ CSC_DEV void see_pos(double x, int e, DivCheck &dc) { dc.pos |= hi_word(x) - ((u
 // Floating-Point Arithmetic, ch. 5).  For b = (2 - 2^-52) 2^E the step ends on
 // the tie 2^(-E-1) while 1/b = 2^(-E-1) (1 + 2^-53 + 2^-106 + ...).
 CSC_DEV double fast_rcp_y(double b) {
-#if defined(__CUDA_ARCH__)
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  double e = __fma_rn(-b, y, 1.0);
-  y = __fma_rn(y, e, y);
-  e = __fma_rn(-b, y, 1.0);
-  y = __fma_rn(y, e, y);
-  e = __fma_rn(-b, y, 1.0);
-  return __fma_rn(y, e, y);
+#if CSC_SEQUENCES
+  double y = rcp_estimate(b);
+  double e = fmad(-b, y, 1.0);
+  y = fmad(y, e, y);
+  e = fmad(-b, y, 1.0);
+  y = fmad(y, e, y);
+  e = fmad(-b, y, 1.0);
+  return fmad(y, e, y);
 #else
   return 1.0 / b;
 #endif
@@ -128,12 +167,12 @@ CSC_DEV double fast_rcp_y(double b) {
 // (up to the sign of a zero) when no step under- or overflows, for instance
 // for 2^-256 <= |b| < 2^256 and a = 0 or 2^-256 <= |a| < 2^256.
 CSC_DEV double fast_quot(double a, double b, double y) {
-#if defined(__CUDA_ARCH__)
-  const double q0 = __dmul_rn(a, y);
-  double r = __fma_rn(-b, q0, a);
-  const double q1 = __fma_rn(r, y, q0);
-  r = __fma_rn(-b, q1, a);
-  return __fma_rn(r, y, q1);
+#if CSC_SEQUENCES
+  const double q0 = muld(a, y);
+  double r = fmad(-b, q0, a);
+  const double q1 = fmad(r, y, q0);
+  r = fmad(-b, q1, a);
+  return fmad(r, y, q1);
 #else
   (void)y;
   return a / b;
@@ -150,20 +189,19 @@ CSC_DEV double fast_quot(double a, double b, double y) {
 // 0.881; FP64 at 128 and 168 registers no gain (262,144 columns 9.494 / 9.472),
 // so the level code there keeps the other order (SHORT).
 CSC_DEV double fast_quot_rcp(double a, double b) {
-#if defined(__CUDA_ARCH__)
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  double e = __fma_rn(-b, y, 1.0);
-  y = __fma_rn(y, e, y);
-  e = __fma_rn(-b, y, 1.0);
-  y = __fma_rn(y, e, y);
-  const double q0 = __dmul_rn(a, y);
-  e = __fma_rn(-b, y, 1.0);
-  double r = __fma_rn(-b, q0, a);
-  y = __fma_rn(y, e, y);
-  const double q1 = __fma_rn(r, y, q0);
-  r = __fma_rn(-b, q1, a);
-  return __fma_rn(r, y, q1);
+#if CSC_SEQUENCES
+  double y = rcp_estimate(b);
+  double e = fmad(-b, y, 1.0);
+  y = fmad(y, e, y);
+  e = fmad(-b, y, 1.0);
+  y = fmad(y, e, y);
+  const double q0 = muld(a, y);
+  e = fmad(-b, y, 1.0);
+  double r = fmad(-b, q0, a);
+  y = fmad(y, e, y);
+  const double q1 = fmad(r, y, q0);
+  r = fmad(-b, q1, a);
+  return fmad(r, y, q1);
 #else
   return a / b;
 #endif
@@ -183,20 +221,19 @@ CSC_DEV unsigned ones_word(double b) { return (hi_word(b) | 0xfff00000u) & lo_wo
 // Both are reported to the rerun.
 template <bool FAST>
 CSC_DEV double csqrt(double x, DivCheck &dc) {
-#if defined(__CUDA_ARCH__)
+#if CSC_SEQUENCES
   if constexpr (FAST) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    double g = __dmul_rn(x, y), h = __dmul_rn(0.5, y);
-    double r = __fma_rn(-g, h, 0.5);
-    g = __fma_rn(g, r, g);
-    h = __fma_rn(h, r, h);
-    r = __fma_rn(-g, h, 0.5);
-    g = __fma_rn(g, r, g);
-    h = __fma_rn(h, r, h);
-    g = __fma_rn(__fma_rn(-g, g, x), h, g);
-    const double d = __fma_rn(-g, g, x);
-    const double gu = __dmul_rn(g, __hiloint2double((__double2hiint(g) & 0x7ff00000) - (52 << 20), 0));
+    const double y = rsqrt_estimate(x);
+    double g = muld(x, y), h = muld(0.5, y);
+    double r = fmad(-g, h, 0.5);
+    g = fmad(g, r, g);
+    h = fmad(h, r, h);
+    r = fmad(-g, h, 0.5);
+    g = fmad(g, r, g);
+    h = fmad(h, r, h);
+    g = fmad(fmad(-g, g, x), h, g);
+    const double d = fmad(-g, g, x);
+    const double gu = muld(g, from_words((hi_word(g) & 0x7ff00000u) - (52u << 20), 0u));
     dc.pos |= fabs(d) < gu ? 0u : kPosRange;
     const unsigned o = ones_word(x);
     dc.ones = dc.ones > o ? dc.ones : o;

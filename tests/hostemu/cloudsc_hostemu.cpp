@@ -3,7 +3,7 @@
 // The GPU kernels' per-column code (openifs_b200/csrc/cloudsc_body.cuh),
 // compiled unchanged for the host with no FMA contraction.  Double precision
 // uses plibm.h's exp/pow, exactly as on the GPU; compiled with
-// -DHOSTEMU_GLIBC the double-precision exp/pow are glibc's instead.  The tests
+// -DCLOUDSC_HOST_LIBM_GLIBC the double-precision exp/pow are glibc's instead.  The tests
 // compare it with the oracle built against the same libm: a bit-for-bit match
 // proves that the kernel's logic (its fused single pass, sparse 5x5 matrices,
 // operation order) restates the reference exactly.
@@ -12,6 +12,19 @@
 #include <cstring>
 
 #define CSC_DEV inline
+// The "lanes" builds stand for a column whose warp neighbours need every
+// process: each vote is won, whatever the column itself needs, and the fast
+// pass runs the GPU's own division and root sequences.
+#if defined(CLOUDSC_HOST_LANES)
+#define CLOUDSC_HOST_SEQUENCES
+#define CLOUDSC_HOST_WINDOW_CHECK
+#define CSC_ANY(C) ((void)(C), true)
+#endif
+// Parked values and process groups of the fast pass as in the kernels' narrow
+// (0) or 256-thread (-1) builds.
+#if !defined(CLOUDSC_HOST_PARK)
+#define CLOUDSC_HOST_PARK 0
+#endif
 #include "../../openifs_b200/csrc/cloudsc_column.cuh"
 #include "../../openifs_b200/csrc/cloudsc_kparams.h"
 
@@ -47,7 +60,7 @@ static void column(const Fields &f, const Shape &sh, int ib, int jl) {
   if (FD && sh.klev <= kMaxLevFast) {
     double plude_in[kMaxLevFast];
     bool bad = false;
-    cloudsc_column<Real, F32M, false, false, Fields, GEN, kPassFast>(f, sh, ib, jl, true, &bad, plude_in);
+    cloudsc_column<Real, F32M, false, false, Fields, GEN, kPassFast, CLOUDSC_HOST_PARK>(f, sh, ib, jl, true, &bad, plude_in);
     if (bad) cloudsc_column<Real, F32M, false, false, Fields, GEN, kPassRedo>(f, sh, ib, jl, true, nullptr, plude_in);
   } else {
     cloudsc_column<Real, F32M, false, false, Fields, GEN>(f, sh, ib, jl);
@@ -201,7 +214,8 @@ static void column_opt(const Fields &f, const Shape &sh, int ib, int jl) {
     double plude_in[kMaxLevFast];
     bool bad = false;
     int kbud = sh.klev;
-    cloudsc_column<double, false, BUD, OPT, Fields, GEN, kPassFast>(f, sh, ib, jl, true, &bad, plude_in, &kbud);
+    cloudsc_column<double, false, BUD, OPT, Fields, GEN, kPassFast, CLOUDSC_HOST_PARK>(f, sh, ib, jl, true, &bad,
+                                                                                      plude_in, &kbud);
     if (bad)
       cloudsc_column<double, false, BUD, OPT, Fields, GEN, kPassRedo>(f, sh, ib, jl, true, nullptr, plude_in,
                                                                       &kbud);

@@ -1,0 +1,106 @@
+"""The column kernels on inputs no column should have -- tiny, huge, infinite and
+NaN values scattered over the fields: the fast pass ends and reports those
+columns, their rerun gives the plain column code's bits (host build), and the
+other columns of the warp are untouched by them (GPU tests)."""
+import numpy as np
+import pytest
+
+from openifs_b200 import cloudsc, fields, inputs
+from tests import util
+from tests.test_fast_pass_votes import NBLK, NGPTOT, NPROMA, _inputs
+
+pytestmark = pytest.mark.gpu
+
+# by size (the 256-thread build at this size), and the narrow builds
+SCHEDULES = [None, (1, 448, 0), (2, 384, 0)]
+
+
+def _same(got, ref):
+    for n in util.COMPARED:
+        a, b = (util.defined(n, util._valid_cols(x[n], NGPTOT, NPROMA)) for x in (got, ref))
+        assert np.array_equal(a, b, equal_nan=True), n
+
+
+def _with_schedule(sched, run, precision=cloudsc.FP64):
+    before = cloudsc.get_schedule(precision)
+    if sched is None:
+        return run()
+    try:
+        cloudsc.set_schedule(precision, *sched)
+        return run()
+    finally:
+        cloudsc.set_schedule(precision, *before)
+
+
+@pytest.mark.parametrize("sched", SCHEDULES)
+@pytest.mark.parametrize("case", ["hostile", "non_finite"])
+def test_fp64(cuda, case, sched):
+    p, _ = util.params()
+    arrs = _inputs(case, p, 81)
+    ref, nw = util.run_hostemu(p, arrs, NPROMA, NBLK, NGPTOT, precision=0x100)
+    gpu, nwg = _with_schedule(sched, lambda: util.run_gpu(p, arrs, NPROMA, NBLK, NGPTOT))
+    _same(gpu, ref)
+    assert nwg == nw
+
+
+@pytest.mark.parametrize("precision", [cloudsc.MIXED, cloudsc.PHYS32])
+def test_other_columns_untouched(cuda, precision):
+    """The FP32 forms (their powf and expf are the GPU's): the columns without a
+    foreign value equal those of a run without any."""
+    p, _ = util.params()
+    clean = _inputs("plain", p, 81)
+    arrs = _inputs("non_finite", p, 81)
+    foreign = np.zeros((NBLK, NPROMA), bool)
+    for n in clean:
+        if clean[n].ndim >= 3:
+            d = ~((arrs[n] == clean[n]) | (np.isnan(arrs[n]) & np.isnan(clean[n])))
+            foreign |= d.reshape(NBLK, -1, NPROMA).any(axis=1)
+    assert 0 < foreign.sum() < foreign.size // 2
+    a, _ = util.run_gpu(p, arrs, NPROMA, NBLK, NGPTOT, precision=precision)
+    b, _ = util.run_gpu(p, clean, NPROMA, NBLK, NGPTOT, precision=precision)
+    for n in util.COMPARED:
+        x, y = (util.defined(n, util._valid_cols(v[n], NGPTOT, NPROMA)).reshape(NBLK, -1, NPROMA) for v in (a, b))
+        keep = ~foreign[:, None, :] & np.ones(x.shape, bool)
+        assert np.array_equal(x[keep], y[keep]), n
+
+
+@pytest.mark.parametrize("case", ["hostile", "non_finite"])
+def test_single_precision_interface(cuda, case):
+    import torch
+    p, _ = util.params()
+    with np.errstate(over="ignore"):
+        sp = fields.to_single(_inputs(case, p, 81))
+    wide = {k: (v.astype(np.float64) if v.dtype == np.float32 else v.copy()) for k, v in sp.items()}
+    ref, nw = util.run_hostemu(p, wide, NPROMA, NBLK, NGPTOT, precision=0x100)
+    cloudsc.setup(p)
+    d = {k: torch.from_numpy(v).cuda() for k, v in sp.items()}
+    cnt = torch.zeros(1, dtype=torch.int32, device="cuda")
+    cloudsc.cloudsc_batched_sp(p, d, NPROMA, util.KLEV, NBLK, NGPTOT, util.PTSPHY, counter=cnt)
+    torch.cuda.synchronize()
+    with np.errstate(over="ignore"):
+        _same({n: d[n].cpu().numpy() for n in util.COMPARED}, {n: ref[n].astype(np.float32) for n in util.COMPARED})
+    assert int(cnt.item()) == nw
+
+
+@pytest.mark.parametrize("opt", ["budgets", "spp", "all+budgets"])
+def test_optional_forms(cuda, opt):
+    import torch
+    p0, _ = util.params()
+    p = util.with_flags(p0, util.BUDGET_CASES[-1]) if opt == "budgets" else util.opt_params(p0, opt)
+    arrs = _inputs("non_finite", p, 83)
+    diag = inputs.generate_diag(arrs, NPROMA, fields.budget_fields_needed(p) + 1, seed=84)
+    ref, dref, nw = util.run_hostemu_diag(p, arrs, diag, NPROMA, NBLK, NGPTOT, flags=0x100)
+    try:
+        cloudsc.setup(p)
+        d = {k: torch.from_numpy(v).cuda() for k, v in arrs.items()}
+        g = {k: torch.from_numpy(v).cuda() for k, v in diag.items()}
+        cnt = torch.zeros(1, dtype=torch.int32, device="cuda")
+        cloudsc.cloudsc_batched_diag(p, d, g, NPROMA, util.KLEV, NBLK, NGPTOT, util.PTSPHY, counter=cnt)
+        torch.cuda.synchronize()
+    finally:
+        cloudsc.setup(p0)
+    _same({n: d[n].cpu().numpy() for n in util.COMPARED}, ref)
+    for n in ("pfsd", "pextra"):
+        a, b = (util._valid_cols(x, NGPTOT, NPROMA) for x in (g[n].cpu().numpy(), dref[n]))
+        assert np.array_equal(a, b, equal_nan=True), n
+    assert int(cnt.item()) == nw

@@ -71,26 +71,31 @@ def run_oracle(po, arrs, nproma, ngpblks, ngptot, nthreads=0, libm="plibm", klev
     return ref, nwarn
 
 
+# Host builds of the column code.  "redo": every column of the fast pass reports
+# and runs again with IEEE division; "window": counts operands outside the fast
+# pass's windows; "lanes", "lanes_wide": every warp vote won, the GPU's division
+# and root sequences, and the same count, in the kernels' narrow and 256-thread
+# forms.
+HOSTEMU = {"plibm": "libcloudsc_hostemu.so", "glibc": "libcloudsc_hostemu_glibc.so",
+           "redo": "libcloudsc_hostemu_redo.so", "window": "libcloudsc_hostemu_window.so",
+           "lanes": "libcloudsc_hostemu_lanes.so", "lanes_wide": "libcloudsc_hostemu_lanes_wide.so"}
+HOSTEMU_COUNTS = ("window", "lanes", "lanes_wide")
+
+
 def run_hostemu(p, arrs, nproma, ngpblks, ngptot, precision=0, libm="plibm", klev=KLEV):
     """The kernel's own column code built for the host (tests/hostemu)."""
     import ctypes
     import os
+    import subprocess
     here = os.path.join(os.path.dirname(os.path.abspath(__file__)), "hostemu")
-    # "redo": every column of the fast pass reports and runs again with IEEE
-    # division; "window": counts operands outside the fast pass's windows
-    name = {"plibm": "libcloudsc_hostemu.so", "glibc": "libcloudsc_hostemu_glibc.so",
-            "redo": "libcloudsc_hostemu_redo.so", "window": "libcloudsc_hostemu_window.so"}[libm]
-    path = os.path.join(here, name)
-    if not os.path.exists(path):
-        import subprocess
-        subprocess.run(["make", "-s", "-C", here], check=True)
-    L = ctypes.CDLL(path)
+    subprocess.run(["make", "-s", "-j4", "-C", here], check=True)
+    L = ctypes.CDLL(os.path.join(here, HOSTEMU[libm]))
     out = {k: v.copy() for k, v in arrs.items()}
     ptrs = (ctypes.c_void_p * len(fields.BATCHED_FIELDS))(
         *[out[n].ctypes.data for n, *_ in fields.BATCHED_FIELDS])
     nw = L.hostemu_batched(ctypes.byref(p), int(nproma), int(klev), int(ngpblks), int(ngptot),
                            ctypes.c_double(PTSPHY), ptrs, int(precision))
-    if libm == "window":
+    if libm in HOSTEMU_COUNTS:
         L.hostemu_window_violations.restype = ctypes.c_ulonglong
         return out, nw, L.hostemu_window_violations()
     return out, nw
@@ -252,10 +257,8 @@ def run_hostemu_diag(p, arrs, diag, nproma, ngpblks, ngptot, libm="plibm", flags
     import os
     import subprocess
     here = os.path.join(os.path.dirname(os.path.abspath(__file__)), "hostemu")
-    subprocess.run(["make", "-s", "-C", here], check=True)
-    name = {"plibm": "libcloudsc_hostemu.so", "glibc": "libcloudsc_hostemu_glibc.so",
-            "redo": "libcloudsc_hostemu_redo.so"}[libm]
-    L = ctypes.CDLL(os.path.join(here, name))
+    subprocess.run(["make", "-s", "-j4", "-C", here], check=True)
+    L = ctypes.CDLL(os.path.join(here, HOSTEMU[libm]))
     out = {k: v.copy() for k, v in arrs.items()}
     dout = {k: v.copy() for k, v in diag.items()}
     a = (ctypes.c_void_p * len(fields.BATCHED_FIELDS))(*[out[n].ctypes.data for n, *_ in fields.BATCHED_FIELDS])
@@ -263,6 +266,9 @@ def run_hostemu_diag(p, arrs, diag, nproma, ngpblks, ngptot, libm="plibm", flags
         *[(dout[n].ctypes.data if dout.get(n) is not None else None) for n, *_ in fields.DIAG_FIELDS])
     nw = L.hostemu_batched_diag(ctypes.byref(p), int(nproma), int(klev), int(ngpblks), int(ngptot),
                                 ctypes.c_double(PTSPHY), a, b, int(dout["pextra"].shape[1]), int(flags))
+    if libm in HOSTEMU_COUNTS:
+        L.hostemu_window_violations.restype = ctypes.c_ulonglong
+        return out, dout, nw, L.hostemu_window_violations()
     return out, dout, nw
 
 
