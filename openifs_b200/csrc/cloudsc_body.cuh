@@ -1227,6 +1227,10 @@ CSC_DEV void cloudsc_column(const FT &F, const Shape &sh, int ib, int jl, bool a
         const bool dep = t < (P.rtt - C(5.)) && qxfg_l > P.rlmin;
         if (CSC_ANY(dep)) {
           Real zsupersatice = DIV((zqsliq - zqsice), zqsice);
+          // 0.9 at most with the physical saturation constants; others that
+          // fast_pass_params_ok lets through can take the exponential below, and
+          // the powers of its result, out of their windows
+          if constexpr (FAST_) REPORT_IF(!(zsupersatice < C(8.0)));
           Real zvpice = DIVP((P.r2es * ei_e) * P.rv, P.rd, P.rcp_rd);
           Real zicenuclei = C(1000.0) * mexp<F32M, FAST_>(C(12.96) * zsupersatice - C(0.639));
           Real zadd = DIV(P.rlstt * (DIV(P.rlstt, (P.rv * t)) - C(1.0)), (C(2.4E-2) * t));

@@ -285,3 +285,7 @@ extern "C" int hostemu_batched_diag(const cloudsc_params *p, int nproma, int kle
   }
   return (int)nwarn;
 }
+
+// Whether the fast pass takes these parameters at all (every column of any
+// others is run again with IEEE division and plibm's full functions).
+extern "C" int hostemu_params_ok(const cloudsc_params *p) { return fast_pass_params_ok(*p) ? 1 : 0; }

@@ -85,20 +85,32 @@ HOSTEMU_COUNTS = ("window", "lanes", "lanes_wide")
 def run_hostemu(p, arrs, nproma, ngpblks, ngptot, precision=0, libm="plibm", klev=KLEV):
     """The kernel's own column code built for the host (tests/hostemu)."""
     import ctypes
-    import os
-    import subprocess
-    here = os.path.join(os.path.dirname(os.path.abspath(__file__)), "hostemu")
-    subprocess.run(["make", "-s", "-j4", "-C", here], check=True)
-    L = ctypes.CDLL(os.path.join(here, HOSTEMU[libm]))
+    L = hostemu(libm)
     out = {k: v.copy() for k, v in arrs.items()}
     ptrs = (ctypes.c_void_p * len(fields.BATCHED_FIELDS))(
         *[out[n].ctypes.data for n, *_ in fields.BATCHED_FIELDS])
     nw = L.hostemu_batched(ctypes.byref(p), int(nproma), int(klev), int(ngpblks), int(ngptot),
                            ctypes.c_double(PTSPHY), ptrs, int(precision))
     if libm in HOSTEMU_COUNTS:
-        L.hostemu_window_violations.restype = ctypes.c_ulonglong
-        return out, nw, L.hostemu_window_violations()
+        return out, nw, hostemu_violations(L)
     return out, nw
+
+
+def hostemu(libm):
+    """The host build `libm` of the column code, made up to date."""
+    import ctypes
+    import os
+    import subprocess
+    here = os.path.join(os.path.dirname(os.path.abspath(__file__)), "hostemu")
+    subprocess.run(["make", "-s", "-j4", "-C", here], check=True)
+    return ctypes.CDLL(os.path.join(here, HOSTEMU[libm]))
+
+
+def hostemu_violations(L):
+    """Operands outside the windows that a counting build has met so far."""
+    import ctypes
+    L.hostemu_window_violations.restype = ctypes.c_ulonglong
+    return L.hostemu_window_violations()
 
 
 EDGE_CASES = ["clear", "overcast", "warm", "cold", "no_convection", "all_convection", "land",
@@ -254,11 +266,7 @@ def run_hostemu_diag(p, arrs, diag, nproma, ngpblks, ngptot, libm="plibm", flags
     flags 0x100 for the GEN column code, 0x200 for the kernels' fast pass with
     its rerun."""
     import ctypes
-    import os
-    import subprocess
-    here = os.path.join(os.path.dirname(os.path.abspath(__file__)), "hostemu")
-    subprocess.run(["make", "-s", "-j4", "-C", here], check=True)
-    L = ctypes.CDLL(os.path.join(here, HOSTEMU[libm]))
+    L = hostemu(libm)
     out = {k: v.copy() for k, v in arrs.items()}
     dout = {k: v.copy() for k, v in diag.items()}
     a = (ctypes.c_void_p * len(fields.BATCHED_FIELDS))(*[out[n].ctypes.data for n, *_ in fields.BATCHED_FIELDS])
@@ -267,8 +275,7 @@ def run_hostemu_diag(p, arrs, diag, nproma, ngpblks, ngptot, libm="plibm", flags
     nw = L.hostemu_batched_diag(ctypes.byref(p), int(nproma), int(klev), int(ngpblks), int(ngptot),
                                 ctypes.c_double(PTSPHY), a, b, int(dout["pextra"].shape[1]), int(flags))
     if libm in HOSTEMU_COUNTS:
-        L.hostemu_window_violations.restype = ctypes.c_ulonglong
-        return out, dout, nw, L.hostemu_window_violations()
+        return out, dout, nw, hostemu_violations(L)
     return out, dout, nw
 
 
