@@ -563,8 +563,11 @@ size_t cloudsc_b200_params_size(void);
  *
  * cloudsc_b200_set_schedule(): variant, columns per CTA (a multiple of 32 up
  * to the variant's max_threads) and ctas_per_sm, the persistent CTAs resident
- * per SM (0 = one CTA per tile of columns, a grid over all tiles).  Default:
- * the (448, 1) variant, 448 columns per CTA, ctas_per_sm 0.
+ * per SM (0 = one CTA per tile of columns, a grid over all tiles).
+ * threads_per_cta 0 with ctas_per_sm 0 is the default: each call takes the
+ * variant and the CTA size that its number of columns asks for (spread evenly
+ * over the SMs and the waves).  cloudsc_b200_get_schedule() reports what is
+ * set, so that setting what it reports restores it.
  * cloudsc_b200_set_launch(): the same with the variant chosen as the one-CTA-
  * per-SM variant with the most registers that holds threads_per_cta.
  * Return CLOUDSC_E_SHAPE for values outside these limits.

@@ -148,12 +148,15 @@ def variant_info(precision, variant):
 
 
 def set_schedule(precision, variant, threads_per_cta, ctas_per_sm):
+    """The schedule of every later call of `precision`; threads_per_cta and
+    ctas_per_sm 0: each call by its number of columns (the default)."""
     return _check(lib().cloudsc_b200_set_schedule(int(precision), int(variant), int(threads_per_cta),
                                                   int(ctas_per_sm)))
 
 
 def get_schedule(precision):
-    """(variant, threads_per_cta, ctas_per_sm) used for `precision`."""
+    """(variant, threads_per_cta, ctas_per_sm) set for `precision`; threads_per_cta
+    0: by size.  set_schedule of these restores them."""
     v = [ctypes.c_int32() for _ in range(3)]
     _check(lib().cloudsc_b200_get_schedule(int(precision), *[ctypes.byref(x) for x in v]))
     return tuple(x.value for x in v)

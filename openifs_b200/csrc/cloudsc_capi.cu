@@ -59,13 +59,13 @@ unsigned long long g_gen_count = 0;  // parameter uploads so far
 constexpr int kMaxDev = 64;
 unsigned long long g_dev_gen[kMaxDev] = {0};
 // Launch schedule per precision (0 FP64, 1 FP32-mixed, 2 FP32 physics): compiled variant,
-// columns per CTA, persistent CTAs per SM (0: one CTA per column tile).  Until
-// one is set, each call takes the one pick_schedule gives for its size.
+// columns per CTA, persistent CTAs per SM (0: one CTA per column tile).  With
+// threads = 0 (the default) each call takes the one pick_schedule gives for its
+// size.
 struct Schedule {
   int variant, threads, ctas_per_sm;
-  bool set = false;
 };
-Schedule g_sched[3] = {{default_variant(), 448, 0}, {default_variant(), 448, 0}, {default_variant(), 448, 0}};
+Schedule g_sched[3] = {{default_variant(), 0, 0}, {default_variant(), 0, 0}, {default_variant(), 0, 0}};
 
 // The fixed device array of cloudsc_b200_block_noalloc (see that entry).  It
 // is the only device object of this file, so this file's device module --
@@ -458,12 +458,13 @@ int cloudsc_b200_set_schedule(int32_t precision, int32_t variant, int32_t thread
   if (variant < 0 || variant >= num_variants()) return fail(CLOUDSC_E_SHAPE, "no such variant");
   int mt = 0, mb = 0;
   variant_bounds(variant, &mt, &mb);
-  if (threads_per_cta < 32 || threads_per_cta > mt || threads_per_cta % 32)
+  const bool by_size = threads_per_cta == 0 && ctas_per_sm == 0;
+  if (!by_size && (threads_per_cta < 32 || threads_per_cta > mt || threads_per_cta % 32))
     return fail(CLOUDSC_E_SHAPE, "threads_per_cta must be a multiple of 32, at least 32 and at most "
-                                 "the variant's compiled limit");
+                                 "the variant's compiled limit (or 0 with ctas_per_sm 0: by size)");
   if (ctas_per_sm < 0 || ctas_per_sm > 32) return fail(CLOUDSC_E_SHAPE, "ctas_per_sm must be in [0,32]");
   std::lock_guard<std::mutex> lk(g_mu);
-  g_sched[precision] = {variant, threads_per_cta, ctas_per_sm, true};
+  g_sched[precision] = {variant, threads_per_cta, ctas_per_sm};
   return CLOUDSC_OK;
 }
 
@@ -503,7 +504,7 @@ int cloudsc_b200_set_launch(int32_t precision, int32_t threads_per_cta, int32_t 
 // kMaxLevFast levels and some forms have fewer builds), or pick_schedule's.
 static Schedule resolve_schedule(Schedule sc, int form, bool gen, const Shape &sh, bool sp, int *grid) {
   const long long cols = (long long)sh.ngpblks * sh.nproma;
-  if (!sc.set) {
+  if (sc.threads == 0) {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -44,6 +44,24 @@ def test_schedule_limits(restore_schedule):
     assert t == 128 and info[v]["max_threads"] == min(info[u]["max_threads"] for u in fits)
 
 
+def test_setting_what_is_reported_changes_nothing(restore_schedule):
+    """A set schedule can be taken back: the default, each call by its number of
+    columns, reads as 0 threads and is restored by setting what was read."""
+    for prec in (cloudsc.FP64, cloudsc.MIXED, cloudsc.PHYS32):
+        default = cloudsc.get_schedule(prec)
+        assert default[1:] == (0, 0)
+        cloudsc.set_schedule(prec, *default)
+        assert cloudsc.get_schedule(prec) == default
+        cloudsc.set_schedule(prec, 1, 448, 0)
+        assert cloudsc.get_schedule(prec) == (1, 448, 0)
+        cloudsc.set_schedule(prec, *default)
+        assert cloudsc.get_schedule(prec) == default
+    with pytest.raises(cloudsc.CloudscError):
+        cloudsc.set_schedule(cloudsc.FP64, 1, 0, 2)
+    with pytest.raises(cloudsc.CloudscError):
+        cloudsc.set_launch(cloudsc.FP64, 0, 0)
+
+
 def test_tune_picks_fastest_and_caches(tmp_path, restore_schedule):
     cache = str(tmp_path / "sched.json")
     cands = autotune.candidates(cloudsc.FP64)
