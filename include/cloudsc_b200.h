@@ -571,6 +571,11 @@ size_t cloudsc_b200_params_size(void);
  * cloudsc_b200_set_launch(): the same with the variant chosen as the one-CTA-
  * per-SM variant with the most registers that holds threads_per_cta.
  * Return CLOUDSC_E_SHAPE for values outside these limits.
+ *
+ * cloudsc_b200_schedule_by_size(): with on != 0, the calling thread's calls
+ * take the choice by size whatever is set, until it is turned off; returns
+ * whether it was on.  For a library that runs small batches of its own beside
+ * its caller's.
  */
 int cloudsc_b200_num_variants(void);
 int cloudsc_b200_variant_info(int32_t precision, int32_t variant, int32_t *max_threads,
@@ -580,6 +585,7 @@ int cloudsc_b200_set_schedule(int32_t precision, int32_t variant, int32_t thread
 int cloudsc_b200_get_schedule(int32_t precision, int32_t *variant, int32_t *threads_per_cta,
                               int32_t *ctas_per_sm);
 int cloudsc_b200_set_launch(int32_t precision, int32_t threads_per_cta, int32_t ctas_per_sm);
+int cloudsc_b200_schedule_by_size(int32_t on);
 
 /*
  * Self-check of the division the column kernels use (no reference

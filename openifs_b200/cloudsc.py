@@ -11,6 +11,7 @@ warning events the reference would have written to NULOUT
 There is no CPU fallback: if the library is missing or no GPU is present the
 calls raise.
 """
+import contextlib
 import ctypes
 import functools
 import os
@@ -63,6 +64,8 @@ def lib():
         L.cloudsc_b200_set_schedule.restype = ctypes.c_int
         L.cloudsc_b200_get_schedule.argtypes = [i32, pi32, pi32, pi32]
         L.cloudsc_b200_get_schedule.restype = ctypes.c_int
+        L.cloudsc_b200_schedule_by_size.argtypes = [i32]
+        L.cloudsc_b200_schedule_by_size.restype = ctypes.c_int
         from .fields import DIAG_FIELDS
         L.cloudsc_b200_batched_diag.argtypes = ([P, i32, i32, i32, i32, ctypes.c_double] +
                                                 [vp] * (len(BATCHED_FIELDS) + len(DIAG_FIELDS)) + [i32, vp, vp])
@@ -160,6 +163,17 @@ def get_schedule(precision):
     v = [ctypes.c_int32() for _ in range(3)]
     _check(lib().cloudsc_b200_get_schedule(int(precision), *[ctypes.byref(x) for x in v]))
     return tuple(x.value for x in v)
+
+
+@contextlib.contextmanager
+def schedule_by_size():
+    """Within it, this thread's calls take the schedule that their number of
+    columns asks for, whatever schedule is set."""
+    before = lib().cloudsc_b200_schedule_by_size(1)
+    try:
+        yield
+    finally:
+        lib().cloudsc_b200_schedule_by_size(before)
 
 
 def _ptr(x):

@@ -66,6 +66,8 @@ struct Schedule {
   int variant, threads, ctas_per_sm;
 };
 Schedule g_sched[3] = {{default_variant(), 0, 0}, {default_variant(), 0, 0}, {default_variant(), 0, 0}};
+// Whether this thread's calls take the choice by size whatever is set.
+thread_local bool t_by_size = false;
 
 // The fixed device array of cloudsc_b200_block_noalloc (see that entry).  It
 // is the only device object of this file, so this file's device module --
@@ -479,6 +481,12 @@ int cloudsc_b200_get_schedule(int32_t precision, int32_t *variant, int32_t *thre
   return CLOUDSC_OK;
 }
 
+int cloudsc_b200_schedule_by_size(int32_t on) {
+  const int before = t_by_size ? 1 : 0;
+  t_by_size = on != 0;
+  return before;
+}
+
 // The variant with the most registers per thread that still holds a CTA of
 // threads_per_cta: the smallest compiled limit >= threads_per_cta among the
 // one-CTA-per-SM variants.
@@ -504,7 +512,7 @@ int cloudsc_b200_set_launch(int32_t precision, int32_t threads_per_cta, int32_t 
 // kMaxLevFast levels and some forms have fewer builds), or pick_schedule's.
 static Schedule resolve_schedule(Schedule sc, int form, bool gen, const Shape &sh, bool sp, int *grid) {
   const long long cols = (long long)sh.ngpblks * sh.nproma;
-  if (sc.threads == 0) {
+  if (sc.threads == 0 || t_by_size) {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

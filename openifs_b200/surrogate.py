@@ -483,10 +483,12 @@ class Runner:
                               1, s), "cs_move_columns")
 
     def _fallback(self, s):
-        """FP64 CLOUDSC on the compact batch of flagged columns (a fraction of
-        a wave of columns: the call spreads them over every SM)."""
-        cloudsc.cloudsc_batched(self.params, self.compact, self.nproma, KLEV, self.cap // self.nproma, self.cap,
-                                self.ptsphy, stream=s)
+        """FP64 CLOUDSC on the compact batch of flagged columns: a fraction of
+        a wave of columns, spread over every SM whatever schedule is set for
+        full-size calls (3,072 columns in CTAs of 384 would run on 8 SMs)."""
+        with cloudsc.schedule_by_size():
+            cloudsc.cloudsc_batched(self.params, self.compact, self.nproma, KLEV, self.cap // self.nproma, self.cap,
+                                    self.ptsphy, stream=s)
 
     def flops_per_batch(self):
         """Multiply-add FLOPs of the network's GEMMs for one batch (padded rows included)."""

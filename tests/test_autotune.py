@@ -98,3 +98,36 @@ def test_tune_restores_schedule_on_error(tmp_path, restore_schedule):
         autotune.tune(None, None, 128, 137, 4, 512, 3600.0, cloudsc.MIXED, cache=None, timer=timer,
                       device_name="fake")
     assert cloudsc.get_schedule(cloudsc.MIXED) == before
+
+
+def test_fallback_columns_take_the_choice_by_size(restore_schedule, monkeypatch):
+    """The surrogate's FP64 fallback runs its few columns by size, whatever
+    schedule is set for full-size calls, and leaves the thread and the set
+    schedule as it found them, also when the call raises."""
+    from openifs_b200 import surrogate
+    L, seen = cloudsc.lib(), []
+
+    def by_size():
+        on = L.cloudsc_b200_schedule_by_size(0)
+        L.cloudsc_b200_schedule_by_size(on)
+        return on
+
+    def call(*args, **kw):
+        seen.append(by_size())
+        if len(seen) == 2:
+            raise RuntimeError("launch failed")
+
+    monkeypatch.setattr(cloudsc, "cloudsc_batched", call)
+    r = surrogate.Runner.__new__(surrogate.Runner)
+    r.params, r.compact, r.nproma, r.cap, r.ptsphy = None, {}, 128, 3072, 3600.0
+    cloudsc.set_schedule(cloudsc.FP64, 2, 384, 0)
+    assert by_size() == 0
+    r._fallback(None)
+    assert by_size() == 0
+    with pytest.raises(RuntimeError):
+        r._fallback(None)
+    assert by_size() == 0 and seen == [1, 1]
+    with cloudsc.schedule_by_size(), cloudsc.schedule_by_size():
+        assert by_size() == 1
+    assert by_size() == 0
+    assert cloudsc.get_schedule(cloudsc.FP64) == (2, 384, 0)
