@@ -846,7 +846,7 @@ __device__ __forceinline__ void red_add_v4(float *p, float a, float b, float c, 
 template <int BN>
 __global__ void __launch_bounds__(128, 1)
     wgrad_tc_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmX, int rows,
-                    int chunk, int n, int taps, float *dw, float *db, unsigned *err) {
+                    int chunk, int n, int taps, int dbtaps, float *dw, float *db, unsigned *err) {
   // transpose bits 15 and 16: both operands MN-major
   constexpr uint32_t IDESC = tcg::idesc_bf16_f32(128, BN) | (1u << 15) | (1u << 16);
   constexpr uint32_t IDESC1 = tcg::idesc_bf16_f32(128, 16) | (1u << 15) | (1u << 16);
@@ -866,8 +866,9 @@ __global__ void __launch_bounds__(128, 1)
   const int nh = n / 64;
   constexpr int KH = BN / 64;
   // the bias gradient, dZ's column sums: one more product with a matrix of
-  // ones (16 of its columns, the narrowest N), by the CTAs of the first tap
-  const bool bias = db != nullptr && t == 0;
+  // ones (16 of its columns, the narrowest N), by the CTAs of the first dbtaps
+  // taps, which share the chunk's row blocks
+  const bool bias = db != nullptr && t < dbtaps && t < nkb;
   if (bias) {
     for (int i = tid; i < WG_HALF / 4; i += blockDim.x) reinterpret_cast<uint32_t *>(smem + WG_ONES)[i] = 0x3f803f80u;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -934,12 +935,12 @@ __global__ void __launch_bounds__(128, 1)
       for (int kk = 0; kk < WG_RK / 16; ++kk)  // 16 rows = two 1024-byte groups per instruction
         tcg::mma_bf16(tmem, da + (uint64_t)(kk * (2048 >> 4)), dbx + (uint64_t)(kk * (2048 >> 4)), IDESC,
                       (kb > 0 || kk > 0) ? 1u : 0u);
-      if (bias) {
+      if (bias && kb % dbtaps == t) {
         const uint64_t d1 = sdesc_mn_sw128(tcg::smem_u32(smem + WG_ONES), WG_HALF);
 #pragma unroll
         for (int kk = 0; kk < WG_RK / 16; ++kk)
           tcg::mma_bf16(tmem + BN, da + (uint64_t)(kk * (2048 >> 4)), d1 + (uint64_t)(kk * (2048 >> 4)), IDESC1,
-                        (kb > 0 || kk > 0) ? 1u : 0u);
+                        (kb > t || kk > 0) ? 1u : 0u);
       }
       tcg::mma_commit(&empty[s]);
       *consumed = (uint32_t)(kb + 1);
@@ -1067,14 +1068,14 @@ cudaError_t launch_ws_n(const CUtensorMap &ma, const CUtensorMap &mb, const Args
 
 template <int BN>
 cudaError_t launch_wgrad_t(const CUtensorMap &md, const CUtensorMap &mx, int rows, int chunk, int nchunks, int n,
-                           int taps, float *dw, float *db, unsigned *err, cudaStream_t st) {
+                           int taps, int dbtaps, float *dw, float *db, unsigned *err, cudaStream_t st) {
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(wgrad_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM);
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  wgrad_tc_kernel<BN><<<dim3(nchunks, taps), 128, WG_SMEM, st>>>(md, mx, rows, chunk, n, taps, dw, db, err);
+  wgrad_tc_kernel<BN><<<dim3(nchunks, taps), 128, WG_SMEM, st>>>(md, mx, rows, chunk, n, taps, dbtaps, dw, db, err);
   return cudaGetLastError();
 }
 
@@ -1187,19 +1188,26 @@ int wgrad_tc(const void *dz, const void *x, int32_t rows, int32_t n, int32_t k, 
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // one CTA per SM (its ring and the ones fill the shared memory) over all
-  // taps, in one wave; chunks of at least 512 rows (each chunk adds its n x k
-  // partial to dW)
-  int nchunks = sms / taps;
+  // about two CTAs per SM over all taps, in two waves; chunks of at least 512
+  // rows (each chunk adds its n x k partial to dW).  The tensor cores' f32
+  // accumulation drifts in proportion to the rows of a chunk: one wave of
+  // chunks twice as long doubles dW's error against 64-bit sums (5 taps,
+  // 73,728 rows: 2.7e-6 relative against 1.3e-6).
+  int nchunks = (2 * sms + taps - 1) / taps;
   const int maxchunks = (rows + 511) / 512;
   if (nchunks > maxchunks) nchunks = maxchunks;
   if (nchunks < 1) nchunks = 1;
   int chunk = (rows + nchunks - 1) / nchunks;
   chunk = (chunk + WG_RK - 1) / WG_RK * WG_RK;
   nchunks = (rows + chunk - 1) / chunk;
+  // db: each CTA's sum drifts with its length, each one more adds a rounding;
+  // one tap's CTAs sum chunks of up to 2,048 rows, all taps' longer ones (5
+  // taps, chunks of 20,000 rows by one tap: 4e-6 relative; f32 sums of 128 rows
+  // added atomically: 1e-6)
+  const int dbtaps = chunk > 2048 ? taps : 1;
   cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t e = k == 128 ? launch_wgrad_t<128>(md, mx, rows, chunk, nchunks, n, taps, dw, db, err, st)
-                           : launch_wgrad_t<64>(md, mx, rows, chunk, nchunks, n, taps, dw, db, err, st);
+  cudaError_t e = k == 128 ? launch_wgrad_t<128>(md, mx, rows, chunk, nchunks, n, taps, dbtaps, dw, db, err, st)
+                           : launch_wgrad_t<64>(md, mx, rows, chunk, nchunks, n, taps, dbtaps, dw, db, err, st);
   return e == cudaSuccess ? CS_OK : CS_E_CUDA;
 }
 extern "C" int cs_wgrad_tc(const void *dz, const void *x, int32_t rows, int32_t n, int32_t k, int32_t taps,

@@ -98,6 +98,60 @@ def test_weight_gradient_gemm(cuda, n, k, taps, rows):
     assert np.abs(got - ref).max() <= 1e-4 * scale, np.abs(got - ref).max()
 
 
+def _wgrad(dz, x, taps, dw, db):
+    L = S._lib()
+    S._ok(L.cs_wgrad(dz.data_ptr(), x.data_ptr(), dz.shape[0], dz.shape[1], x.shape[1], taps, dw.data_ptr(),
+                     db.data_ptr(), S._stream()), "cs_wgrad")
+
+
+@pytest.mark.parametrize("n,k,taps,rows", [(128, 128, 5, 20_000), (128, 128, 1, 7_777), (64, 128, 1, 9_000),
+                                           (64, 64, 5, 12_345), (128, 64, 5, 3_001), (64, 64, 1, 100), (64, 64, 5, 100),
+                                           (128, 128, 5, 1), (128, 128, 5, 513), (64, 128, 1, 64)])
+def test_bias_gradient(cuda, n, k, taps, rows):
+    """cs_wgrad's db, the column sums of dZ shared by the taps' CTAs (down to
+    fewer row blocks than taps), against float64 sums of the same bf16 values;
+    it accumulates onto what db holds, and dW is that of cs_wgrad_tc.  The sums
+    are about sqrt(rows); f32 sums of up to a few thousand of them are off by
+    less than 1e-6 of that."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(rows + n)
+    dz = torch.randn(rows, n, generator=g, device="cuda").bfloat16()
+    x = torch.randn(rows, k, generator=g, device="cuda").bfloat16()
+    init = torch.randn(n, generator=g, device="cuda")
+    db, dw, dw2 = init.clone(), torch.zeros(taps, n, k, device="cuda"), torch.zeros(taps, n, k, device="cuda")
+    _wgrad(dz, x, taps, dw, db)
+    assert S._lib().cs_wgrad_tc(dz.data_ptr(), x.data_ptr(), rows, n, k, taps, dw2.data_ptr(), None, S._stream()) == 0
+    ref = init.double() + dz.double().sum(0)
+    assert (db.double() - ref).abs().max().item() <= 4e-6 * np.sqrt(rows)
+    assert (dw - dw2).abs().max().item() <= 1e-5 * np.sqrt(rows)
+
+
+@pytest.mark.parametrize("n,k,taps,cols", [(128, 128, 5, 333), (128, 128, 5, 512), (128, 128, 1, 1000), (64, 64, 5, 1000)])
+def test_weight_gradient_precision(cuda, n, k, taps, cols):
+    """Over the batches training uses: the relative error of dW (2-norm) against
+    64-bit sums grows with the rows a CTA accumulates, ceil(rows / CTAs per tap)
+    of them: 1.05e-9 a row measured, 5e-7 for the f32 rounding of the rest; a
+    third more allowed.  db, summed by all taps' CTAs, stays below 6e-7."""
+    import torch
+    rows = cols * S.LP
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    dz = torch.randn(rows, n, generator=g, device="cuda").bfloat16()
+    x = torch.randn(rows, k, generator=g, device="cuda").bfloat16()
+    dw, db = torch.zeros(taps, n, k, device="cuda"), torch.zeros(n, device="cuda")
+    _wgrad(dz, x, taps, dw, db)
+    D, X = dz.double(), x.double()
+    ref = torch.zeros(taps, n, k, dtype=torch.float64, device="cuda")
+    for t in range(taps):
+        s = t - taps // 2
+        lo, hi = max(0, -s), min(rows, rows - s)
+        ref[t] = D[lo:hi].T @ X[lo + s:hi + s]
+    rel = ((dw.double() - ref).norm() / ref.norm()).item()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    chunk = max(512, rows / (2 * sms / taps))
+    assert rel <= (5e-7 + 1.05e-9 * chunk) * 4 / 3, rel
+    assert ((db.double() - D.sum(0)).norm() / D.sum(0).norm()).item() <= 6e-7
+
+
 def test_weight_gradient_rejects_bad_shapes(cuda):
     import torch
     L = S._lib()
