@@ -563,7 +563,9 @@ size_t cloudsc_b200_params_size(void);
  *
  * cloudsc_b200_set_schedule(): variant, columns per CTA (a multiple of 32 up
  * to the variant's max_threads) and ctas_per_sm, the persistent CTAs resident
- * per SM (0 = one CTA per tile of columns, a grid over all tiles).
+ * per SM (0 = one CTA per tile of columns, a grid over all tiles).  CTAs of at
+ * most 256 columns on a variant that only fits one CTA on an SM run on the
+ * (256, 1) variant, or by size where the form has none.
  * threads_per_cta 0 with ctas_per_sm 0 is the default: each call takes the
  * variant and the CTA size that its number of columns asks for (spread evenly
  * over the SMs and the waves).  cloudsc_b200_get_schedule() reports what is

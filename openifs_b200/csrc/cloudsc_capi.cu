@@ -30,6 +30,7 @@ void variant_bounds(int v, int *maxt, int *minb);
 cudaError_t variant_attributes(int precision, int v, int *regs, int *local_bytes);
 cudaError_t prepare_kernels(size_t *max_local);
 int kernel_max_threads(int precision, int v, bool gen, int klev, bool sp);
+int variant_for_threads(int precision, int v, int threads, bool gen, int klev, bool sp);
 void pick_schedule(int precision, bool gen, int klev, bool sp, long long ncols, int sms, int *variant, int *threads);
 cudaError_t launch(int precision, int v, const Fields &f, const Shape &sh, int threads, int grid,
                    cudaStream_t stream, bool gen);
@@ -509,10 +510,18 @@ int cloudsc_b200_set_launch(int32_t precision, int32_t threads_per_cta, int32_t 
 
 // The schedule of one call: the caller's, its CTA cut to what the kernel that
 // will run takes (parameters that rule out the GEN kernels, more than
-// kMaxLevFast levels and some forms have fewer builds), or pick_schedule's.
+// kMaxLevFast levels and some forms have fewer builds) and small CTAs moved to
+// the build that shares an SM among them (variant_for_threads), or
+// pick_schedule's.
 static Schedule resolve_schedule(Schedule sc, int form, bool gen, const Shape &sh, bool sp, int *grid) {
   const long long cols = (long long)sh.ngpblks * sh.nproma;
-  if (sc.threads == 0 || t_by_size) {
+  bool by_size = sc.threads == 0 || t_by_size;
+  if (!by_size) {
+    const int v = variant_for_threads(form, sc.variant, sc.threads, gen, sh.klev, sp);
+    by_size = v < 0;
+    if (v >= 0) sc.variant = v;
+  }
+  if (by_size) {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

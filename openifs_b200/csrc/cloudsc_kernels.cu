@@ -55,6 +55,23 @@ int kernel_max_threads(int precision, int v, bool gen, int klev, bool sp) {
   return (sp ? find_kernel_sp(precision, v, gen, fast) : find_kernel(precision, v, gen, fast)).maxt;
 }
 
+// The variant that runs CTAs of `threads` columns set for variant v.  A build
+// that parks values in shared memory takes that of a full CTA, so an SM holds
+// one CTA however small; up to 256 threads the 256-thread build, which parks
+// nothing and shares an SM, is the faster one for every form (ms, CTAs of 224
+// and 128: FP64, 120,000 columns, on the 448-thread build 7.13 and 10.87, on the
+// 256-thread one 5.44 and 5.78; FP32-mixed 5.98 and 9.21, 4.34 and 4.17; budgets,
+// 60,000 columns, 7.19 and 12.46, 5.70 and 5.79).  -1: the form has no such
+// build (parameters that rule out the GEN kernels).
+int variant_for_threads(int precision, int v, int threads, bool gen, int klev, bool sp) {
+  const bool fast = klev <= kMaxLevFast;
+  const auto find = [&](int u) { return sp ? find_kernel_sp(precision, u, gen, fast) : find_kernel(precision, u, gen, fast); };
+  if (threads > 256 || find(v).smem == 0) return v;
+  for (int u = 0; u < kNumVariants; ++u)
+    if (kVariants[u].maxt == 256 && kVariants[u].minb == 1 && find(u).maxt == 256) return u;
+  return -1;
+}
+
 // Variant and CTA size for a call of ncols columns when the caller has set no
 // schedule.  A launch is one CTA per SM at a time in every variant, its CTAs
 // run in waves, and the time of a wave grows little with the columns in it

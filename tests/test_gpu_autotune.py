@@ -47,3 +47,36 @@ def test_variants_identical_and_tuned(cuda):
     finally:
         for pr, s in saved.items():
             cloudsc.set_schedule(pr, *s)
+
+
+@pytest.mark.parametrize("precision", [cloudsc.FP64, cloudsc.MIXED])
+def test_small_ctas_share_an_sm(cuda, precision):
+    """A set schedule of small CTAs on the (448, 1) variant, whose build takes the
+    shared memory of a full CTA, still runs several of them on an SM: 60,000
+    columns in CTAs of 128 take less than twice the time of CTAs of 448 (1.2
+    times measured; 2.3 with one CTA per SM)."""
+    p, _ = util.params()
+    cloudsc.setup(p)
+    nproma, nblk = 100, 600
+    one = inputs.generate(20, nproma, p, seed=78)
+    d = {k: torch.from_numpy(np.concatenate([v] * 30)).cuda() for k, v in one.items()}
+    plude = d["plude"].clone()
+    before = cloudsc.get_schedule(precision)
+    ms = {}
+    try:
+        for threads in (448, 128):
+            cloudsc.set_schedule(precision, 1, threads, 0)
+            t = []
+            for _ in range(5):
+                d["plude"].copy_(plude)
+                a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                a.record()
+                cloudsc.cloudsc_batched(p, d, nproma, util.KLEV, nblk, nproma * nblk, util.PTSPHY, precision=precision,
+                                        stream=torch.cuda.current_stream())
+                b.record()
+                torch.cuda.synchronize()
+                t.append(a.elapsed_time(b))
+            ms[threads] = sorted(t)[2]
+    finally:
+        cloudsc.set_schedule(precision, *before)
+    assert ms[128] < 2.0 * ms[448], ms
