@@ -590,24 +590,27 @@ int cloudsc_b200_set_launch(int32_t precision, int32_t threads_per_cta, int32_t 
 int cloudsc_b200_schedule_by_size(int32_t on);
 
 /*
- * Self-check of the division the column kernels use (no reference
+ * Self-check of the divisions the column kernels use (no reference
  * counterpart).  The column kernels divide in double precision with a
  * branch-free reciprocal-and-residual sequence that returns IEEE a/b exactly
- * for 2^-256 <= |b| < 2^256 and a = 0 or 2^-256 <= |a| < 2^256, and records
- * every operand outside that window; a column with such an operand is run
- * again with IEEE division, so the kernels' results are those of IEEE
- * division throughout.  This entry runs that division alone on n device
- * operand pairs: q[i] = its quotient, bad[i] = 1 where an operand lies outside
- * the window (0 otherwise).  Device pointers; stream may be NULL.
+ * for 2^-256 <= |b| < 2^256 and a = 0 or 2^-256 <= |a| < 2^256, except for a
+ * divisor whose significand is all ones, which they record.  Checks of each
+ * level's inputs and solved amounts keep the operands inside that window; a
+ * column that fails one, or has such a divisor, is run again with IEEE
+ * division, so the kernels' results are those of IEEE division throughout.
+ * This entry runs the kernels' divisions alone on n device operand pairs, in
+ * each of the forms they take: q[i] = the quotient (the IEEE one for an
+ * all-ones divisor; a zero with IEEE's sign), bad[i] = 1 where an operand lies
+ * outside the window or the forms differ (0 otherwise).  Device pointers;
+ * stream may be NULL.
  * CLOUDSC_E_SHAPE for n < 0, CLOUDSC_E_NULL for a NULL array with n > 0.
  */
 int cloudsc_b200_division_check(const double *a, const double *b, int64_t n, double *q, int32_t *bad,
                                 void *stream);
 
 /*
- * The reciprocal half of that division on its own (no reference
- * counterpart): the kernels take 1/b this way, and the reciprocal of a
- * divisor shared by several quotients once.  y[i] = the reciprocal of b[i],
+ * The reciprocal the kernels take for 1/b, and once for a divisor that several
+ * quotients share (no reference counterpart).  y[i] = the reciprocal of b[i],
  * IEEE 1/b bit for bit for 2^-256 <= |b| < 2^256; bad[i] = 1 where b lies
  * outside that window (0 otherwise).  Device pointers; stream may be NULL.
  * CLOUDSC_E_SHAPE for n < 0, CLOUDSC_E_NULL for a NULL array with n > 0.

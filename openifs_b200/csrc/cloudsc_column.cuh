@@ -244,38 +244,6 @@ CSC_DEV double csqrt(double x, DivCheck &dc) {
   return sqrt(x);
 }
 
-// The two halves as one self-contained division with its own checks (the
-// division and reciprocal check entries): an all-ones divisor's reciprocal
-// gets its low significand bit set (which gives RN(1/b) = 2^(-E-1)(1 + 2^-52);
-// a clamped shift of the all-ones test, no branch), a's sign is put back at
-// the end so that zero quotients have IEEE's sign, and operands outside the
-// windows 2^-256 <= |b| < 2^256, a = 0 or 2^-256 <= |a| < 2^256 are recorded.
-CSC_DEV double fast_rcp(double b, DivCheck &dc) {
-#if defined(__CUDA_ARCH__)
-  double y = fast_rcp_y(b);
-  y = __hiloint2double(__double2hiint(y), __double2loint(y) | (int)__funnelshift_rc(1u, 0u, ~ones_word(b)));
-  dc.acc |= hi_word(b) * 2u - kDivBase;
-  return y;
-#else
-  dc.acc |= hi_word(b) * 2u - kDivBase;
-  return 1.0 / b;
-#endif
-}
-CSC_DEV double fast_div(double a, double b, DivCheck &dc) {
-#if defined(__CUDA_ARCH__)
-  const double y = fast_rcp(b, dc);
-  const double q = fast_quot(fabs(a), b, y);
-  see(a, dc);
-  // the short form must agree wherever its divisor is not reported
-  if (ones_word(b) != ~0u && !dc.bad() && fast_quot_rcp(fabs(a), b) != q) dc.acc = ~0u;
-  return __hiloint2double(__double2hiint(q) ^ (__double2hiint(a) & (int)0x80000000), __double2loint(q));
-#else
-  see(a, dc);
-  dc.acc |= hi_word(b) * 2u - kDivBase;
-  return a / b;
-#endif
-}
-
 #if defined(CLOUDSC_HOST_WINDOW_CHECK) && !defined(__CUDA_ARCH__)
 // Test builds: count the operands of the fast pass outside the range its
 // operations are exact in, in columns that have not been reported.
@@ -346,10 +314,10 @@ CSC_DEV B crcp(B b, DivCheck &dc) {
   }
 }
 
-// Passes of the column code (cloudsc_column's PASS): plain, IEEE division
-// throughout; fast, the branch-free fast_div, recording operands outside its
-// exact window; redo, the rerun with IEEE division of a column whose fast
-// pass recorded one.
+// Passes of the column code (cloudsc_column's PASS): plain, IEEE division and
+// plibm's full functions throughout; fast, the branch-free forms, with checks
+// that report what could leave their exact windows; redo, the plain code again
+// for a column whose fast pass reported.
 enum { kPassPlain = 0, kPassFast = 1, kPassRedo = 2 };
 
 // Double precision uses the portable exp/pow of plibm.h (bit-identical on the
@@ -548,9 +516,10 @@ struct KParams {
   Real rnice;
   int laericesed, laericeauto;
   // Divisions by parameters: RV/RD in the working precision, and the
-  // correctly rounded reciprocals of the parameter divisors, for fast_div_k.
-  // rcp_force: one of those divisors is outside fast_div's window or has an
-  // all-ones significand, and every column takes the IEEE rerun.
+  // correctly rounded reciprocals of the parameter divisors, for cdivk.
+  // rcp_force: one of those divisors is outside the division's window or has an
+  // all-ones significand, or a parameter lies outside fast_pass_params_ok's
+  // ranges, and every column takes the IEEE rerun.
   Real rv_rd;
   double rcp_rd, rcp_rtaumel, rcp_rcl_lam1r, rcp_rdepliqrefdepth, rcp_rvrfactor;
   int rcp_force;

@@ -161,11 +161,11 @@ constexpr size_t park_bytes(int form, int maxt, int minb, bool fast) {
 // forms 0-2 only).  GEN: the parameter-exponent pows without their tests for
 // the exponents 0.5, 1.5, 2 and 3 (the host launches it when the uploaded
 // parameters have none of these, gen_exponents_ok).  FAST (KLEV <=
-// kMaxLevFast): every column runs the fast pass (the branch-free division,
-// fast_div); a column whose pass reported an operand outside that division's
-// exact window is run again with IEEE division, so that the outputs are
-// those of IEEE division for every input (with the budgets, the two passes
-// split PEXTRA's levels between them: cloudsc_column, kbud).
+// kMaxLevFast): every column runs the fast pass (branch-free division, root,
+// exp, log and pow); a column whose checks reported is run again with IEEE
+// division and plibm's full functions, so that the outputs are those for every
+// input (with the budgets, the two passes split PEXTRA's levels between them:
+// cloudsc_column, kbud).
 template <int FORM, int MAXT, int MINB, typename FT = Fields, bool GEN = false, bool FAST = false>
 __global__ void __launch_bounds__(MAXT, MINB) cloudsc_kernel(FT F, Shape sh) {
   // Without parking: let ptxas place part of the register spills in shared memory instead of

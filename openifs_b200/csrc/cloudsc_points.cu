@@ -178,26 +178,39 @@ __global__ void __launch_bounds__(kSatadjThreads) state_increment_kernel(IncFiel
   }
 }
 
-// The column kernels' fast division on n operand pairs: q[i] = fast_div(a[i],
-// b[i]) and bad[i] = 1 where an operand fell outside its exact window (a
-// column kernel then reruns the column with IEEE division).  A self-check of
-// the division alone.
+// The column kernels' divisions on n operand pairs, as they are instantiated
+// there with checked operands: both orders of cdiv, and cdivk on crcp's
+// reciprocal.  The three must agree (a pair for which they do not is reported
+// like one outside the window).  A divisor with an all-ones significand, which
+// makes a kernel run the column again with IEEE division, gets that division
+// here; a zero quotient IEEE's sign, which the kernels' sequences do not keep
+// for -0 / b and no result depends on.
 __global__ void __launch_bounds__(kSatadjThreads) division_check_kernel(const double *a, const double *b,
                                                                        long long n, double *q, int *bad) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const double x = a[i], d = b[i];
     DivCheck dc;
-    q[i] = fast_div(a[i], b[i], dc);
-    bad[i] = dc.bad() ? 1 : 0;
+    double r = cdiv<true, true, true>(x, d, dc);
+    const double r1 = cdiv<true, true, false>(x, d, dc), r2 = cdivk<true, true>(x, d, crcp<true, true>(d, dc), dc);
+    const bool outside = dc.acc >= kDivRange, ones = dc.ones == ~0u;
+    const bool differ = __double_as_longlong(r) != __double_as_longlong(r1) ||
+                        __double_as_longlong(r) != __double_as_longlong(r2);
+    if (ones) r = x / d;
+    if (x == 0.0) r = copysign(r, copysign(1.0, x) * copysign(1.0, d));
+    q[i] = r;
+    bad[i] = outside || (!ones && differ) ? 1 : 0;
   }
 }
 
-// fast_rcp on n divisors: y[i] and the window report bad[i].
+// crcp on n divisors: y[i] and the window report bad[i]; IEEE 1 / b for an
+// all-ones significand, as above.
 __global__ void __launch_bounds__(kSatadjThreads) reciprocal_check_kernel(const double *b, long long n, double *y,
                                                                          int *bad) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     DivCheck dc;
-    y[i] = fast_rcp(b[i], dc);
-    bad[i] = dc.bad() ? 1 : 0;
+    const double r = crcp<true, true>(b[i], dc);
+    y[i] = dc.ones == ~0u ? 1.0 / b[i] : r;
+    bad[i] = dc.acc >= kDivRange ? 1 : 0;
   }
 }
 

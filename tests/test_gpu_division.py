@@ -1,15 +1,15 @@
-"""The column kernels' branch-free division (fast_div in cloudsc_column.cuh)
-against IEEE division, and the column rerun that keeps the kernels' results
-those of IEEE division where it reports an operand (GPU tests).
+"""The column kernels' branch-free divisions (cdiv, cdivk and crcp in
+cloudsc_column.cuh) against IEEE division, and the column rerun that keeps the
+kernels' results those of IEEE division where a column reports (GPU tests).
 
-The division returns a quotient from a Newton-refined reciprocal (corrected
-for divisors whose significand is all ones), corrected twice with its
-residual, with the dividend's sign put back at the end.  Inside its window
-(2^-256 <= |b| < 2^256, and a = 0 or 2^-256 <= |a| < 2^256) it must equal
-IEEE a / b bit for bit, zeros included; every operand outside it must be
-reported (bad = 1), because the kernels then run the column again with IEEE
-division.  The reference quotients are numpy's, IEEE double division on the
-host."""
+The division returns a quotient from a Newton-refined reciprocal, corrected
+twice with its residual, in three forms whose bits the check entry compares.
+Inside the window (2^-256 <= |b| < 2^256, and a = 0 or 2^-256 <= |a| < 2^256)
+the result must equal IEEE a / b bit for bit (the entry returns IEEE division
+for divisors whose significand is all ones, which make a kernel run the column
+again, and IEEE's sign of a zero); every operand outside it, and any pair for
+which the forms differ, is reported (bad = 1).  The reference quotients are
+numpy's, IEEE double division on the host."""
 import numpy as np
 import pytest
 
@@ -132,7 +132,7 @@ def test_hard_operands(cuda):
 
 def test_reciprocal(cuda):
     """The reciprocal the kernels take for 1/b and for a divisor shared by
-    several quotients (fast_rcp, the first half of fast_div): equal to IEEE
+    several quotients (crcp, the first half of the division): equal to IEEE
     1 / b bit for bit inside the window 2^-256 <= |b| < 2^256 and reported
     outside it.  Random significands over exponents of +-1000, all-ones and
     power-of-two significands and a few ulps from them, lognormal values, and
