@@ -231,11 +231,10 @@ int cloudsc_b200_batched(
 /*
  * Batched call with HOST pointers (same arrays and order as
  * cloudsc_b200_batched): blocks are processed in chunks of chunk_blocks
- * (<= 0: as many as give the least estimated time, at most 8,192 columns a
- * chunk), each chunk's host-to-device copy, kernel and
- * device-to-host copy pipelined on three streams over three device buffers,
- * so transfers overlap compute.  Host arrays should be page-locked for the
- * copies to run asynchronously.  Synchronous: returns when all outputs are
+ * (<= 0: cloudsc_b200_host_chunk_blocks), each chunk's host-to-device copy,
+ * kernel and device-to-host copy pipelined on three streams over three device
+ * buffers, so transfers overlap compute.  Host arrays should be page-locked for
+ * the copies to run asynchronously.  Synchronous: returns when all outputs are
  * back in host memory.  Columns beyond NGPTOT in the last block are left
  * untouched.  Replaces the whole EC_PHYS_DRV block loop over CLOUDSC
  * (ec_phys_drv.F90:430-442) for callers that keep the state on the host.
@@ -256,6 +255,16 @@ int cloudsc_b200_batched_host(
     double *pfcqrng, double *pfcqsng, double *pfsqltur, double *pfsqitur,
     double *pfplsl, double *pfplsn, double *pfhpsl, double *pfhpsn,
     int32_t precision, int32_t chunk_blocks);
+
+/*
+ * The blocks per chunk that chunk_blocks <= 0 selects for arrays of this shape
+ * with reals of real_bytes (8 or 4): at most 8,192 columns' worth, or one block;
+ * below that, for page-locked arrays, as many chunks as give the least estimated
+ * time, and for others (whose copies overlap nothing) as few as the limit
+ * allows.  CLOUDSC_E_SHAPE for values out of range.
+ */
+int cloudsc_b200_host_chunk_blocks(int32_t nproma, int32_t klev, int32_t ngpblks, int32_t real_bytes,
+                                   int32_t page_locked);
 
 /*
  * The single-precision interface: the OpenIFS single-precision build

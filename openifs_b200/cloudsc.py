@@ -64,6 +64,8 @@ def lib():
         L.cloudsc_b200_set_schedule.restype = ctypes.c_int
         L.cloudsc_b200_get_schedule.argtypes = [i32, pi32, pi32, pi32]
         L.cloudsc_b200_get_schedule.restype = ctypes.c_int
+        L.cloudsc_b200_host_chunk_blocks.argtypes = [i32] * 5
+        L.cloudsc_b200_host_chunk_blocks.restype = ctypes.c_int
         L.cloudsc_b200_schedule_by_size.argtypes = [i32]
         L.cloudsc_b200_schedule_by_size.restype = ctypes.c_int
         from .fields import DIAG_FIELDS
@@ -288,6 +290,12 @@ def cloudsc_batched_host_sp(params, arrays, nproma, klev, ngpblks, ngptot, ptsph
     return _check(lib().cloudsc_b200_batched_host_sp(
         ctypes.byref(params), int(nproma), int(klev), int(ngpblks), int(ngptot), float(ptsphy),
         *args, int(precision), int(chunk_blocks)))
+
+
+def host_chunk_blocks(nproma, klev, ngpblks, real_bytes=8, page_locked=True):
+    """Blocks per chunk that chunk_blocks=0 of the host entries selects."""
+    return _check(lib().cloudsc_b200_host_chunk_blocks(int(nproma), int(klev), int(ngpblks), int(real_bytes),
+                                                       int(bool(page_locked))))
 
 
 def cloudsc_batched_host(params, arrays, nproma, klev, ngpblks, ngptot, ptsphy, precision=FP64,

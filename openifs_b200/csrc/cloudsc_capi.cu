@@ -898,32 +898,48 @@ int launch_sp_checked(int precision, const FieldsSP &f, const Shape &sh, cudaStr
   return CLOUDSC_OK;
 }
 
-// Blocks per chunk of the host pipeline when the caller leaves it open: the
-// number of chunks n (at most 8,192 columns each) with the least estimated
-// time.  The first chunk's copy in and the last one's copy out are exposed,
-// the rest overlaps; between them run n kernels of one chunk, each the walk
-// down one column (1.25 ms at 137 levels for up to 8,192 columns, however
-// few), or the remaining copies, both directions at once.  Rates measured:
-// 55 GB/s in, 52 out, 80 both.  8,192 columns (host arrays touched before): one
-// chunk 10.0 ms, three 8.6.
-int default_chunk_blocks(size_t np, size_t kl, int ngpblks, size_t fb) {
-  const double cols = (double)np * ngpblks;
-  const double copies = cols * kl * (26.0 / 55e9 + 23.1 / 52e9) * fb;  // seconds, one after the other
-  const double walk = 1.25e-3 * kl / 137.0;
-  int n0 = (int)(cols / 8192.0);
-  if (n0 * 8192.0 < cols) ++n0;
+// Blocks per chunk of the host pipeline when the caller leaves it open, at most
+// 8,192 columns' worth (or one block).  With page-locked arrays, the number of
+// chunks n with the least estimated time: the first chunk's copy in and the last
+// one's copy out are exposed, the rest overlaps; between them run n kernels of
+// one chunk, each the walk down one column (1.25 ms at 137 levels for up to
+// 8,192 columns, however few), or the remaining copies, both directions at once.
+// Rates measured: 55 GB/s in, 52 out, 80 both.  8,192 columns: one chunk 9.3 ms,
+// three 7.7.  Copies of pageable arrays are staged by the host and overlap
+// nothing, so more chunks only add kernels: as few as the limit allows (8,192
+// columns: one chunk 46.6 ms, three 50; 32,768: four 131, eight 145).
+int default_chunk_blocks(size_t np, size_t kl, int ngpblks, size_t fb, bool page_locked) {
+  const int most = np >= 8192 ? 1 : (int)(8192 / np);  // blocks
+  const int n0 = (ngpblks + most - 1) / most;
   int best = n0;
-  double least = 0.0;
-  for (int n = n0; n <= n0 + 8 && n <= ngpblks; ++n) {
-    const double busy = copies * 0.67 * (n - 1) / n;
-    const double t = copies / n + (n * walk > busy ? n * walk : busy);
-    if (n == n0 || t < least) {
-      least = t;
-      best = n;
+  if (page_locked) {
+    const double cols = (double)np * ngpblks;
+    const double copies = cols * kl * (26.0 / 55e9 + 23.1 / 52e9) * fb;  // seconds, one after the other
+    const double walk = 1.25e-3 * kl / 137.0;
+    double least = 0.0;
+    for (int n = n0; n <= n0 + 8 && n <= ngpblks; ++n) {
+      const double busy = copies * 0.67 * (n - 1) / n;
+      const double t = copies / n + (n * walk > busy ? n * walk : busy);
+      if (n == n0 || t < least) {
+        least = t;
+        best = n;
+      }
     }
   }
-  if (best > ngpblks) best = ngpblks;
   return (ngpblks + best - 1) / best;
+}
+
+// Whether every array is page-locked (or device-accessible in another way).
+bool all_page_locked(const void *const host[42]) {
+  for (int i = 0; i < 42; ++i) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, host[i]) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return false;
+    }
+    if (a.type == cudaMemoryTypeUnregistered) return false;
+  }
+  return true;
 }
 
 // The host-pointer pipeline of cloudsc_b200_batched_host(_sp): chunks of
@@ -937,7 +953,8 @@ int host_pipeline(const void *host[42], int32_t nproma, int32_t klev, int32_t ng
   int rc = ensure_params(&dev);
   if (rc) return rc;
   const size_t np = nproma, kl = klev;
-  int cb = chunk_blocks > 0 ? chunk_blocks : default_chunk_blocks(np, kl, ngpblks, fb);
+  int cb = chunk_blocks > 0 ? chunk_blocks
+                            : default_chunk_blocks(np, kl, ngpblks, fb, all_page_locked(host));
   if (cb > ngpblks) cb = ngpblks;
   const int nslot = 3;
   const size_t slot_bytes = carve(nullptr, np, kl, cb, nullptr, fb);
@@ -1603,6 +1620,13 @@ int cloudsc_b200_reciprocal_check(const double *b, int64_t n, double *y, int32_t
   cudaError_t e = launch_reciprocal_check(b, (long long)n, y, bad, (cudaStream_t)stream);
   if (e != cudaSuccess) return fail(CLOUDSC_E_CUDA, "kernel launch", e);
   return CLOUDSC_OK;
+}
+
+int cloudsc_b200_host_chunk_blocks(int32_t nproma, int32_t klev, int32_t ngpblks, int32_t real_bytes,
+                                   int32_t page_locked) {
+  if (nproma < 1 || klev < 2 || ngpblks < 1 || (real_bytes != 4 && real_bytes != 8))
+    return fail(CLOUDSC_E_SHAPE, "inconsistent NPROMA/KLEV/NGPBLKS or size of a real");
+  return default_chunk_blocks(nproma, klev, ngpblks, real_bytes, page_locked != 0);
 }
 
 int cloudsc_b200_sqrt_check(const double *x, int64_t n, double *y, int32_t *bad, void *stream) {
