@@ -19,6 +19,7 @@
 #define CLOUDSC_HOST_SEQUENCES
 #define CLOUDSC_HOST_WINDOW_CHECK
 #define CSC_ANY(C) ((void)(C), true)
+#define CSC_ANY_LEFT(ROWS) ((ROWS) != 0u)  // a neighbour's rows change nothing here
 #endif
 // Parked values and process groups of the fast pass as in the kernels' narrow
 // (0) or 256-thread (-1) builds.
