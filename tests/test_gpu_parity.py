@@ -149,11 +149,12 @@ def test_launch_shapes(cuda, threads):
     boundaries), with a persistent grid, give identical results."""
     p, po = util.params()
     arrs = inputs.generate(6, 128, p, seed=31)
+    before = cloudsc.get_schedule(cloudsc.FP64)
     try:
         cloudsc.set_launch(cloudsc.FP64, threads, 1)
         _check(p, po, arrs, 128, 6, 6 * 128 - 3)
     finally:
-        cloudsc.set_launch(cloudsc.FP64, 448, 0)
+        cloudsc.set_schedule(cloudsc.FP64, *before)
 
 
 def test_config2_sampled_blocks(cuda):
