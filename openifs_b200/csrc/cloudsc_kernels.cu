@@ -62,9 +62,14 @@ int kernel_max_threads(int precision, int v, bool gen, int klev, bool sp) {
 // and 128: FP64, 120,000 columns, on the 448-thread build 7.13 and 10.87, on the
 // 256-thread one 5.44 and 5.78; FP32-mixed 5.98 and 9.21, 4.34 and 4.17; budgets,
 // 60,000 columns, 7.19 and 12.46, 5.70 and 5.79).  -1: the form has no such
-// build (parameters that rule out the GEN kernels).
+// build (parameters that rule out the GEN kernels).  The FP32-physics form parks
+// nothing, so its 448-thread build shares an SM already: in the single-precision
+// interface CTAs set for the 256-thread variant run on it (CTAs of 256, 65,536
+// columns: 2.28 ms against 2.66); its 256-thread build serves few columns, by
+// size.
 int variant_for_threads(int precision, int v, int threads, bool gen, int klev, bool sp) {
   const bool fast = klev <= kMaxLevFast;
+  if (sp && precision == 2 && kVariants[v].maxt == 256) return kDefaultVariant;
   const auto find = [&](int u) { return sp ? find_kernel_sp(precision, u, gen, fast) : find_kernel(precision, u, gen, fast); };
   if (threads > 256 || find(v).smem == 0) return v;
   for (int u = 0; u < kNumVariants; ++u)
