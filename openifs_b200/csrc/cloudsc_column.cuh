@@ -184,9 +184,9 @@ CSC_DEV double fast_quot(double a, double b, double y) {
 // of a division, the same operations otherwise.  q0 lies within two ulp of
 // a/b, its residual is then off by at most one rounding, the first correction
 // (with RN(1/b)) still ends within one ulp, and the second is Markstein's.
-// Measured with it and without (ms): FP64 3,200 columns 1.203 / 1.225, FP32-
-// mixed 90,005 2.700 / 2.757, SPP 24,576 2.267 / 2.286, satadj 100,000 0.857 /
-// 0.881; FP64 at 128 and 168 registers no gain (262,144 columns 9.494 / 9.472),
+// Measured with it and without in one session (ms): FP64 3,200 columns 1.203 /
+// 1.225, FP32-mixed 90,005 2.700 / 2.757, SPP 24,576 2.267 / 2.286, satadj
+// 100,000 0.857 / 0.881 (0.87-0.90 elsewhere); FP64 at 128 and 168 registers no gain (262,144 columns 9.494 / 9.472),
 // so the level code there keeps the other order (SHORT).
 CSC_DEV double fast_quot_rcp(double a, double b) {
 #if CSC_SEQUENCES

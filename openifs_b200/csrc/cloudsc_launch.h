@@ -11,17 +11,15 @@ namespace cloudsc {
 // registers, so each pair fixes the register budget per thread (and with it
 // the spills) and the CTA size it is meant for; the autotuner picks a
 // variant, a CTA size up to its MAXT and the persistence at run time.
-// 448 columns per CTA fill 148 SMs 3.96 times at 262,144 columns; the
-// (448, 1) bound gives them 144 registers (0.8 % faster than the 128 of a
-// (512, 1) bound, same bits).  Earlier measurements at 262,144 columns, FP64:
-// 384 columns per CTA at 168 registers 17.77 ms against 15.98 ms at 448;
-// three 128-thread CTAs per SM 21.7 ms.
+// At 262,144 columns, FP64, by size: five waves of 384 columns per CTA at 168
+// registers 9.46 ms; four of 448 at 128 registers 9.7; seven of 256 at 255
+// registers 10.0 (pick_schedule has the time of a wave of each).
 struct Variant {
   int maxt, minb;
 };
 constexpr Variant kVariants[] = {{640, 1}, {448, 1}, {384, 1}, {256, 1}, {256, 2}, {128, 3}};
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
-constexpr int kDefaultVariant = 1;  // (448, 1), run with 448 columns per CTA
+constexpr int kDefaultVariant = 1;  // (448, 1): exists in every form
 
 // A compiled column kernel: its function, the largest CTA it takes and the
 // dynamic shared memory of its parking slots.

@@ -14,13 +14,15 @@ cudaError_t upload_points(const KParams<double> &kd, const KParams<float> &kf, c
 // (ib * KLEV + jk) * NPROMA + jl -- the element offset of a level field -- so
 // consecutive threads read consecutive columns of one level (coalesced).  A
 // grid-stride loop covers all points of all blocks; levels above NCLDTOP get
-// zero tendencies (cloud_satadj.F90:338-345).  Bound by FP64 latency and issue
-// (about 900 instructions a point, two fifths of them FP64).  128-thread CTAs
-// at 96 registers (5 CTAs, 20 warps per SM), 100,000 columns of 137 levels:
-// 881 us; 913 with IEEE division, the full exponential and two 64-bit index
-// divisions a point (256 threads, 64 registers).  128 registers 3 % and 80 or
-// fewer 4-14 % slower; prefetching the next point's lines to L2, or copying
-// its inputs to shared memory ahead of time, no faster.
+// zero tendencies (cloud_satadj.F90:338-345).  Bound by the latency of its
+// FP64 chains (four saturation evaluations one after the other): about 1,600
+// instructions a point, 44 % of them FP64; FP64 pipe 58 %, issue 66 %.
+// 128-thread CTAs at 96 registers (5 CTAs, 20 warps per SM), 100,000 columns of
+// 137 levels: 869-897 us; 913-915 with IEEE division, the full exponential and
+// two 64-bit index divisions a point (256 threads, 64 registers; 1,900
+// instructions).  128 registers 3 % and 80 or fewer 4-14 % slower; prefetching
+// the next point's lines to L2, or copying its inputs to shared memory ahead of
+// time, no faster.
 // INC: STATE_INCREMENT of the cumulative tendencies fused in
 // (callpar.F90:1278-1280): each point writes CML + LOC back into the CML
 // arrays it has just read (inc_* not NULL), one addition each, as the
